@@ -15,11 +15,10 @@ namespace h3g {
 
 namespace {
 
-constexpr int kET = 256;
+constexpr int kET = jac::kThreads;
 constexpr int kEigMaxSweeps = 30;
-constexpr size_t kModelEigSmem = size_t(2) * SP * jac::LD * sizeof(double);
 
-// grid (nmod), block 256: one model per CTA.
+// grid (nmod), block kET: one model per CTA.
 __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q, const double* __restrict__ pi, int S,
                                                    double* lam, double* U, double* UT, double* V) {
     pdl_enter();
@@ -52,12 +51,12 @@ __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q,
         }
     }
     __syncthreads();
-    jac::sweeps<kET>(A, E, js, kEigMaxSweeps);
+    jac::sweeps(sm, js, kEigMaxSweeps);
     double* lk = lam + size_t(k) * SP;
     double* Uk = U + size_t(k) * SP2;
     double* UTk = UT + size_t(k) * SP2;
     double* Vk = V + size_t(k) * SP2;
-    if (tid < SP) lk[tid] = tid < S ? fmin(A[tid * LD + tid], 0.0) : 0.0;
+    if (tid < SP) lk[tid] = tid < S ? fmin(js.lam[tid], 0.0) : 0.0;
     for (int e = tid; e < SP2; e += kET) {
         const int a = e >> 6, b = e & 63;
         const bool real = a < S && b < S;
@@ -71,12 +70,12 @@ __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q,
 }  // namespace
 
 void eigen_configure() {
-    cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kModelEigSmem));
+    cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem));
 }
 
 int launch_model_eig(const double* Q, const double* pi, int S, int nmod, double* lam, double* U, double* UT, double* V,
                      cudaStream_t s) {
-    launch_k(k_model_eig, nmod, kET, kModelEigSmem, s, Q, pi, S, lam, U, UT, V);
+    launch_k(k_model_eig, nmod, kET, jac::kSmem, s, Q, pi, S, lam, U, UT, V);
     return 1;
 }
 

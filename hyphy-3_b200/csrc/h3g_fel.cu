@@ -39,7 +39,6 @@ constexpr int kFT = 256;                  // threads per CTA
 constexpr int LD = jac::LD;               // padded row stride: column walks hit 32 distinct banks
 constexpr int kMaxSweeps = 30;
 constexpr int kMaxDepth = 1024;           // open internal nodes on the traversal stack
-constexpr size_t kEigSmem = size_t(2) * SP * LD * sizeof(double);
 
 struct FelModel {
     int S;
@@ -55,14 +54,12 @@ struct FelModel {
 };
 
 // ----------------------------------------------------------------- eigensystems
-// grid n_eig, block 256.  Jacobi rotations as in Golub & Van Loan (Alg. 8.5.3);
-// one sweep = 63 rounds of 32 disjoint pairs (circle schedule), each round
-// A <- A J (columns) then A <- J^T A (rows), E <- E J.
+// grid n_eig, block jac::kThreads: the symmetric form diagonalised by the sweeps of h3g_jacobi.cuh.
 // Warm start: when prev[r] >= 0 the eigenvectors E0 of that slot (E0 = D^1/2 U)
 // are the starting basis: A <- E0^T A E0, E <- E0.  A pattern's next omega is
 // usually close to its last one, so the rotated matrix is nearly diagonal and
-// the sweeps needed drop from ~8 to 2-3.
-__global__ void __launch_bounds__(kFT) k_fel_eig(FelModel f, const double* __restrict__ omega, const int* __restrict__ slot,
+// the sweeps needed drop from 8 to 3-5.
+__global__ void __launch_bounds__(jac::kThreads, 2) k_fel_eig(FelModel f, const double* __restrict__ omega, const int* __restrict__ slot,
                                                  const int* __restrict__ prev) {
     pdl_enter();
     extern __shared__ __align__(16) double sm[];
@@ -72,7 +69,7 @@ __global__ void __launch_bounds__(kFT) k_fel_eig(FelModel f, const double* __res
     const int tid = threadIdx.x, S = f.S;
     const double om = omega[blockIdx.x];
     const int sl = slot[blockIdx.x];
-    for (int e = tid; e < SP2; e += kFT) {
+    for (int e = tid; e < SP2; e += jac::kThreads) {
         const int i = e >> 6, j = e & 63;
         double v = 0.0;
         if (i < S && j < S && i != j) v = f.sq[i] * (f.Qs[i * S + j] + om * f.Qn[i * S + j]) * f.isq[j];
@@ -87,7 +84,7 @@ __global__ void __launch_bounds__(kFT) k_fel_eig(FelModel f, const double* __res
         A[tid * LD + tid] = -row;
     }
     __syncthreads();
-    for (int e = tid; e < SP2; e += kFT) {        // symmetric part (rate_matrix.hpp:236-237)
+    for (int e = tid; e < SP2; e += jac::kThreads) {        // symmetric part (rate_matrix.hpp:236-237)
         const int i = e >> 6, j = e & 63;
         if (i < j) {
             const double m = 0.5 * (A[i * LD + j] + A[j * LD + i]);
@@ -99,36 +96,43 @@ __global__ void __launch_bounds__(kFT) k_fel_eig(FelModel f, const double* __res
     const int pv = prev[blockIdx.x];
     if (pv >= 0) {
         const double* U0 = f.U + size_t(pv) * SP2;
-        for (int e = tid; e < SP2; e += kFT) {
+        for (int e = tid; e < SP2; e += jac::kThreads) {
             const int i = e >> 6, k = e & 63;
             E[i * LD + k] = i < S ? f.sq[i] * U0[e] : (i == k ? 1.0 : 0.0);
         }
         __syncthreads();
+        const bool on = tid < 256;                       // the products: 256 threads, 16 entries each
         const int i = tid & 63, kq = (tid >> 6) * 16;
         double acc[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) acc[m] = 0.0;
-        for (int j = 0; j < SP; ++j) {                   // T = A E0, row i, columns kq..kq+15
-            const double aij = A[i * LD + j];
+        if (on)
+            for (int j = 0; j < SP; ++j) {               // T = A E0, row i, columns kq..kq+15
+                const double aij = A[i * LD + j];
 #pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = fma(aij, E[j * LD + kq + m], acc[m]);
-        }
+                for (int m = 0; m < 16; ++m) acc[m] = fma(aij, E[j * LD + kq + m], acc[m]);
+            }
         __syncthreads();
+        if (on) {
 #pragma unroll
-        for (int m = 0; m < 16; ++m) A[i * LD + kq + m] = acc[m];
+            for (int m = 0; m < 16; ++m) A[i * LD + kq + m] = acc[m];
+        }
         __syncthreads();
 #pragma unroll
         for (int m = 0; m < 16; ++m) acc[m] = 0.0;
-        for (int j = 0; j < SP; ++j) {                   // B = E0^T T, row k = i, columns kq..kq+15
-            const double ejk = E[j * LD + i];
+        if (on)
+            for (int j = 0; j < SP; ++j) {               // B = E0^T T, row k = i, columns kq..kq+15
+                const double ejk = E[j * LD + i];
 #pragma unroll
-            for (int m = 0; m < 16; ++m) acc[m] = fma(ejk, A[j * LD + kq + m], acc[m]);
+                for (int m = 0; m < 16; ++m) acc[m] = fma(ejk, A[j * LD + kq + m], acc[m]);
+            }
+        __syncthreads();
+        if (on) {
+#pragma unroll
+            for (int m = 0; m < 16; ++m) A[i * LD + kq + m] = acc[m];
         }
         __syncthreads();
-#pragma unroll
-        for (int m = 0; m < 16; ++m) A[i * LD + kq + m] = acc[m];
-        __syncthreads();
-        for (int e = tid; e < SP2; e += kFT) {           // re-symmetrise the rounding
+        for (int e = tid; e < SP2; e += jac::kThreads) {           // re-symmetrise the rounding
             const int a = e >> 6, b = e & 63;
             if (a < b) {
                 const double m = 0.5 * (A[a * LD + b] + A[b * LD + a]);
@@ -138,12 +142,12 @@ __global__ void __launch_bounds__(kFT) k_fel_eig(FelModel f, const double* __res
         }
         __syncthreads();
     }
-    jac::sweeps<kFT>(A, E, js, kMaxSweeps);
+    jac::sweeps(sm, js, kMaxSweeps);
     double* lam = f.lam + size_t(sl) * SP;
     double* U = f.U + size_t(sl) * SP2;
     double* V = f.V + size_t(sl) * SP2;
-    if (tid < SP) lam[tid] = fmin(A[tid * LD + tid], 0.0);
-    for (int e = tid; e < SP2; e += kFT) {
+    if (tid < SP) lam[tid] = fmin(js.lam[tid], 0.0);
+    for (int e = tid; e < SP2; e += jac::kThreads) {
         const int a = e >> 6, b = e & 63;
         U[e] = f.isq[a] * E[a * LD + b];                  // U_pi[i = a][k = b]
         V[e] = E[b * LD + a] * f.sq[b];                   // V_pi[k = a][j = b]
@@ -775,7 +779,7 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
          cudaStreamSynchronize(d->s) == cudaSuccess;
     static bool configured = false;
     if (ok && !configured) {
-        ok = cudaFuncSetAttribute(k_fel_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kEigSmem)) == cudaSuccess &&
+        ok = cudaFuncSetAttribute(k_fel_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(1, false))) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(2, false))) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(1, true))) == cudaSuccess &&
@@ -893,7 +897,7 @@ bool stage_batch(FelDevice* d, int n_eig, const double* eig_omega, const int* ei
     d->h2d += bytes;
     unsigned char* g = d->d_req;
     if (n_eig > 0) {
-        launch_k(k_fel_eig, n_eig, kFT, kEigSmem, s, d->f, reinterpret_cast<const double*>(g),
+        launch_k(k_fel_eig, n_eig, jac::kThreads, jac::kSmem, s, d->f, reinterpret_cast<const double*>(g),
                  reinterpret_cast<const int*>(g + o_es), reinterpret_cast<const int*>(g + o_pv));
         ++d->launches;
     }

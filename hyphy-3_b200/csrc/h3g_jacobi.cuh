@@ -3,11 +3,32 @@
 // engine's model eigensystems (h3g_eigen.cu).
 //
 // Golub & Van Loan, "Matrix Computations" (Alg. 8.5.1 / 8.5.3): one sweep = 63 rounds of 32
-// disjoint rotations (p_k, q_k) covering all 64 indices (circle schedule).  Warp 0 computes the
-// round's rotations (t from one square root and one divide, c = rsqrt(1 + t^2)); then every 2x2
-// block (I, J) of A is replaced by R_I^T A_IJ R_J in one pass, the diagonal blocks by their exact
-// annihilated values a_pp - t a_pq, a_qq + t a_pq and 0, and the columns of E by E R.  Two
-// barriers per round.  The sweeps stop when the off-diagonal mass is below 1e-30 of the total.
+// disjoint rotations (p_k, q_k), p < q, covering all 64 indices (circle schedule: seat k of round r
+// pairs x = r + k with y = r - k mod 63, seat 0 pairs 63 with r).  A round replaces every 2x2 block
+// (I, J) of A by R_I^T A_IJ R_J, the diagonal blocks by their exact annihilated values
+// a_pp - t a_pq, a_qq + t a_pq and 0, and the columns of E by E R.  The sweeps stop when the
+// off-diagonal mass is below 1e-30 of the total.
+//
+// One matrix is a chain of ~500 dependent rounds (8 sweeps), and shared-memory bandwidth is what a
+// round costs once several matrices share an SM.  So:
+//   - A warp of its own runs one round ahead: from the rotations of round r and the A before it, it forms
+//     just the 32 entries that round r + 1 annihilates (one 2x2 block each, in the workers' arithmetic, so
+//     with the same bits) and from them the rotations of round r + 1 (square root, divide, reciprocal
+//     square root: the longest chain of a round), while the workers apply round r from one buffer into the
+//     other: one barrier a round.
+//   - A is stored by seat, not by index: x_k at position k, y_k at 32 + k.  From one round to the next the
+//     occupants move to the neighbouring seat (x_k -> x_{k-1}, y_k -> y_{k+1}; y_0 <- x_1, x_31 <- y_31, 63
+//     stays), so a worker stores its results one position on and all its addresses are fixed.  A row's 32 p
+//     (or q) entries then lie in nearly as many banks whichever of x and y is the p, and no index is computed
+//     modulo 63.
+//   - E stays in the workers' registers, four threads to a row with eight seats each; a round passes two
+//     entries per thread on through shared memory (E in shared memory cost as much bandwidth as A).
+// A round takes 1540 cycles with one CTA on the SM and 1320 per matrix with two; it moves 1060 wavefronts through
+// shared memory (A's loads and stores 750, the rest c, s and E's entries), which bounds the second figure.
+// Measured, dense random 61-state matrices (8 sweeps) at 148 / 296 / 444 at once: 397 / 593 / 904 us; with A and E in
+// shared memory by index and two barriers a round, the rotations between them: 874 / 1215 / 1695 us.  Tried: 512
+// workers (437 / 679 / 1002), A and E on warps of their own (393 / 624 / 925), the rotation warp alone on
+// its quarter of the SM (454 / 735 / 1068).
 #pragma once
 
 #include "h3g_common.cuh"
@@ -15,97 +36,280 @@
 namespace h3g {
 namespace jac {
 
-constexpr int LD = SP + 1;                // padded row stride: column walks hit 32 distinct banks
+constexpr int LD = SP + 1;                // row stride of the callers' A and E: column walks hit 16 distinct 8-byte banks
+constexpr int kWorkers = 256;             // threads that update A and E
+constexpr int kWarps = kWorkers / 32;
+constexpr int kSeats = 8;                 // seats of E a worker holds
+constexpr int kGroups = 32 / kSeats;      // workers that share a row of E
+constexpr int kBlocks = 32 / kWarps;      // blocks of A a worker updates
+constexpr int kThreads = kWorkers + 32;   // and the warp that computes the rotations
+// A by position: rows 0 .. 31 hold x, 32 .. 63 y; columns 0 .. 31 x, 47 .. 78 y.  With y's columns one bank
+// behind x's, the loads (x_k or y_k from lane k) and the stores one seat on (x_1 to y_0 and y_31 to x_31
+// among them) hit 16 distinct banks per half warp but for the one where the roles change.
+constexpr int kYCol = 47;
+constexpr int kPitch = 80;
+constexpr int kBuf = SP * kPitch;         // one buffer of A
+constexpr size_t kSmem = size_t(2) * kBuf * sizeof(double);   // the callers' A and E fit in it too
 
-struct Scratch {                          // shared-memory scratch of one round
-    double c[32], s[32], t[32], apq[32], app[32], aqq[32];
-    int p[32], q[32];
-    double red[32];
+struct Scratch {
+    double2 cs[2][32];                    // (c, s) of a round's seats, by round parity
+    double up[2][kGroups * SP], down[2][kGroups * SP];   // entries of E on their way to the next lower / higher seat group
+    double lam[SP];                       // the diagonal, by index, when the sweeps are done
+    double red[kWarps];
 };
 
-template <int NT>
-__device__ __forceinline__ double block_sum_or_max(double v, double* red, bool is_max) {
-    for (int o = 16; o > 0; o >>= 1) {
-        const double w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = is_max ? fmax(v, w) : v + w;
-    }
+// sum over the worker threads' v (the rotation warp's is not counted); all threads call
+__device__ __forceinline__ double block_sum(double v, double* red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) red[warp] = v;
+    if ((threadIdx.x & 31) == 0 && warp < kWarps) red[warp] = v;
     __syncthreads();
     double r = red[0];
-    for (int k = 1; k < NT / 32; ++k) r = is_max ? fmax(r, red[k]) : r + red[k];
+    for (int k = 1; k < kWarps; ++k) r += red[k];
     __syncthreads();
     return r;
 }
 
-// A (symmetric, [64][LD]) is diagonalised in place; E ([64][LD]) is multiplied by the rotations
-// (start it at the identity, or at a warm-start basis with A already rotated into it).
-// NT threads (a multiple of 32, at least 64).
-template <int NT>
-__device__ void sweeps(double* A, double* E, Scratch& js, int max_sweeps) {
-    const int tid = threadIdx.x;
-    for (int sweep = 0; sweep < max_sweeps; ++sweep) {
-        double off = 0.0, tot = 0.0;
-        for (int e = tid; e < SP2; e += NT) {
-            const int i = e >> 6, j = e & 63;
-            const double x = A[i * LD + j] * A[i * LD + j];
-            tot += x;
-            if (i != j) off += x;
-        }
-        off = block_sum_or_max<NT>(off, js.red, false);
-        tot = block_sum_or_max<NT>(tot, js.red, false);
-        if (off <= 1e-30 * tot || off == 0.0) break;
-        for (int round = 0; round < SP - 1; ++round) {
-            if (tid < 32) {
-                int p, q;
-                if (tid == 0) { p = SP - 1; q = round; }
-                else { p = (round + tid) % (SP - 1); q = (round - tid + (SP - 1)) % (SP - 1); }
-                if (p > q) { const int tmp = p; p = q; q = tmp; }
-                const double apq = A[p * LD + q], app = A[p * LD + p], aqq = A[q * LD + q];
-                double c = 1.0, s = 0.0, t = 0.0;
-                if (fabs(apq) >= 1e-300) {
-                    // t = tan(theta) of the smaller rotation, tau = (a_qq - a_pp) / (2 a_pq):
-                    // t = sign(tau) / (|tau| + sqrt(1 + tau^2)) = 2 a_pq sign(d) / (|d| + sqrt(d^2 + 4 a_pq^2)), d = a_qq - a_pp
-                    const double d = aqq - app;
-                    const double tt = 2.0 * apq / (fabs(d) + sqrt(d * d + 4.0 * apq * apq));
-                    t = d >= 0.0 ? tt : -tt;
-                    c = rsqrt(1.0 + t * t);
-                    s = t * c;
-                }
-                js.p[tid] = p; js.q[tid] = q; js.c[tid] = c; js.s[tid] = s;
-                js.t[tid] = t; js.apq[tid] = apq; js.app[tid] = app; js.aqq[tid] = aqq;
-            }
-            __syncthreads();
-            for (int e = tid; e < 32 * 32; e += NT) {      // block (I, J) of A
-                const int I = e >> 5, J = e & 31;
-                const int pI = js.p[I], qI = js.q[I], pJ = js.p[J], qJ = js.q[J];
-                if (I == J) {
-                    A[pI * LD + pI] = js.app[I] - js.t[I] * js.apq[I];
-                    A[qI * LD + qI] = js.aqq[I] + js.t[I] * js.apq[I];
-                    A[pI * LD + qI] = 0.0;
-                    A[qI * LD + pI] = 0.0;
-                    continue;
-                }
-                const double cI = js.c[I], sI = js.s[I], cJ = js.c[J], sJ = js.s[J];
-                const double a = A[pI * LD + pJ], b = A[pI * LD + qJ], cc = A[qI * LD + pJ], dd = A[qI * LD + qJ];
-                const double m0 = cJ * a - sJ * b, m1 = sJ * a + cJ * b;      // [a b; c d] R_J
-                const double m2 = cJ * cc - sJ * dd, m3 = sJ * cc + cJ * dd;
-                A[pI * LD + pJ] = cI * m0 - sI * m2;                        // R_I^T (...)
-                A[pI * LD + qJ] = cI * m1 - sI * m3;
-                A[qI * LD + pJ] = sI * m0 + cI * m2;
-                A[qI * LD + qJ] = sI * m1 + cI * m3;
-            }
-            for (int e = tid; e < 32 * SP; e += NT) {      // columns p, q of E
-                const int k = e >> 6, i = e & 63;
-                const int p = js.p[k], q = js.q[k];
-                const double c = js.c[k], s = js.s[k];
-                const double ekp = E[i * LD + p], ekq = E[i * LD + q];
-                E[i * LD + p] = c * ekp - s * ekq;
-                E[i * LD + q] = s * ekp + c * ekq;
-            }
-            __syncthreads();
+// the index at a position in round 0 (and after every whole sweep)
+__device__ __forceinline__ int index_at(int pos) {
+    if (pos < 32) return pos == 0 ? SP - 1 : pos;
+    return pos == 32 ? 0 : SP - 1 - (pos - 32);
+}
+// where the x / y of seat k goes after a round: row, and column
+__device__ __forceinline__ int next_x(int k, int y_at) { return k == 0 ? 0 : (k == 1 ? y_at : k - 1); }
+__device__ __forceinline__ int next_y(int k, int y_at) { return k == 31 ? 31 : y_at + k + 1; }
+// seats k >= first_xp(r) have x < y, so x is their p; in the others y is
+__device__ __forceinline__ int first_xp(int r) { return r <= 31 ? r + 1 : SP - 1 - r; }
+
+// One pair of entries through a rotation, the p and the q result.  The roundings are spelled out: the
+// rotation warp and the workers form the same entry independently, and the bits must agree.
+__device__ __forceinline__ double rot_p(double2 r, double a, double b) { return fma(r.x, a, -__dmul_rn(r.y, b)); }
+__device__ __forceinline__ double rot_q(double2 r, double a, double b) { return fma(r.y, a, __dmul_rn(r.x, b)); }
+
+// rotation that annihilates a_pq: (c, s) and t = tan(theta)
+__device__ __forceinline__ double2 rotation(double apq, double app, double aqq, double& t) {
+    double c = 1.0, s = 0.0;
+    t = 0.0;
+    if (fabs(apq) >= 1e-300) {
+        // t = tan(theta) of the smaller rotation, tau = (a_qq - a_pp) / (2 a_pq):
+        // t = sign(tau) / (|tau| + sqrt(1 + tau^2)) = 2 a_pq sign(d) / (|d| + sqrt(d^2 + 4 a_pq^2)), d = a_qq - a_pp
+        const double d = aqq - app;
+        const double tt = 2.0 * apq / (fabs(d) + sqrt(fma(4.0 * apq, apq, __dmul_rn(d, d))));
+        t = d >= 0.0 ? tt : -tt;
+        c = rsqrt(fma(t, t, 1.0));
+        s = t * c;
+    }
+    return make_double2(c, s);
+}
+
+// A worker's four seats of one row of E through their rotations.  kRole: x is the p of 0 no seat, 1 every seat,
+// 2 the seats k >= first.
+template <int kRole>
+__device__ __forceinline__ void rotate_seats(double (&ex)[kSeats], double (&ey)[kSeats], const double2* cs, int first) {
+#pragma unroll
+    for (int k = 0; k < kSeats; ++k) {
+        const double2 q = cs[k];
+        const double x = ex[k], y = ey[k];
+        if (kRole == 1 || (kRole == 2 && k >= first)) {
+            ex[k] = rot_p(q, x, y);
+            ey[k] = rot_q(q, x, y);
+        } else {
+            ey[k] = rot_p(q, y, x);
+            ex[k] = rot_q(q, y, x);
         }
     }
+}
+
+// What a worker keeps through all rounds: its part of E, and the offsets of its column and rows of A and of
+// where they move to.
+struct Worker {
+    double ex[kSeats], ey[kSeats];
+    int cx, cy, tx, ty;                                // column of x_J and y_J, J = lane, and where they go
+    int rx[kBlocks], ry[kBlocks], sx[kBlocks], sy[kBlocks];   // rows of x_I and y_I of its blocks, and where they go
+    int xe;                                            // its place in the entries of E passed on
+};
+// keep a value in its register: recomputing the offsets every round doubled the round's instructions
+__device__ __forceinline__ void pin(int& x) { asm volatile("" : "+r"(x)); }
+
+// Workers: apply round r to E (registers) and A (cur -> nxt).  `in` is the parity that the round's inputs have.
+__device__ __forceinline__ void worker_round(Worker& w, const double* cur, double* nxt, Scratch& js, int in, int r, int wp, int lane,
+                                             bool moved) {
+    const double2* cs = js.cs[in];
+    const int first = first_xp(r);
+    {   // E first: the rotation warp's few loads then go ahead of the workers' many
+        const int eh = wp >> 1;
+        if (moved) {                                   // the entries that the last round passed on
+            if (eh < kGroups - 1) w.ex[kSeats - 1] = js.up[in][w.xe];
+            if (eh > 0) w.ey[0] = js.down[in][w.xe];
+        }
+        const int f = first - kSeats * eh;
+        if (f >= kSeats) rotate_seats<0>(w.ex, w.ey, cs + kSeats * eh, f);
+        else if (f <= 0) rotate_seats<1>(w.ex, w.ey, cs + kSeats * eh, f);
+        else rotate_seats<2>(w.ex, w.ey, cs + kSeats * eh, f);
+        if (eh > 0) js.up[in ^ 1][w.xe - SP] = w.ex[0];
+        if (eh < kGroups - 1) js.down[in ^ 1][w.xe + SP] = w.ey[kSeats - 1];
+        const double x0 = w.ex[0], x1 = w.ex[1], y_last = w.ey[kSeats - 1];
+#pragma unroll
+        for (int k = 0; k < kSeats - 1; ++k) w.ex[k] = w.ex[k + 1];
+        if (eh == 0) w.ex[0] = x0;                     // 63 stays in seat 0
+        w.ex[kSeats - 1] = y_last;                     // seat 31's x (the other groups' comes from above)
+#pragma unroll
+        for (int k = kSeats - 1; k > 0; --k) w.ey[k] = w.ey[k - 1];
+        w.ey[0] = x1;                                  // seat 0's y (the other groups' comes from below)
+    }
+    const bool xc = lane >= first;
+    const int pc = xc ? w.cx : w.cy, qc = xc ? w.cy : w.cx, pt = xc ? w.tx : w.ty, qt = xc ? w.ty : w.tx;
+    const double2 rJ = cs[lane];
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {                // blocks (I, J) of A, J = lane
+        const int I = wp + kWarps * i;
+        const bool xr = I >= first;
+        const int pr = xr ? w.rx[i] : w.ry[i], qr = xr ? w.ry[i] : w.rx[i];
+        const double2 rI = cs[I];
+        const double a = cur[pr + pc], b = cur[pr + qc], c = cur[qr + pc], d = cur[qr + qc];
+        const double m0 = rot_p(rJ, a, b), m1 = rot_q(rJ, a, b);      // [a b; c d] R_J
+        const double m2 = rot_p(rJ, c, d), m3 = rot_q(rJ, c, d);
+        const int sp = xr ? w.sx[i] : w.sy[i], sq = xr ? w.sy[i] : w.sx[i];
+        if (I != lane) {                                             // R_I^T (...); the rotation warp writes the diagonal blocks
+            nxt[sp + pt] = rot_p(rI, m0, m2);
+            nxt[sp + qt] = rot_p(rI, m1, m3);
+            nxt[sq + pt] = rot_q(rI, m0, m2);
+            nxt[sq + qt] = rot_q(rI, m1, m3);
+        }
+    }
+}
+
+// The rotation warp's round r, seat k = lane: the rotations of round r + 1.  dx, dy: the diagonal entries of the seat's
+// occupants after round r, moved on here to round r + 1's occupants.
+__device__ __forceinline__ void ahead_round(double& dx, double& dy, const double* cur, double* nxt, const double2* cs, double2* cs_next,
+                                            int r, int k) {
+    const int first = first_xp(r), next = first_xp(r + 1 < SP - 1 ? r + 1 : 0);
+    // the next occupants' seats in this round, and whether they are its p: x comes from seat k + 1 (seat 31's is
+    // its own y, seat 0's stays), y from seat k - 1 (seat 0's is seat 1's x)
+    const int sx = k == 0 ? 0 : (k == 31 ? 31 : k + 1), sy = k == 0 ? 1 : k - 1;
+    const bool x_is_p = (sx >= first) == (k != 31), y_is_p = (sy >= first) == (k == 0);
+    const bool xp = k >= next;                         // the row of a_pq is the smaller index
+    const int sr = xp ? sx : sy, sc = xp ? sy : sx;
+    const bool rp = xp ? x_is_p : y_is_p, cp = xp ? y_is_p : x_is_p;
+    const int pr = (sr >= first ? sr : 32 + sr) * kPitch, qr = (sr >= first ? 32 + sr : sr) * kPitch;
+    const int pc = sc >= first ? sc : kYCol + sc, qc = sc >= first ? kYCol + sc : sc;
+    const double2 rI = cs[sr], rJ = cs[sc];
+    const double a = cur[pr + pc], b = cur[pr + qc], c = cur[qr + pc], d = cur[qr + qc];
+    const double up = __shfl_down_sync(0xffffffffu, dx, 1), down = __shfl_up_sync(0xffffffffu, dy, 1);
+    const double nx = k == 0 ? dx : (k == 31 ? dy : up), ny = k == 0 ? up : down;
+    // rot_p or rot_q by choice of the coefficients
+    const double c0 = cp ? rJ.x : rJ.y, c1 = cp ? -rJ.y : rJ.x, r0 = rp ? rI.x : rI.y, r1 = rp ? -rI.y : rI.x;
+    const double u = fma(c0, a, __dmul_rn(c1, b)), v = fma(c0, c, __dmul_rn(c1, d));
+    const double apq = fma(r0, u, __dmul_rn(r1, v));
+    const double app = xp ? nx : ny, aqq = xp ? ny : nx;
+    double t;
+    cs_next[k] = rotation(apq, app, aqq, t);
+    // this round's diagonal blocks
+    nxt[next_x(k, 32) * kPitch + next_y(k, kYCol)] = 0.0;
+    nxt[next_y(k, 32) * kPitch + next_x(k, kYCol)] = 0.0;
+    nxt[k * (kPitch + 1)] = nx;
+    nxt[(32 + k) * kPitch + kYCol + k] = ny;
+    const double np = fma(-t, apq, app), nq = fma(t, apq, aqq);
+    dx = xp ? np : nq;
+    dy = xp ? nq : np;
+}
+
+// sm (kSmem bytes) holds A (symmetric, [64][LD]) and after it E ([64][LD]).  A is diagonalised, E multiplied by
+// the rotations (start it at the identity, or at a warm-start basis with A already rotated into it).  On
+// return js.lam holds the diagonal and E is where it was; A is lost.  All kThreads threads call.
+__device__ __forceinline__ void sweeps(double* sm, Scratch& js, int max_sweeps) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int wp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const bool worker = wp < kWarps;
+    // a warp holds one seat group of 32 rows of E, so which entry of a pair is its p is the same for all lanes
+    const int eh = (wp >> 1) & (kGroups - 1), er = 32 * (wp & 1) + lane;
+    double* E = sm + SP * LD + er * LD;
+    Worker w;
+#pragma unroll
+    for (int k = 0; k < kSeats; ++k) {
+        w.ex[k] = E[index_at(kSeats * eh + k)];
+        w.ey[k] = E[index_at(32 + kSeats * eh + k)];
+    }
+    w.cx = lane; w.cy = kYCol + lane; w.tx = next_x(lane, kYCol); w.ty = next_y(lane, kYCol);
+    w.xe = SP * eh + er;
+    pin(w.cx); pin(w.cy); pin(w.tx); pin(w.ty); pin(w.xe);
+#pragma unroll
+    for (int i = 0; i < kBlocks; ++i) {
+        const int I = (wp & (kWarps - 1)) + kWarps * i;
+        w.rx[i] = I * kPitch; w.ry[i] = (32 + I) * kPitch; w.sx[i] = next_x(I, 32) * kPitch; w.sy[i] = next_y(I, 32) * kPitch;
+        pin(w.rx[i]); pin(w.ry[i]); pin(w.sx[i]); pin(w.sy[i]);
+    }
+    // A by position, into the first buffer (it overlays the callers' A and E)
+    double mine[SP2 / kWorkers];
+    if (worker)
+#pragma unroll
+        for (int i = 0; i < SP2 / kWorkers; ++i) {
+            const int e = tid + kWorkers * i;
+            mine[i] = sm[index_at(e >> 6) * LD + index_at(e & 63)];
+        }
+    __syncthreads();
+    if (worker)
+#pragma unroll
+        for (int i = 0; i < SP2 / kWorkers; ++i) {
+            const int e = tid + kWorkers * i, j = e & 63;
+            sm[(e >> 6) * kPitch + (j < 32 ? j : j - 32 + kYCol)] = mine[i];
+        }
+    int par = 0;                                       // parity of the round to apply: the buffer that holds A
+    double dx = 0.0, dy = 0.0;                         // rotation warp: the seat's diagonal after that round
+    bool moved = false;
+    __syncthreads();
+    for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+        const double* cur = sm + (par ? kBuf : 0);
+        double off = 0.0, tot = 0.0;
+        if (worker)
+            for (int e = tid; e < SP2; e += kWorkers) {
+                const int i = e >> 6, j = e & 63;
+                const double v = cur[i * kPitch + (j < 32 ? j : j - 32 + kYCol)], x = v * v;
+                tot += x;
+                if (i != j) off += x;
+            }
+        off = block_sum(off, js.red);
+        tot = block_sum(tot, js.red);
+        if (off <= 1e-30 * tot || off == 0.0) break;
+        if (!moved && !worker) {                       // round 0's rotations from A itself
+            const bool xp = lane >= first_xp(0);
+            const int pr = (xp ? lane : 32 + lane) * kPitch, qr = (xp ? 32 + lane : lane) * kPitch;
+            const int pc = xp ? lane : kYCol + lane, qc = xp ? kYCol + lane : lane;
+            const double apq = cur[pr + qc], app = cur[pr + pc], aqq = cur[qr + qc];
+            double t;
+            js.cs[par][lane] = rotation(apq, app, aqq, t);
+            const double np = fma(-t, apq, app), nq = fma(t, apq, aqq);
+            dx = xp ? np : nq;
+            dy = xp ? nq : np;
+        }
+        for (int r = 0; r < SP - 1; ++r) {
+            __syncthreads();                           // A of this round, its rotations and the other buffer are ready
+            if (worker) {
+                if (par == 0) worker_round(w, sm, sm + kBuf, js, 0, r, wp, lane, moved);
+                else worker_round(w, sm + kBuf, sm, js, 1, r, wp, lane, moved);
+            } else {
+                if (par == 0) ahead_round(dx, dy, sm, sm + kBuf, js.cs[0], js.cs[1], r, lane);
+                else ahead_round(dx, dy, sm + kBuf, sm, js.cs[1], js.cs[0], r, lane);
+            }
+            moved = true;
+            par ^= 1;
+        }
+        __syncthreads();                               // the sweep's last round is complete
+    }
+    const double* cur = sm + (par ? kBuf : 0);
+    if (tid < SP) js.lam[index_at(tid)] = cur[tid * kPitch + (tid < 32 ? tid : tid - 32 + kYCol)];
+    if (worker && moved) {
+        if (eh < kGroups - 1) w.ex[kSeats - 1] = js.up[par][w.xe];
+        if (eh > 0) w.ey[0] = js.down[par][w.xe];
+    }
+    __syncthreads();                                   // A has been read: E's place is free
+    if (worker)
+#pragma unroll
+        for (int k = 0; k < kSeats; ++k) {             // a whole number of sweeps: the seats of round 0 again
+            E[index_at(kSeats * eh + k)] = w.ex[k];
+            E[index_at(32 + kSeats * eh + k)] = w.ey[k];
+        }
+    __syncthreads();
 }
 
 }  // namespace jac
