@@ -56,12 +56,14 @@ struct h3g_problem {
     h3g_ctx* ctx = nullptr;
     h3g_batch* batch = nullptr;        // the batch this problem evaluates in (its workspace lives there)
     int n = 0, root = -1, T = 0, P = 0, Pp = 0, NI = 0, max_state = -1;
-    std::vector<int> ch_off, ch, iidx, taxon, in_off, out_off, in_nodes, out_nodes, parent_h;
+    std::vector<int> ch_off, ch, iidx, taxon, in_off, out_off, in_nodes, out_nodes, out_split, out_int_off, parent_h;
     std::vector<uint8_t> leaf;
     std::vector<int> bfs_order, depth_h, height_h;   // BFS order from the root, node depths and heights
     std::vector<int8_t> states_pm;     // [P][T] as uploaded (per-pattern checks on the host)
     DevArena topo_mem, model_mem, work_mem;
-    int *d_ch_off = nullptr, *d_ch = nullptr, *d_iidx = nullptr, *d_taxon = nullptr, *d_in_nodes = nullptr, *d_out_nodes = nullptr;
+    int *d_ch_off = nullptr, *d_ch = nullptr, *d_iidx = nullptr, *d_taxon = nullptr, *d_in_nodes = nullptr;
+    int* d_out_split = nullptr;        // out_nodes: the internal ones (levels out_int_off), then leaf pairs (split_kids)
+    int pairs_at = 0, n_pairs = 0;
     int* d_parent = nullptr;
     uint8_t* d_leaf = nullptr;
     int2* d_kdesc = nullptr;
@@ -135,7 +137,7 @@ struct h3g_problem {
     int *d_ck_iidx = nullptr, *d_ck_vidx = nullptr, *d_ck_lists = nullptr;
     int2* d_ck_kdesc = nullptr;
     int4* d_ck_info = nullptr;
-    struct CkOffsets { int in, out, acc, in_info, out_info, in_next, in_heads, n_in_heads, out_next, out_heads, n_out_heads; };
+    struct CkOffsets { int in, out, pairs_at, n_pairs, acc; std::vector<int> out_int_off; int in_info, out_info, in_next, in_heads, n_in_heads, out_next, out_heads, n_out_heads; };
     std::vector<CkOffsets> ck_off;
     uint64_t ws_bytes = 0, full_bytes = 0;
     Topo topo() const {
@@ -210,6 +212,30 @@ extern "C" h3g_status h3g_ctx_destroy(h3g_ctx* ctx) {
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return H3G_OK;
+}
+
+// kids (children grouped by parent, levels off): the internal ones by level (int_off) and after them, from an even
+// position on, the leaves as pairs: the two of a node with just these, else (leaf, -1).
+static void split_kids(const std::vector<int>& kids, const std::vector<int>& off, const uint8_t* leaf, const int* parent,
+                       const std::vector<int>& n_kids, std::vector<int>& split, std::vector<int>& int_off, int& pairs_at, int& n_pairs) {
+    split.clear();
+    int_off.assign(1, 0);
+    for (size_t l = 0; l + 1 < off.size(); ++l) {
+        for (int k = off[l]; k < off[l + 1]; ++k)
+            if (!leaf[kids[size_t(k)]]) split.push_back(kids[size_t(k)]);
+        int_off.push_back(int(split.size()));
+    }
+    if (split.size() % 2) split.push_back(-1);
+    pairs_at = int(split.size());
+    for (size_t k = 0; k < kids.size(); ++k) {
+        const int c = kids[k];
+        if (!leaf[c]) continue;
+        const bool pair = n_kids[size_t(parent[c])] == 2 && k + 1 < kids.size() && parent[kids[k + 1]] == parent[c] && leaf[kids[k + 1]];
+        split.push_back(c);
+        split.push_back(pair ? kids[k + 1] : -1);
+        k += pair ? 1 : 0;
+    }
+    n_pairs = (int(split.size()) - pairs_at) / 2;
 }
 
 extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_t* parent, const uint8_t* is_leaf,
@@ -290,6 +316,9 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
                 if (!is_leaf[i] && depth[i] == d) for (int c : kids[i]) pr->out_nodes.push_back(c);
             pr->out_off.push_back(int(pr->out_nodes.size()));
         }
+        std::vector<int> n_kids(n);
+        for (int i = 0; i < n; ++i) n_kids[i] = int(kids[i].size());
+        split_kids(pr->out_nodes, pr->out_off, is_leaf, parent, n_kids, pr->out_split, pr->out_int_off, pr->pairs_at, pr->n_pairs);
         pr->parent_h.assign(parent, parent + n);
         if (n_patterns > 0) pr->states_pm.assign(states, states + size_t(n_patterns) * n_taxa);
         // patterns, taxon-major with padding (missing data, weight 0)
@@ -317,7 +346,7 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_taxon, n));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_leaf, n));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_in_nodes, std::max<size_t>(pr->in_nodes.size(), 1)));
-        H3G_TRY_CUDA(ctx, A.alloc(&pr->d_out_nodes, std::max<size_t>(pr->out_nodes.size(), 1)));
+        H3G_TRY_CUDA(ctx, A.alloc(&pr->d_out_split, std::max<size_t>(pr->out_split.size(), 1)));
         // descriptors for the persistent passes
         std::vector<int2> kdesc(std::max<size_t>(pr->ch.size(), 1));
         for (size_t j = 0; j < pr->ch.size(); ++j) {
@@ -397,8 +426,8 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_leaf, pr->leaf.data(), n, cudaMemcpyHostToDevice, s));
         if (!pr->in_nodes.empty())
             H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_in_nodes, pr->in_nodes.data(), pr->in_nodes.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-        if (!pr->out_nodes.empty())
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_out_nodes, pr->out_nodes.data(), pr->out_nodes.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        if (!pr->out_split.empty())
+            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_out_split, pr->out_split.data(), pr->out_split.size() * sizeof(int), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_states, st.data(), st.size(), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_masks, mk.data(), mk.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_w, wt.data(), wt.size() * sizeof(double), cudaMemcpyHostToDevice, s));
@@ -528,7 +557,7 @@ struct WsLayout {
 
 // part_nodes / vf_nodes: partial slots of internal nodes and gradient-operand slots (NI and n, or
 // fewer under a checkpoint plan).
-static WsLayout ws_layout(size_t n, size_t NI, size_t Pp, int M, int K, int nmod, int ndirs, const h3g_tuning& tu,
+static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, int K, int nmod, int ndirs, const h3g_tuning& tu,
                           size_t part_nodes = 0, size_t vf_nodes = 0) {
     (void)K;
     if (!part_nodes) part_nodes = NI;
@@ -540,11 +569,12 @@ static WsLayout ws_layout(size_t n, size_t NI, size_t Pp, int M, int K, int nmod
     L.pcols = size_t(M) * Pp;
     L.ecols = part_nodes * M * Pp;
     L.gt = size_t(M) * n;
-    // enough A chunks for ~600 CTAs, never below 256 patterns per chunk
+    // enough A chunks for ~600 CTAs, never below 64 patterns per chunk (two stages: a chunk of 256 left the smallest
+    // genes with 8 stages in a row on a handful of CTAs)
+    constexpr size_t kGrain = 64;
     const int want_chunks = std::max<int>(1, int((600 + n * M - 1) / (n * M)));
-    const int max_chunks = std::max<int>(1, int(Pp / 256));
-    L.nchunk = std::min(want_chunks, max_chunks);
-    L.chunk = int((Pp / TP + L.nchunk - 1) / L.nchunk) * TP;
+    L.nchunk = std::min<int>(want_chunks, int(Pp / kGrain));
+    L.chunk = int((Pp / kGrain + L.nchunk - 1) / L.nchunk * kGrain);
     if (tu.a_chunk > 0) L.chunk = int(std::min<size_t>(Pp, size_t(std::max(2 * TP, tu.a_chunk / TP * TP))));
     L.nchunk = int((Pp + L.chunk - 1) / L.chunk);
     L.apart = n * M * size_t(L.nchunk) * SP2;
@@ -560,7 +590,8 @@ static WsLayout ws_layout(size_t n, size_t NI, size_t Pp, int M, int K, int nmod
     L.gdir = size_t(std::max(ndirs, 1)) * nmod * SP2;
     L.out = 2 + n + 2 * size_t(nmod) + M;
     L.part = part_nodes * M * SP * Pp;
-    L.vf = vf_nodes * M * SP * Pp;
+    // gradient operands: the FP64 path keeps those of internal branches, in the partials' slots
+    L.vf = precision == H3G_PREC_MIXED ? vf_nodes * M * SP * Pp : L.part;
     return L;
 }
 
@@ -658,9 +689,11 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
     const h3g::CkPlan& pl = pr->ck_plan;
     const int n = pr->n;
     const auto kids = children_of(pr);
-    std::vector<int> n_int(n, 0);
-    for (int u = 0; u < n; ++u)
+    std::vector<int> n_int(n, 0), n_kids(n, 0);
+    for (int u = 0; u < n; ++u) {
+        n_kids[u] = int(kids[u].size());
         for (int c : kids[u]) n_int[u] += pr->leaf[c] ? 0 : 1;
+    }
     std::vector<int2> kdesc(std::max<size_t>(pr->ch.size(), 1));
     for (size_t j = 0; j < pr->ch.size(); ++j) {
         const int c = pr->ch[j];
@@ -674,8 +707,11 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
         h3g_problem::CkOffsets o{};
         o.in = int(lists.size());
         lists.insert(lists.end(), B.in_nodes.begin(), B.in_nodes.end());
+        std::vector<int> split;
+        split_kids(B.out_kids, B.out_lv, pr->leaf.data(), pr->parent_h.data(), n_kids, split, o.out_int_off, o.pairs_at, o.n_pairs);
+        if (lists.size() % 2) lists.push_back(-1);              // the pairs are read as int2
         o.out = int(lists.size());
-        lists.insert(lists.end(), B.out_kids.begin(), B.out_kids.end());
+        lists.insert(lists.end(), split.begin(), split.end());
         o.acc = int(lists.size());
         lists.insert(lists.end(), B.acc.begin(), B.acc.end());
         // inside items
@@ -757,7 +793,7 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
 // no block size is forced; else the plan with the largest block size whose layout fits.
 static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndirs, const h3g_tuning& tu, uint64_t held,
                                 WsLayout& L) {
-    const WsLayout full = ws_layout(size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu);
+    const WsLayout full = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu);
     pr->full_bytes = ws_bytes(full, pr->precision);
     uint64_t budget = pr->mem_budget;
     if (!budget) {
@@ -775,7 +811,7 @@ static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndi
         return h3g::plan_checkpoints(pr->n, pr->root, kids, pr->leaf.data(), pr->bfs_order, pr->depth_h, pr->height_h, target);
     };
     auto layout_of = [&](const h3g::CkPlan& p) {
-        return ws_layout(size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu, size_t(p.ncp + p.scratch_int),
+        return ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu, size_t(p.ncp + p.scratch_int),
                          size_t(p.ncp + p.scratch_all));
     };
     if (pr->ck_target_req > 0) {
@@ -1086,14 +1122,16 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
         if (mixed) {
             l = launch_outside_mixed(t, md, w, mwk, pr->n_out_heads, pr->wait, s);
         } else {
-            for (size_t lv = 0; lv + 1 < pr->out_off.size(); ++lv) {
-                const int cnt = pr->out_off[lv + 1] - pr->out_off[lv];
+            for (size_t lv = 0; lv + 1 < pr->out_int_off.size(); ++lv) {
+                const int cnt = pr->out_int_off[lv + 1] - pr->out_int_off[lv];
                 if (!cnt) continue;
-                l += launch_outside_fp64(t, md, w, pr->d_out_nodes + pr->out_off[lv], cnt, 1, s);
+                l += launch_outside_fp64(t, md, w, pr->d_out_split + pr->out_int_off[lv], cnt, s);
             }
         }
         mark(ST_OUTSIDE, l);
-        mark(ST_ACCUM_A, mixed ? launch_accumA_mixed(t, md, w, mwk, nullptr, 0, s) : launch_accumA_fp64(t, md, w, nullptr, 0, s));
+        mark(ST_ACCUM_A, mixed ? launch_accumA_mixed(t, md, w, mwk, nullptr, 0, s)
+                               : launch_accumA_fp64(t, md, w, pr->d_out_split, pr->out_int_off.back(),
+                                                    reinterpret_cast<const int2*>(pr->d_out_split + pr->pairs_at), pr->n_pairs, s));
         mark(ST_FRECHET, launch_frechet(t, md, w, global ? 1 : 0, s));
         if (side) cudaStreamWaitEvent(s, pr->ev_join, 0);
         if (global) mark(ST_HSUM, launch_global(t, md, w, s));
@@ -1172,9 +1210,12 @@ static int enqueue_eval_ck(h3g_problem* pr, unsigned want, bool from_given_P, cu
                 l += launch_outside_mixed(tb, md, w, mwk, o.n_out_heads, pr->wait, s);
                 if (!B.acc.empty()) l += launch_accumA_mixed(t, md, w, mwk, lists + o.acc, int(B.acc.size()), s);
             } else {
-                for (size_t lv = 0; lv + 1 < B.out_lv.size(); ++lv)
-                    l += launch_outside_fp64(t, md, w, lists + o.out + B.out_lv[lv], B.out_lv[lv + 1] - B.out_lv[lv], 1, s);
-                if (!B.acc.empty()) l += launch_accumA_fp64(t, md, w, lists + o.acc, int(B.acc.size()), s);
+                for (size_t lv = 0; lv + 1 < o.out_int_off.size(); ++lv)
+                    if (const int cnt = o.out_int_off[lv + 1] - o.out_int_off[lv])
+                        l += launch_outside_fp64(t, md, w, lists + o.out + o.out_int_off[lv], cnt, s);
+                // the branches below this block's nodes: V or the parents' U and the siblings' messages, and their own D, are here
+                l += launch_accumA_fp64(t, md, w, lists + o.out, o.out_int_off.back(),
+                                        reinterpret_cast<const int2*>(lists + o.out + o.pairs_at), o.n_pairs, s);
             }
         }
         mark(ST_OUTSIDE, l);
@@ -1369,7 +1410,7 @@ extern "C" h3g_status h3g_problem_set_tuning(h3g_problem* pr, const h3g_tuning* 
 
 extern "C" h3g_status h3g_problem_get_tuning(const h3g_problem* pr, h3g_tuning* tu) {
     if (!pr || !tu) return H3G_ERR_ARG;
-    const WsLayout L = ws_layout(size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), std::max(pr->M, 1), pr->K,
+    const WsLayout L = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), std::max(pr->M, 1), pr->K,
                                  std::max(pr->nmod, 1), pr->ndirs, effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
     tu->a_chunk = L.chunk;
     tu->ctas_per_sm = pr->wait.ctas_per_sm;
@@ -1404,7 +1445,7 @@ extern "C" h3g_status h3g_autotune(h3g_problem* pr, const double* bl, unsigned w
         *ms = tot / reps;
         return H3G_OK;
     };
-    const WsLayout L0 = ws_layout(size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs, h3g_tuning{});
+    const WsLayout L0 = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs, h3g_tuning{});
     h3g_tuning cur{L0.chunk, 2, L0.ngroups};
     double cur_ms = 0.0;
     if (h3g_status st = measure(cur, &cur_ms); st != H3G_OK) return st;
@@ -1779,7 +1820,7 @@ static h3g_status batch_prepare(h3g_batch* b) {
     std::vector<WsLayout> lay(G);
     for (int g = 0; g < G; ++g) {
         const h3g_problem* pr = b->probs[g];
-        lay[g] = ws_layout(size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs,
+        lay[g] = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs,
                            effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
     }
     const bool first = b->slots[0]->genes.empty() && b->slots[0]->w.P == nullptr;

@@ -10,8 +10,8 @@
 //                                           a warp reading one state of 32
 //                                           consecutive patterns is coalesced
 //   Ecum, Eown         [NI][M][Pp]          power-of-two scaling exponents
-//   Vf                 [n][M][64][Pp]       outside vector at the top of each branch
-//                                           times w_p * posterior_m / L_m
+//   Vf                 [n][M][64][Pp]       outside vector at the top of each branch times
+//                                           w_p * posterior_m / L_m (FP64 path: [NI], internal branches only)
 // Leaves never get a partial: their message P_b * leaf_vector is a column of P_b
 // (a row of PT_b), a masked column sum, or the P_b row sums for missing data.
 #pragma once
@@ -116,7 +116,7 @@ struct Work {
     double* U;               // [NI][M][64][Pp]
     int* Ecum;               // [NI][M][Pp]
     int* Eown;               // [NI][M][Pp]
-    double* Vf;              // [n][M][64][Pp]
+    double* Vf;              // [NI][M][64][Pp] f V of the internal branches (FP64 path)
     double* f;               // [M][Pp]   w_p * post_{m,p} / L_{m,p}
     double* contrib;         // [Pp]      this pattern's term of lnL
     double* site;            // [Pp]      per-pattern lnL

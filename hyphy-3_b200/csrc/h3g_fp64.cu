@@ -15,6 +15,8 @@
 //                  (likelihood.hpp:1428-1471)
 //   k_hsum, k_dir, k_small   fixed-order reductions -> lnL, gradients
 // All reductions run in a fixed order, so repeated evaluations are bit-identical.
+#include <algorithm>
+#include <climits>
 #include <cstdlib>
 #include "h3g_common.cuh"
 #include "h3g_kernels.h"
@@ -22,45 +24,6 @@
 #include "h3g_tc.cuh"
 
 namespace h3g {
-
-__device__ __forceinline__ int renorm64(double (&v)[SP]) {
-    double mx = 0.0;
-#pragma unroll
-    for (int i = 0; i < SP; ++i) mx = fmax(mx, v[i]);
-    if (mx > 0.0 && mx < 0x1p-256) {
-        const int sh = -ilogb(mx) - 1;    // brings the max into [0.5, 1)
-#pragma unroll
-        for (int i = 0; i < SP; ++i) v[i] = ldexp(v[i], sh);
-        return sh;
-    }
-    return 0;
-}
-
-// v *= P_c * leaf_vector(c, p): a column of P_c, a masked column sum or the row sums.
-__device__ __forceinline__ void mul_leaf_msg(double (&v)[SP], const Topo& t, const Work& w, int m, int c, int p) {
-    const int tx = t.taxon[c];
-    const double* PTc = w.PT + mat_off(m, c, t.n);
-    const int st = tx < 0 ? -1 : int(t.states[size_t(tx) * t.Pp + p]);
-    if (st >= 0) {
-        const double2* r = reinterpret_cast<const double2*>(PTc + st * SP);
-#pragma unroll
-        for (int i = 0; i < SP / 2; ++i) { double2 x = __ldg(r + i); v[2 * i] *= x.x; v[2 * i + 1] *= x.y; }
-        return;
-    }
-    const uint64_t mk = tx < 0 ? t.all_mask : t.masks[size_t(tx) * t.Pp + p];
-    if (mk == 0 || (mk & t.all_mask) == t.all_mask) {
-        const double2* r = reinterpret_cast<const double2*>(w.rs + (size_t(m) * t.n + c) * SP);
-#pragma unroll
-        for (int i = 0; i < SP / 2; ++i) { double2 x = __ldg(r + i); v[2 * i] *= x.x; v[2 * i + 1] *= x.y; }
-        return;
-    }
-#pragma unroll
-    for (int i = 0; i < SP; ++i) {
-        double s = 0.0;
-        for (uint64_t b = mk; b; b &= b - 1) s += __ldg(PTc + (__ffsll((long long)b) - 1) * SP + i);
-        v[i] *= s;
-    }
-}
 
 __device__ __forceinline__ void stage_matrix(double* __restrict__ s, const double* __restrict__ g, int tid, int nthr) {
     const double2* g2 = reinterpret_cast<const double2*>(g);
@@ -135,6 +98,7 @@ __global__ void __launch_bounds__(256) k_build_P(Topo t, Model md, Work w, Mixed
     double* sX = sm;                 // U_k diag(e), then Q_k
     double* sY = sm + SP * LDM;      // V_k, then clamp(P_k)
     __shared__ double se[SP];
+    __shared__ double srow[2][SP];
     const int b = blockIdx.x, m = blockIdx.y, tid = threadIdx.x;
     if (kMixed && b == 0 && m == 0 && tid == 0) {        // a new evaluation: new epoch, fresh item counters
         mw.sync[0] += 1;
@@ -204,6 +168,18 @@ __global__ void __launch_bounds__(256) k_build_P(Topo t, Model md, Work w, Mixed
                 w.PT[o + c * SP + r] = accP.v[i][j][0];
                 w.PT[o + (c + 1) * SP + r] = accP.v[i][j][1];
             }
+        // row sums (the message of a leaf without data): the four lanes of a row, then its two column halves
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            double rs = 0.0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) rs += accP.v[i][j][0] + accP.v[i][j][1];
+            rs += __shfl_xor_sync(0xffffffffu, rs, 1);
+            rs += __shfl_xor_sync(0xffffffffu, rs, 2);
+            if ((tid & 3) == 0) srow[(tid >> 5) & 1][frag_row(i)] = rs;
+        }
+        __syncthreads();
+        if (tid < SP) w.rs[(size_t(m) * t.n + b) * SP + tid] = srow[0][tid] + srow[1][tid];
     } else {
         __syncthreads();                          // every warp is done reading sX (Q) and sY
 #pragma unroll
@@ -251,17 +227,6 @@ __global__ void __launch_bounds__(256) k_build_P(Topo t, Model md, Work w, Mixed
     }
 }
 
-// Row sums of P_{m,b} (the message of a leaf with missing data).  grid (n, M), block 64.
-__global__ void k_rowsum(Topo t, Model md, Work w) {
-    pdl_enter();
-    const int b = blockIdx.x, m = blockIdx.y, r = threadIdx.x;
-    if (b == t.root) return;
-    const double* PT = w.PT + mat_off(m, b, t.n) + r;
-    double s = 0.0;
-    for (int j = 0; j < SP; ++j) s += PT[j * SP];     // sum_j P[r][j], read along PT rows
-    w.rs[(size_t(m) * t.n + b) * SP + r] = s;
-}
-
 // Caller-supplied P (compute_tree_log_likelihood_from_P): derive PT and row sums.
 __global__ void k_prep_given_P(Topo t, Work w) {
     pdl_enter();
@@ -280,34 +245,44 @@ __global__ void k_prep_given_P(Topo t, Work w) {
 // ------------------------------------------------------------------- inside
 // CTA = 8 warps x 32 patterns; warp g owns states [8g, 8g+8) of its 32 patterns
 // (lane = pattern), so every global access of a partial is a coalesced 256-byte row.
-constexpr int kTileP = 32;      // patterns per CTA in the FP64 pruning kernels
+constexpr int kTileP = 32;      // patterns per tile in the FP64 pruning kernels
 constexpr int kGroups = 8;      // state groups (warps) per CTA
 
-// v[q] *= message of leaf child c for states [8g, 8g+8) of pattern p.
-__device__ __forceinline__ void mul_leaf8(double (&v)[8], const Topo& t, const Work& w, int m, int c, int p, int g) {
-    const int tx = t.taxon[c];
-    const double* PTc = w.PT + mat_off(m, c, t.n);
-    const int st = tx < 0 ? -1 : int(t.states[size_t(tx) * t.Pp + p]);
-    const double* src;
-    if (st >= 0) {
-        src = PTc + st * SP + 8 * g;
-    } else {
-        const uint64_t mk = tx < 0 ? t.all_mask : t.masks[size_t(tx) * t.Pp + p];
+// The observed state of a child at pattern p (its sense index, or -1; 0 for an internal child, which has none).
+__device__ __forceinline__ int child_state(const Topo& t, int2 d, int p) {
+    if (d.y <= -2) return 0;
+    return d.y < 0 ? -1 : int(t.states[size_t(d.y) * t.Pp + p]);
+}
+// A child's message for states [8g, 8g+8) of pattern p: the stored message of an internal child; for a leaf in
+// state st >= 0 a column of P else the row sums or a masked column sum.
+// d: Topo::kdesc entry.
+__device__ __forceinline__ void load_msg8(double (&a)[8], const Topo& t, const Work& w, int m, int M, int2 d, int p, int g, int st) {
+    if (d.y <= -2) {
+        const double* src = w.Ms + part_off(-(d.y + 2), m, M, t.Pp) + size_t(8 * g) * t.Pp + p;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) a[q] = src[size_t(q) * t.Pp];
+        return;
+    }
+    const double* PTc = w.PT + mat_off(m, d.x, t.n);
+    const double* src = PTc + st * SP + 8 * g;
+    if (st < 0) {
+        const uint64_t mk = d.y < 0 ? t.all_mask : t.masks[size_t(d.y) * t.Pp + p];
         if (mk == 0 || (mk & t.all_mask) == t.all_mask) {
-            src = w.rs + (size_t(m) * t.n + c) * SP + 8 * g;
+            src = w.rs + (size_t(m) * t.n + d.x) * SP + 8 * g;
         } else {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                double s = 0.0;
-                for (uint64_t b = mk; b; b &= b - 1) s += __ldg(PTc + (__ffsll((long long)b) - 1) * SP + 8 * g + q);
-                v[q] *= s;
+            for (int q = 0; q < 8; ++q) a[q] = 0.0;
+            for (uint64_t b = mk; b; b &= b - 1) {
+                const double* col = PTc + (__ffsll((long long)b) - 1) * SP + 8 * g;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) a[q] += __ldg(col + q);
             }
             return;
         }
     }
     const double2* s2 = reinterpret_cast<const double2*>(src);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { const double2 x = __ldg(s2 + q); v[2 * q] *= x.x; v[2 * q + 1] *= x.y; }
+    for (int q = 0; q < 4; ++q) { const double2 x = __ldg(s2 + q); a[2 * q] = x.x; a[2 * q + 1] = x.y; }
 }
 
 // Power-of-two renormalisation of a 64-state column spread over the 8 warps:
@@ -330,6 +305,18 @@ __device__ __forceinline__ int renorm_cols(double (&v)[8], double* smax, int g, 
     }
     return 0;
 }
+// The same unless every thread's eight states reach 2^-340: one barrier instead of the exchange.  A column is then
+// left with a maximum of 2^-340 at least; the product of two such stays far from the end of the range, and
+// scaling by powers of two changes no result.  (At 2^-256, the bound of the exchange itself, states 60 powers of
+// two below their column's maximum sent most tiles through it.)  Doubles >= 0 compare like the integers of their
+// upper words.  S: states; a group beyond them does not count.
+__device__ __forceinline__ int renorm_if_small(double (&v)[8], double* smax, int g, int lane, int S) {
+    int hi = 8 * g >= S ? INT_MAX : 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) hi = max(hi, __double2hiint(v[q]));
+    if (__syncthreads_and(hi >= ((1023 - 340) << 20))) return 0;
+    return renorm_cols(v, smax, g, lane);
+}
 
 // Partial tiles of the FP64 pruning CTAs in shared memory: [64 states][32 patterns] with a row
 // stride of kDL = 36 doubles, so the B-fragment loads (k + lane%4) * 36 + col + lane/4 of a half-warp
@@ -341,86 +328,106 @@ __device__ __forceinline__ void cp_async16_f64(double* dst, const double* src) {
                  ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
 }
 
-// Stage a 64x64 matrix row-major with the padded stride LDM (k_build_P's operand layout) by 16-byte
-// cp.async, one commit group: the copy runs while the CTA loads and multiplies its partials;
-// stage_wait() before the product reads it.
-__device__ __forceinline__ void stage_matrix_pad_async(double* __restrict__ s, const double* __restrict__ g, int tid, int nthr) {
-    for (int e = tid; e < SP2 / 2; e += nthr) {
-        const int r = e / (SP / 2), c2 = e % (SP / 2);
-        cp_async16_f64(s + r * LDM + 2 * c2, g + 2 * e);
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+// A warp's rows 8g .. 8g+7 of a 64x64 matrix as the A fragments of 16 m8n8k4 products: 16 doubles a thread.
+struct RowFrags { double a[SP / 4]; };
+__device__ __forceinline__ RowFrags load_rows(const double* __restrict__ mat) {
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const double* row = mat + (8 * wp + (lane >> 2)) * SP + (lane & 3);
+    RowFrags f;
+#pragma unroll
+    for (int k = 0; k < SP / 4; ++k) f.a[k] = __ldg(row + 4 * k);
+    return f;
 }
-__device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// dst[i][p] = sum_k sM[i][k] sX[k][p] for the CTA's 64 x 32 tile on the FP64 tensor cores
-// (mma.sync m8n8k4): warp w owns output rows 8w .. 8w+7, all 32 columns as four 8x8 tiles,
-// 16 k steps of 4.  sM [64][LDM] row-major, sX [64][kDL]; dst has row stride `stride`
+// dst[i][p] = sum_k M[i][k] sX[k][p] for the CTA's 64 x 32 tile on the FP64 tensor cores
+// (mma.sync m8n8k4): warp w owns output rows 8w .. 8w+7 (f), all 32 columns as four 8x8 tiles,
+// 16 k steps of 4.  sX [64][kDL]; dst has row stride `stride`
 // (state-major partials), each thread storing two adjacent patterns as one 16-byte write.
-__device__ __forceinline__ void tile_mm_store(const double* __restrict__ sM, const double* __restrict__ sX,
-                                              double* __restrict__ dst, size_t stride) {
+__device__ __forceinline__ void tile_mm_store(const RowFrags& f, const double* __restrict__ sX, double* __restrict__ dst, size_t stride) {
     const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, g = lane >> 2, q = lane & 3;
     double c[4][2];
 #pragma unroll
     for (int j = 0; j < 4; ++j) c[j][0] = c[j][1] = 0.0;
-    const double* arow = sM + (8 * wp + g) * LDM + q;
-#pragma unroll 4
-    for (int k = 0; k < SP; k += 4) {
-        const double a = arow[k];
-        const double* brow = sX + (k + q) * kDL + g;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) dmma(c[j][0], c[j][1], a, brow[8 * j]);
+    for (int k = 0; k < SP / 4; ++k) {
+        const double* brow = sX + (4 * k + q) * kDL + g;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dmma(c[j][0], c[j][1], f.a[k], brow[8 * j]);
     }
     double* d = dst + size_t(8 * wp + g) * stride + 2 * q;
 #pragma unroll
     for (int j = 0; j < 4; ++j) *reinterpret_cast<double2*>(d + 8 * j) = make_double2(c[j][0], c[j][1]);
 }
 
-// grid (Pp/32, nodes in level, M), block 256, dynamic smem (64*LDM + 64*kDL + 8*32) doubles.
-__global__ void __launch_bounds__(256) k_inside(Topo t, Model md, Work w, const int* __restrict__ nodes) {
+// grid (ceil(Pp/32 / tiles), nodes in level, M), block 256: `tiles` pattern tiles of one node and class.  The
+// node's matrix stays in registers as fragments for all of them, the next tile's first two messages (and the
+// observed states after that) are loaded while this one multiplies, and the rescaling is one vote unless a tile needs it.
+// A tile takes about 4600 cycles of an SM, 2048 of them products: the rest is 2500-3600 wavefronts of the L1 (1050
+// for each leaf's gathered columns of P, 1024 for the products' B fragments).  1024 taxa x 1200 codons x 4 rates:
+// 2.65 ms for all levels; a CTA per tile with the matrix in shared memory and a rescaling exchange per child: 3.40 ms.
+// Tried and slower: leaves' matrices staged in shared memory (2.92), columns fetched by cp.async two tiles ahead
+// (3.09), whole rows of P^T fetched for leaves (2.93).
+__global__ void __launch_bounds__(256, 2) k_inside(Topo t, Model md, Work w, const int* __restrict__ nodes, int tiles) {
     pdl_enter();
-    extern __shared__ __align__(16) double sm[];
-    double* sP = sm;                     // P_u row-major [64][LDM]
-    double* sD = sm + SP * LDM;          // D_u tile [64][kDL]
-    double* smax = sD + SP * kDL;        // [8][32]
+    __shared__ __align__(16) double sD[SP * kDL];
+    __shared__ double smax[kGroups * kTileP];
     const int u = nodes[blockIdx.y], m = blockIdx.z, tid = threadIdx.x;
     const int g = tid >> 5, lane = tid & 31;
-    const int p = blockIdx.x * kTileP + lane;
+    const int k0 = t.ch_off[u], k1 = t.ch_off[u + 1];
     const int iu = t.iidx[u], M = md.M;
     const size_t Pp = size_t(t.Pp);
-    const bool root = (u == t.root);
-    if (!root) stage_matrix_pad_async(sP, w.P + mat_off(m, u, t.n), tid, 256);
-    double v[8];
+    const bool root = (u == t.root), one = k0 < k1, two = k0 + 1 < k1;
+    const int t0 = blockIdx.x * tiles, t1 = min(t0 + tiles, t.Pp / kTileP);
+    const int2 d0 = one ? t.kdesc[k0] : make_int2(0, -1), d1 = two ? t.kdesc[k0 + 1] : d0;
+    double a0[8], a1[8];
+    int p = t0 * kTileP + lane;
+    int s0 = child_state(t, d0, p), s1 = child_state(t, d1, p);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = (8 * g + q) < t.S ? 1.0 : 0.0;
-    int ecum = 0, eown = 0;
-    for (int k = t.ch_off[u]; k < t.ch_off[u + 1]; ++k) {
-        const int c = t.ch[k];
-        if (t.leaf[c]) {
-            mul_leaf8(v, t, w, m, c, p, g);
-        } else {
-            const int ic = t.iidx[c];
-            const double* src = w.Ms + part_off(ic, m, M, t.Pp) + size_t(8 * g) * Pp + p;
+    for (int q = 0; q < 8; ++q) a0[q] = 8 * g + q < t.S ? 1.0 : 0.0;      // a node without children
+    if (one) load_msg8(a0, t, w, m, M, d0, p, g, s0);
+    if (two) load_msg8(a1, t, w, m, M, d1, p, g, s1);
+    RowFrags f;
+    if (!root) f = load_rows(w.P + mat_off(m, u, t.n));
+    int n0 = 0, n1 = 0;                                            // the next tile's states
+    if (t0 + 1 < t1) { n0 = child_state(t, d0, p + kTileP); n1 = child_state(t, d1, p + kTileP); }
+    for (int tile = t0; tile < t1; ++tile, p += kTileP) {
+        double v[8];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] *= src[q * Pp];
-            ecum += w.Ecum[col_off(ic, m, M, t.Pp) + p];
+        for (int q = 0; q < 8; ++q) v[q] = two ? a0[q] * a1[q] : a0[q];
+        int eown = renorm_if_small(v, smax, g, lane, t.S);  // (its barrier: the last tile's products are done with sD)
+        for (int k = k0 + 2; k < k1; ++k) {
+            const int2 d = t.kdesc[k];
+            double x[8];
+            load_msg8(x, t, w, m, M, d, p, g, child_state(t, d, p));
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] *= x[q];
+            eown += renorm_if_small(v, smax, g, lane, t.S);
         }
-        eown += renorm_cols(v, smax, g, lane);
-    }
-    double* dst = w.D + part_off(iu, m, M, t.Pp) + size_t(8 * g) * Pp + p;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) dst[q * Pp] = v[q];
-    if (g == 0) {
-        w.Eown[col_off(iu, m, M, t.Pp) + p] = eown;
-        w.Ecum[col_off(iu, m, M, t.Pp) + p] = ecum + eown;
-    }
-    if (root) return;
+        for (int q = 0; q < 8; ++q) sD[(8 * g + q) * kDL + lane] = v[q];
+        double* dst = w.D + part_off(iu, m, M, t.Pp) + size_t(8 * g) * Pp + p;
 #pragma unroll
-    for (int q = 0; q < 8; ++q) sD[(8 * g + q) * kDL + lane] = v[q];
-    stage_wait();
-    __syncthreads();
-    // message to the parent: (P_u D_u)_i = sum_j P[i][j] D_j
-    tile_mm_store(sP, sD, w.Ms + part_off(iu, m, M, t.Pp) + size_t(blockIdx.x) * kTileP, Pp);
+        for (int q = 0; q < 8; ++q) dst[q * Pp] = v[q];
+        if (g == 0) {
+            int ecum = eown;
+            for (int k = k0; k < k1; ++k) {
+                const int code = t.kdesc[k].y;
+                if (code <= -2) ecum += w.Ecum[col_off(-(code + 2), m, M, t.Pp) + p];
+            }
+            w.Eown[col_off(iu, m, M, t.Pp) + p] = eown;
+            w.Ecum[col_off(iu, m, M, t.Pp) + p] = ecum;
+        }
+        if (tile + 1 < t1) {
+            s0 = n0;
+            s1 = n1;
+            if (one) load_msg8(a0, t, w, m, M, d0, p + kTileP, g, s0);
+            if (two) load_msg8(a1, t, w, m, M, d1, p + kTileP, g, s1);
+            if (tile + 2 < t1) { n0 = child_state(t, d0, p + 2 * kTileP); n1 = child_state(t, d1, p + 2 * kTileP); }
+        }
+        __syncthreads();
+        // message to the parent: (P_u D_u)_i = sum_j P[i][j] D_j
+        if (!root) tile_mm_store(f, sD, w.Ms + part_off(iu, m, M, t.Pp) + size_t(tile) * kTileP, Pp);
+    }
 }
 
 // --------------------------------------------------------------------- root
@@ -470,122 +477,113 @@ __global__ void k_root(Topo t, Model md, Work w) {
 }
 
 // ------------------------------------------------------------------ outside
-// One CTA per (child c of a node at this depth, 32-pattern tile, rate class):
-// V_c = 2^{e_u} U_u o prod_{s != c} (P_s D_s), then U_c = P_c^T V_c for internal c.
-// grid (Pp/32, children in level, M), block 256, dynamic smem (64*64 + 64*32 + 8*32) doubles.
-__global__ void __launch_bounds__(256) k_outside(Topo t, Model md, Work w, const int* __restrict__ kids, int want_v) {
+// The outside partials of the internal children of one depth's nodes: with u the parent of c,
+// V_c = 2^{e_u} U_u o prod_{s != c} (P_s D_s), U_c = P_c^T V_c, and f V_c for the gradient.  grid and tiles as
+// k_inside, `kids` the children.  Leaves have no outside partial, and their V is formed where the gradient uses
+// it (k_accumA_leaf): storing it for them was half of this kernel's CTAs and the gradient's largest stream
+// (1024 taxa x 1200 codons x 4 rates: 4.87 -> 2.81 ms).
+__global__ void __launch_bounds__(256, 2) k_outside(Topo t, Model md, Work w, const int* __restrict__ kids, int tiles) {
     pdl_enter();
-    extern __shared__ __align__(16) double sm[];
-    double* sPT = sm;                    // P_c^T row-major [64][LDM]
-    double* sV = sm + SP * LDM;          // V_c tile [64][kDL]
-    double* smax = sV + SP * kDL;
-    const int c = kids[blockIdx.y], m = blockIdx.z, tid = threadIdx.x;
-    const int g = tid >> 5, lane = tid & 31;
-    const int p = blockIdx.x * kTileP + lane;
-    const int u = t.parent[c], iu = t.iidx[u], M = md.M;
+    __shared__ __align__(16) double sV[SP * kDL];
+    __shared__ double smax[kGroups * kTileP];
+    const int c = kids[blockIdx.y], m = blockIdx.z, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int u = t.parent[c], iu = t.iidx[u], ic = t.iidx[c], M = md.M;
+    const int k0 = t.ch_off[u], k1 = t.ch_off[u + 1];
     const size_t Pp = size_t(t.Pp);
-    const bool internal = !t.leaf[c];
-    if (internal) stage_matrix_pad_async(sPT, w.PT + mat_off(m, c, t.n), tid, 256);
-    double v[8];
-    if (u == t.root) {
+    const bool at_root = u == t.root;
+    const int ks = t.kdesc[k0].x == c ? k0 + 1 : k0;              // the first sibling
+    const bool sib = ks < k1, more = k1 - k0 > 2;
+    const int2 ds = sib ? t.kdesc[ks] : make_int2(0, -1);
+    const int* eo = w.Eown + col_off(iu, m, M, t.Pp);
+    const double* fp = w.f + size_t(m) * Pp;
+    const int t0 = blockIdx.x * tiles, t1 = min(t0 + tiles, t.Pp / kTileP);
+    const size_t oc = part_off(ic, m, M, t.Pp), ou = part_off(at_root ? ic : iu, m, M, t.Pp);
+    auto load_u = [&](double (&a)[8], int p) {
+        const double* src = w.U + ou + size_t(8 * g) * Pp + p;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = md.pi[8 * g + q];
-    } else {
-        const double* src = w.U + part_off(iu, m, M, t.Pp) + size_t(8 * g) * Pp + p;
+        for (int q = 0; q < 8; ++q) a[q] = at_root ? md.pi[8 * g + q] : src[q * Pp];
+    };
+    double a[8], b[8];
+    int p = t0 * kTileP + lane;
+    int st = child_state(t, ds, p), nx = 0, e = eo[p];
+    double f = fp[p];
+    load_u(a, p);
+    if (sib) load_msg8(b, t, w, m, M, ds, p, g, st);
+    const RowFrags fr = load_rows(w.PT + mat_off(m, c, t.n));
+    if (t0 + 1 < t1) nx = child_state(t, ds, p + kTileP);
+    for (int tile = t0; tile < t1; ++tile, p += kTileP) {
+        double v[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = src[q * Pp];
-    }
-    int ev = w.Eown[col_off(iu, m, M, t.Pp) + p];
-    for (int k = t.ch_off[u]; k < t.ch_off[u + 1]; ++k) {
-        const int s = t.ch[k];
-        if (s == c) continue;
-        if (t.leaf[s]) {
-            mul_leaf8(v, t, w, m, s, p, g);
-        } else {
-            const double* src = w.Ms + part_off(t.iidx[s], m, M, t.Pp) + size_t(8 * g) * Pp + p;
+        for (int q = 0; q < 8; ++q) v[q] = sib ? a[q] * b[q] : a[q];
+        int ev = e - renorm_if_small(v, smax, g, lane, t.S);      // (its barrier: the last tile's products are done with sV)
+        if (more)
+            for (int k = ks + 1; k < k1; ++k) {
+                const int2 d = t.kdesc[k];
+                if (d.x == c) continue;
+                double x[8];
+                load_msg8(x, t, w, m, M, d, p, g, child_state(t, d, p));
 #pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] *= src[q * Pp];
+                for (int q = 0; q < 8; ++q) v[q] *= x[q];
+                ev -= renorm_if_small(v, smax, g, lane, t.S);
+            }
+        if (ev != 0) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = ldexp(v[q], ev);
         }
-        ev -= renorm_cols(v, smax, g, lane);
-    }
-    if (ev != 0) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = ldexp(v[q], ev);
-    }
-    if (want_v) {
-        const double fp = w.f[size_t(m) * Pp + p];
-        double* dst = w.Vf + part_off(vslot(t, c), m, M, t.Pp) + size_t(8 * g) * Pp + p;
+        for (int q = 0; q < 8; ++q) sV[(8 * g + q) * kDL + lane] = v[q];
+        double* vf = w.Vf + oc + size_t(8 * g) * Pp + p;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) dst[q * Pp] = fp * v[q];
+        for (int q = 0; q < 8; ++q) vf[q * Pp] = f * v[q];
+        if (tile + 1 < t1) {
+            st = nx;
+            load_u(a, p + kTileP);
+            if (sib) load_msg8(b, t, w, m, M, ds, p + kTileP, g, st);
+            e = eo[p + kTileP];
+            f = fp[p + kTileP];
+            if (tile + 2 < t1) nx = child_state(t, ds, p + 2 * kTileP);
+        }
+        __syncthreads();
+        tile_mm_store(fr, sV, w.U + oc + size_t(tile) * kTileP, Pp);       // (U_c)_i = sum_j PT[i][j] V_j
     }
-    if (!internal) return;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) sV[(8 * g + q) * kDL + lane] = v[q];
-    stage_wait();
-    __syncthreads();
-    // U_c = P_c^T V_c : (U_c)_i = sum_j PT[i][j] V_j
-    tile_mm_store(sPT, sV, w.U + part_off(t.iidx[c], m, M, t.Pp) + size_t(blockIdx.x) * kTileP, Pp);
 }
 
 // ------------------------------------------------------------------ accum A
-// A_{m,b,chunk} = sum_{p in chunk} Vf_b[:, p] D_b[:, p]^T on the FP64 tensor cores: C = X Y^T with
-// X = Vf (64 states x patterns), Y = D, K = the pattern axis.  8 warps as mm64 (warp w: rows
-// 16(w/2) .. +16, columns 32(w%2) .. +32, 2 x 4 tiles of 8x8), 32 patterns per stage, stages
-// double-buffered by 16-byte cp.async (a leaf's 0/1 vectors are written from its states and
-// masks instead).  grid (branches, M, nchunk), block 256; `branches` lists the branches (NULL: every
-// node id, the root skipped).
+// A_{m,b,chunk} = sum_{p in chunk} f V_b[:, p] D_b[:, p]^T.
+//
+// Internal branches on the FP64 tensor cores: C = X Y^T with X = f V (64 states x patterns), Y = D, K = the pattern
+// axis.  8 warps as mm64 (warp w: rows 16(w/2) .. +16, columns 32(w%2) .. +32, 2 x 4 tiles of 8x8), 32 patterns
+// per stage, stages double-buffered by 16-byte cp.async.  grid (branches, M, nchunk), block 256.
 constexpr int kAccP = 32;                                      // patterns per stage
 constexpr int kAL = kAccP + 4;                                 // row stride of a staged tile (doubles)
 constexpr size_t kAccStage = size_t(2) * SP * kAL;             // V and D tiles of one stage
-static const size_t kAccSmemF = 2 * kAccStage * sizeof(double);
+static const size_t kAccIntSmem = 2 * kAccStage * sizeof(double);
 
-__global__ void __launch_bounds__(256) k_accumA(Topo t, Model md, Work w, const int* __restrict__ branches) {
+__global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, const int* __restrict__ branches) {
     pdl_enter();
     extern __shared__ __align__(16) double smA[];
-    const int b = branches ? branches[blockIdx.x] : int(blockIdx.x), m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x;
-    if (b == t.root) return;
-    const int M = md.M;
+    const int b = branches[blockIdx.x], m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
     const size_t Pp = size_t(t.Pp);
-    const int p_begin = ck * w.chunk, p_end = min(t.Pp, p_begin + w.chunk);
-    const int nst = (p_end - p_begin) / kAccP;
-    const bool lf = t.leaf[b];
-    const int tx = lf ? t.taxon[b] : -1;
-    const double* Vb = w.Vf + part_off(vslot(t, b), m, M, t.Pp);
-    const double* Db = lf ? nullptr : w.D + part_off(t.iidx[b], m, M, t.Pp);
-
-    // stage `st` of the chunk into buffer st & 1: 64 state rows x 32 patterns of Vf (and D)
+    const int p_begin = ck * w.chunk, nst = (min(t.Pp, p_begin + w.chunk) - p_begin) / kAccP;
+    const size_t o = part_off(t.iidx[b], m, M, t.Pp) + p_begin;
+    // 64 state rows x 32 patterns of Vf and D into buffer st & 1
     auto stage = [&](int st) {
         double* sV = smA + size_t(st & 1) * kAccStage;
         double* sD = sV + SP * kAL;
-        const size_t p0 = size_t(p_begin) + size_t(st) * kAccP;
-        for (int c = tid; c < SP * (kAccP / 2); c += 256) {
-            const int r = c / (kAccP / 2), q2 = c % (kAccP / 2);
-            cp_async16_f64(sV + r * kAL + 2 * q2, Vb + size_t(r) * Pp + p0 + 2 * q2);
-            if (!lf) cp_async16_f64(sD + r * kAL + 2 * q2, Db + size_t(r) * Pp + p0 + 2 * q2);
-        }
-        if (lf) {
-            // pattern p0 + (tid % 32), states 8 (tid / 32) .. +8 of the leaf's 0/1 vector
-            const int pp = tid & 31, j0 = 8 * (tid >> 5);
-            const size_t p = p0 + pp;
-            const int sv = tx < 0 ? -1 : int(t.states[size_t(tx) * Pp + p]);
-            const uint64_t mk = (tx < 0 || sv >= 0) ? 0 : t.masks[size_t(tx) * Pp + p];
-            const bool all = tx < 0 || (sv < 0 && (mk == 0 || (mk & t.all_mask) == t.all_mask));
+        const size_t os = o + size_t(st) * kAccP;
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const int j = j0 + q;
-                double d = 0.0;
-                if (j < t.S) d = all ? 1.0 : (sv >= 0 ? (sv == j ? 1.0 : 0.0) : (((mk >> j) & 1) ? 1.0 : 0.0));
-                sD[j * kAL + pp] = d;
-            }
+        for (int i = 0; i < SP * (kAccP / 2) / 256; ++i) {
+            const int c = tid + 256 * i, r = c / (kAccP / 2), q2 = c % (kAccP / 2);
+            cp_async16_f64(sV + r * kAL + 2 * q2, w.Vf + os + size_t(r) * Pp + 2 * q2);
+            cp_async16_f64(sD + r * kAL + 2 * q2, w.D + os + size_t(r) * Pp + 2 * q2);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-
     const int lane = tid & 31, wp = tid >> 5, g = lane >> 2, q = lane & 3;
     const int r0 = 16 * (wp >> 1), c0 = 32 * (wp & 1);
     Frag64 acc;
     frag_zero(acc);
-    if (nst > 0) stage(0);
+    stage(0);
     for (int st = 0; st < nst; ++st) {
         if (st + 1 < nst) stage(st + 1);
         else asm volatile("cp.async.commit_group;" ::: "memory");
@@ -595,15 +593,15 @@ __global__ void __launch_bounds__(256) k_accumA(Topo t, Model md, Work w, const 
         const double* sD = sV + SP * kAL;
 #pragma unroll
         for (int k = 0; k < kAccP; k += 4) {
-            double a[2], bb[4];
+            double x[2], y[4];
 #pragma unroll
-            for (int i = 0; i < 2; ++i) a[i] = sV[(r0 + 8 * i + g) * kAL + k + q];
+            for (int i = 0; i < 2; ++i) x[i] = sV[(r0 + 8 * i + g) * kAL + k + q];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) bb[j] = sD[(c0 + 8 * j + g) * kAL + k + q];
+            for (int j = 0; j < 4; ++j) y[j] = sD[(c0 + 8 * j + g) * kAL + k + q];
 #pragma unroll
             for (int i = 0; i < 2; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) dmma(acc.v[i][j][0], acc.v[i][j][1], a[i], bb[j]);
+                for (int j = 0; j < 4; ++j) dmma(acc.v[i][j][0], acc.v[i][j][1], x[i], y[j]);
         }
         __syncthreads();                         // the buffer is refilled by the next iteration's stage
     }
@@ -613,6 +611,145 @@ __global__ void __launch_bounds__(256) k_accumA(Topo t, Model md, Work w, const 
 #pragma unroll
         for (int j = 0; j < 4; ++j)
             *reinterpret_cast<double2*>(dst + frag_row(i) * SP + frag_col(j, 0)) = make_double2(acc.v[i][j][0], acc.v[i][j][1]);
+}
+
+// Leaf branches: D is a 0/1 vector, one state of each pattern for an unambiguous codon, so A[:, s] is the sum of the f V
+// columns of the patterns in state s: 64 additions a pattern instead of a 64 x 64 outer product.  `leaves` holds
+// one leaf, or the two of a node whose children are just these (x, y; y = -1 without): V of both comes from one read
+// of U and the two messages.  Warp w owns the columns j with j % 8 = w (shared memory [column][64 rows], two rows a
+// lane), walks the stage's patterns in those states in pattern order (a fixed order), and adds a pattern known only up
+// to a set of codons to each of the set's columns; patterns without information (every state) are summed
+// apart, pattern % 8 = w, and added to every column at the end.  grid (entries, M, nchunk), block 256.
+// 1.60 ms for the 1024 leaves of the tree above; as outer products of a stored f V (1.32 ms), the kernel that stored it
+// took 2 ms more.  Tried: each leaf alone with its rows of P^T fetched ahead (1.92 ms), V formed in this layout (2.40 ms).
+constexpr int kLV = kAccP + 1;                                 // row stride of a V tile: a column's rows in 16 banks
+constexpr int kLA = SP + 1;                                    // row stride of a column of A
+constexpr int kLCols = SP + kGroups;
+static const size_t kAccLeafSmem = (2 * SP * kLV + 2 * kLCols * kLA + kGroups * kTileP) * sizeof(double);
+
+// the stage's V tile (sV; own: the observed state at the lane's pattern p) added to the columns of a leaf's A
+__device__ __forceinline__ void leaf_add(double* sA, const double* sV, int own, const uint64_t* masks, int p, uint64_t all_mask, int g, int lane) {
+    auto add = [&](int col, int x) {
+        double* c = sA + col * kLA + lane;
+        const double v0 = sV[lane * kLV + x], v1 = sV[(lane + 32) * kLV + x], c0 = c[0], c1 = c[32];
+        c[0] = c0 + v0;
+        c[32] = c1 + v1;
+    };
+    for (unsigned hit = __ballot_sync(0xffffffffu, own >= 0 && (own & 7) == g); hit; hit &= hit - 1) {
+        const int x = __ffs(int(hit)) - 1;
+        add(__shfl_sync(0xffffffffu, own, x), x);
+    }
+    unsigned rest = __ballot_sync(0xffffffffu, own < 0);
+    if (rest) {
+        uint64_t mk = own >= 0 || !masks ? 0 : masks[p];
+        mk = mk == 0 || (mk & all_mask) == all_mask ? ~uint64_t(0) : mk & all_mask;     // ~0: no information
+        for (; rest; rest &= rest - 1) {
+            const int x = __ffs(int(rest)) - 1;
+            uint64_t set = __shfl_sync(0xffffffffu, mk, x);
+            if (set == ~uint64_t(0)) {
+                if ((x & 7) == g) add(SP + g, x);
+                continue;
+            }
+            for (set &= 0x0101010101010101ull << g; set; set &= set - 1) add(__ffsll((long long)set) - 1, x);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w, const int2* __restrict__ leaves) {
+    pdl_enter();
+    extern __shared__ __align__(16) double smA[];
+    double* sA = smA + 2 * SP * kLV;
+    double* smax = sA + 2 * kLCols * kLA;
+    const int m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
+    const int g = tid >> 5, lane = tid & 31;
+    const int2 cc = leaves[blockIdx.x];
+    const bool pair = cc.y >= 0;
+    const int u = t.parent[cc.x], iu = t.iidx[u], k0 = t.ch_off[u], k1 = t.ch_off[u + 1];
+    const size_t Pp = size_t(t.Pp);
+    const bool at_root = u == t.root;
+    // the message of cc.x's first sibling (cc.y's, for a pair) and, for a pair, cc.x's own
+    const int ks = t.kdesc[k0].x == cc.x ? k0 + 1 : k0;
+    const bool sib = ks < k1, more = k1 - k0 > 2;
+    const int2 ds = sib ? t.kdesc[ks] : make_int2(0, -1), dx = make_int2(cc.x, t.taxon[cc.x]);
+    const int tx = dx.y, ty = pair ? ds.y : -1;
+    const int p_begin = ck * w.chunk, nst = (min(t.Pp, p_begin + w.chunk) - p_begin) / kAccP;
+    const int* eo = w.Eown + col_off(iu, m, M, t.Pp);
+    const double* fp = w.f + size_t(m) * Pp;
+    const size_t ou = part_off(iu, m, M, t.Pp);
+    auto load_u = [&](double (&a)[8], int p) {
+        const double* src = w.U + ou + size_t(8 * g) * Pp + p;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) a[q] = at_root ? md.pi[8 * g + q] : src[q * Pp];
+    };
+    for (int x = tid; x < (pair ? 2 : 1) * kLCols * kLA; x += 256) sA[x] = 0.0;
+    double a[8], b[8], bx[8];
+    int p = p_begin + lane;
+    int own_x = child_state(t, dx, p), own_s = child_state(t, ds, p), e = eo[p];
+    double f = fp[p];
+    load_u(a, p);
+    if (sib) load_msg8(b, t, w, m, M, ds, p, g, own_s);
+    if (pair) load_msg8(bx, t, w, m, M, dx, p, g, own_x);
+    int next_x = 0, next_s = 0;
+    if (nst > 1) { next_x = child_state(t, dx, p + kAccP); next_s = child_state(t, ds, p + kAccP); }
+    for (int st = 0; st < nst; ++st, p += kAccP) {
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = sib ? a[q] * b[q] : a[q];
+        int ev = e - renorm_if_small(v, smax, g, lane, t.S);      // (its barrier: the last stage's additions are done with sV)
+        if (more)
+            for (int k = ks + 1; k < k1; ++k) {
+                const int2 d = t.kdesc[k];
+                if (d.x == cc.x) continue;
+                double x[8];
+                load_msg8(x, t, w, m, M, d, p, g, child_state(t, d, p));
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] *= x[q];
+                ev -= renorm_if_small(v, smax, g, lane, t.S);
+            }
+        if (ev != 0) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = ldexp(v[q], ev);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) smA[(8 * g + q) * kLV + lane] = f * v[q];
+        if (pair) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = a[q] * bx[q];
+            const int ey = e - renorm_if_small(v, smax, g, lane, t.S);
+            if (ey != 0) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] = ldexp(v[q], ey);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) smA[(SP + 8 * g + q) * kLV + lane] = f * v[q];
+        }
+        const int sx = own_x, sy = own_s;
+        if (st + 1 < nst) {
+            own_x = next_x;
+            own_s = next_s;
+            load_u(a, p + kAccP);
+            if (sib) load_msg8(b, t, w, m, M, ds, p + kAccP, g, own_s);
+            if (pair) load_msg8(bx, t, w, m, M, dx, p + kAccP, g, own_x);
+            e = eo[p + kAccP];
+            f = fp[p + kAccP];
+            if (st + 2 < nst) { next_x = child_state(t, dx, p + 2 * kAccP); next_s = child_state(t, ds, p + 2 * kAccP); }
+        }
+        __syncthreads();
+        leaf_add(sA, smA, sx, tx < 0 ? nullptr : t.masks + size_t(tx) * Pp, p, t.all_mask, g, lane);
+        if (pair) leaf_add(sA + kLCols * kLA, smA + SP * kLV, sy, ty < 0 ? nullptr : t.masks + size_t(ty) * Pp, p, t.all_mask, g, lane);
+    }
+    __syncthreads();
+    for (int k = 0; k < (pair ? 2 : 1); ++k) {
+        const double* A = sA + k * kLCols * kLA;
+        double* dst = w.Apart + ((size_t(k ? cc.y : cc.x) * M + m) * w.nchunk + ck) * SP2;
+        for (int x = tid; x < SP2; x += 256) {
+            const int i = x >> 6, j = x & 63;
+            double every = 0.0;
+#pragma unroll
+            for (int q = 0; q < kGroups; ++q) every += A[(SP + q) * kLA + i];
+            dst[x] = j < t.S ? A[j * kLA + i] + every : 0.0;
+        }
+    }
 }
 
 __device__ __forceinline__ double block_sum_256(double x, double* red) {
@@ -633,15 +770,21 @@ __global__ void __launch_bounds__(256) k_areduce(Topo t, Model md, Work w) {
     __shared__ double red[8];
     const int b = blockIdx.x, m = blockIdx.y, tid = threadIdx.x, n = t.n, M = md.M;
     if (b == t.root) return;
-    const double* Ap = w.Apart + (size_t(b) * M + m) * w.nchunk * SP2;
-    const double* dP = w.dP + mat_off(m, b, n);
-    double* Af = w.Afull + (size_t(b) * M + m) * SP2;
+    const double* Ap = w.Apart + (size_t(b) * M + m) * w.nchunk * SP2 + tid;
+    const double* dP = w.dP + mat_off(m, b, n) + tid;
+    double* Af = w.Afull + (size_t(b) * M + m) * SP2 + tid;
+    // a thread's 16 entries side by side: one entry after the other was 16 round trips to memory (19 us for the smallest genes)
+    double s[SP2 / 256], d[SP2 / 256];
+#pragma unroll
+    for (int i = 0; i < SP2 / 256; ++i) { s[i] = Ap[256 * i]; d[i] = dP[256 * i]; }
+    for (int ck = 1; ck < w.nchunk; ++ck)
+#pragma unroll
+        for (int i = 0; i < SP2 / 256; ++i) s[i] += Ap[size_t(ck) * SP2 + 256 * i];
     double g = 0.0;
-    for (int e = tid; e < SP2; e += 256) {
-        double s = 0.0;
-        for (int ck = 0; ck < w.nchunk; ++ck) s += Ap[size_t(ck) * SP2 + e];
-        Af[e] = s;
-        g = fma(s, dP[e], g);
+#pragma unroll
+    for (int i = 0; i < SP2 / 256; ++i) {
+        Af[256 * i] = s[i];
+        g = fma(s[i], d[i], g);
     }
     g = block_sum_256(g, red);
     if (tid == 0) w.gt[size_t(m) * n + b] = g;
@@ -850,7 +993,6 @@ __global__ void __launch_bounds__(256) k_small(Topo t, Model md, Work w, int gra
 }
 
 // ------------------------------------------------------------------ launch
-static const size_t kPruneSmem = (SP * LDM + SP * kDL + kGroups * kTileP) * sizeof(double);
 static const size_t kDirSmem = (2 * SP2 + 16 * SP) * sizeof(double);
 static const size_t kBuildSmem = size_t(2) * SP * LDM * sizeof(double);
 static const size_t kFrechetSmem = size_t(3) * SP * LDM * sizeof(double);
@@ -858,17 +1000,15 @@ static const size_t kFrechetSmem = size_t(3) * SP * LDM * sizeof(double);
 void fp64_configure() {
     cudaFuncSetAttribute(k_build_P<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBuildSmem));
     cudaFuncSetAttribute(k_build_P<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kBuildSmem));
-    cudaFuncSetAttribute(k_inside, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPruneSmem));
-    cudaFuncSetAttribute(k_outside, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kPruneSmem));
     cudaFuncSetAttribute(k_frechet, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFrechetSmem));
     cudaFuncSetAttribute(k_dir, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDirSmem));
-    cudaFuncSetAttribute(k_accumA, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccSmemF));
+    cudaFuncSetAttribute(k_accumA_int, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccIntSmem));
+    cudaFuncSetAttribute(k_accumA_leaf, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccLeafSmem));
 }
 
 int launch_build_P(const Topo& t, const Model& md, const Work& w, cudaStream_t s) {
     launch_k(k_build_P<false>, dim3(t.n, md.M), 256, kBuildSmem, s, t, md, w, MixedWork{});
-    launch_k(k_rowsum, dim3(t.n, md.M), SP, 0, s, t, md, w);
-    return 2;
+    return 1;
 }
 int launch_build_P_mixed(const Topo& t, const Model& md, const Work& w, const MixedWork& mw, cudaStream_t s) {
     launch_k(k_build_P<true>, dim3(t.n, md.M), 256, kBuildSmem, s, t, md, w, mw);
@@ -878,23 +1018,31 @@ int launch_prep_given_P(const Topo& t, const Work& w, cudaStream_t s) {
     launch_k(k_prep_given_P, t.n, 256, 0, s, t, w);
     return 1;
 }
+// Tiles per CTA of the pruning kernels: one while the level leaves SMs without a CTA to spare, up to 8 (four waves of
+// two CTAs per SM are left then, so an uneven last wave costs little).
+static int tiles_per_cta(int ntile, int nodes, int M) {
+    const long items = long(ntile) * nodes * M;
+    return int(std::max(1L, std::min({8L, long(ntile), items / (4 * 2 * 148)})));
+}
 int launch_inside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_nodes, int count, cudaStream_t s) {
-    launch_k(k_inside, dim3(t.Pp / kTileP, count, md.M), 256, kPruneSmem, s, t, md, w, d_nodes);
+    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M);
+    launch_k(k_inside, dim3((nt + k - 1) / k, count, md.M), 256, 0, s, t, md, w, d_nodes, k);
     return 1;
 }
 int launch_root(const Topo& t, const Model& md, const Work& w, cudaStream_t s) {
     launch_k(k_root, (t.Pp + 127) / 128, 128, 0, s, t, md, w);
     return 1;
 }
-int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_kids, int count, int want_v, cudaStream_t s) {
-    launch_k(k_outside, dim3(t.Pp / kTileP, count, md.M), 256, kPruneSmem, s, t, md, w, d_kids, want_v);
+int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_kids, int count, cudaStream_t s) {
+    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M);
+    launch_k(k_outside, dim3((nt + k - 1) / k, count, md.M), 256, 0, s, t, md, w, d_kids, k);
     return 1;
 }
-int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_branches, int count, cudaStream_t s) {
-    const int* none = nullptr;
-    launch_k(k_accumA, dim3(d_branches ? count : t.n, md.M, w.nchunk), 256, kAccSmemF, s, t, md, w,
-             d_branches ? d_branches : none);
-    return 1;
+int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_internal, int n_internal, const int2* d_leaves,
+                       int n_leaves, cudaStream_t s) {
+    if (n_internal) launch_k(k_accumA_int, dim3(n_internal, md.M, w.nchunk), 256, kAccIntSmem, s, t, md, w, d_internal);
+    if (n_leaves) launch_k(k_accumA_leaf, dim3(n_leaves, md.M, w.nchunk), 256, kAccLeafSmem, s, t, md, w, d_leaves);
+    return (n_internal > 0) + (n_leaves > 0);
 }
 int launch_frechet(const Topo& t, const Model& md, const Work& w, int want_global, cudaStream_t s) {
     launch_k(k_areduce, dim3(t.n, md.M), 256, 0, s, t, md, w);

@@ -10,9 +10,11 @@ int launch_build_P(const Topo& t, const Model& md, const Work& w, cudaStream_t s
 int launch_prep_given_P(const Topo& t, const Work& w, cudaStream_t s);
 int launch_inside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_nodes, int count, cudaStream_t s);
 int launch_root(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
-int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_nodes, int count, int want_v, cudaStream_t s);
-// d_branches NULL: every branch (grid over all node ids)
-int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_branches, int count, cudaStream_t s);
+// d_kids: internal children of one depth's nodes
+int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_kids, int count, cudaStream_t s);
+// A of the listed internal branches, and of leaves: entries of one leaf (y = -1) or the two of a two-leaf node
+int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_internal, int n_internal, const int2* d_leaves,
+                       int n_leaves, cudaStream_t s);
 int launch_frechet(const Topo& t, const Model& md, const Work& w, int want_global, cudaStream_t s);
 int launch_global(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 int launch_dir(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
