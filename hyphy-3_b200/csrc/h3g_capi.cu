@@ -1408,11 +1408,14 @@ extern "C" h3g_status h3g_problem_set_tuning(h3g_problem* pr, const h3g_tuning* 
     return H3G_OK;
 }
 
+// A chunk as a tuning can ask for it (the heuristic also takes smaller ones, for the smallest problems).
+static int tunable_chunk(int chunk) { return std::max(2 * TP, (chunk + TP - 1) / TP * TP); }
+
 extern "C" h3g_status h3g_problem_get_tuning(const h3g_problem* pr, h3g_tuning* tu) {
     if (!pr || !tu) return H3G_ERR_ARG;
     const WsLayout L = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), std::max(pr->M, 1), pr->K,
                                  std::max(pr->nmod, 1), pr->ndirs, effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
-    tu->a_chunk = L.chunk;
+    tu->a_chunk = tunable_chunk(L.chunk);
     tu->ctas_per_sm = pr->wait.ctas_per_sm;
     tu->frechet_groups = L.ngroups;
     return H3G_OK;
@@ -1446,8 +1449,10 @@ extern "C" h3g_status h3g_autotune(h3g_problem* pr, const double* bl, unsigned w
         return H3G_OK;
     };
     const WsLayout L0 = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs, h3g_tuning{});
-    h3g_tuning cur{L0.chunk, 2, L0.ngroups};
-    double cur_ms = 0.0;
+    const h3g_tuning heuristic{tunable_chunk(L0.chunk), 2, L0.ngroups};
+    h3g_tuning cur = heuristic;
+    double cur_ms = 0.0, untuned_ms = 0.0;
+    if (h3g_status st = measure(h3g_tuning{}, &untuned_ms); st != H3G_OK) return st;
     if (h3g_status st = measure(cur, &cur_ms); st != H3G_OK) return st;
     auto uniq = [](std::vector<int> v) { std::sort(v.begin(), v.end()); v.erase(std::unique(v.begin(), v.end()), v.end()); return v; };
     const int Pp = pr->Pp;
@@ -1469,11 +1474,20 @@ extern "C" h3g_status h3g_autotune(h3g_problem* pr, const double* bl, unsigned w
             if (ms < cur_ms) { cur = tu; cur_ms = ms; }
         }
     }
-    if (h3g_status st = h3g_problem_set_tuning(pr, &cur); st != H3G_OK) return st;
+    // nothing better than the heuristic's own chunk, below the smallest a tuning can ask for: stay with it
+    const bool keep = L0.chunk < heuristic.a_chunk && untuned_ms <= cur_ms;
+    if (keep) {
+        cur = heuristic;
+        cur_ms = untuned_ms;
+    }
+    const h3g_tuning install = keep ? h3g_tuning{} : cur;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        g_tunings[tune_key(pr, pr->M, pr->K, pr->nmod, pr->ndirs)] = cur;
+        const auto key = tune_key(pr, pr->M, pr->K, pr->nmod, pr->ndirs);
+        if (keep) g_tunings.erase(key);
+        else g_tunings[key] = cur;
     }
+    if (h3g_status st = h3g_problem_set_tuning(pr, &install); st != H3G_OK) return st;
     if (best) *best = cur;
     if (best_ms) *best_ms = cur_ms;
     return H3G_OK;
