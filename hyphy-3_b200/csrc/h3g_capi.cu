@@ -395,8 +395,11 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
                 fused_out[size_t(out_pos[best])] = 1;
             }
         }
-        for (size_t k = 0; k < pr->out_nodes.size(); ++k)
-            if (!fused_out[k]) out_heads.push_back(int(k));
+        // (no item for a leaf with one sibling: leaf_on_the_fly)
+        for (size_t k = 0; k < pr->out_nodes.size(); ++k) {
+            const int c = pr->out_nodes[k];
+            if (!fused_out[k] && !(is_leaf[c] && kids[size_t(parent[c])].size() == 2)) out_heads.push_back(int(k));
+        }
         pr->n_in_heads = int(in_heads.size());
         pr->n_out_heads = int(out_heads.size());
         std::vector<int> chains(in_next);
@@ -759,8 +762,10 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
                 ofused[size_t(pos[best])] = 1;
             }
         }
-        for (size_t k = 0; k < B.out_kids.size(); ++k)
-            if (!ofused[k]) oheads.push_back(int(k));
+        for (size_t k = 0; k < B.out_kids.size(); ++k) {
+            const int c = B.out_kids[k];
+            if (!ofused[k] && !(pr->leaf[c] && kids[size_t(pr->parent_h[c])].size() == 2)) oheads.push_back(int(k));
+        }
         o.out_next = int(lists.size());
         lists.insert(lists.end(), onxt.begin(), onxt.end());
         o.out_heads = int(lists.size());

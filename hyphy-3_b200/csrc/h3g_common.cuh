@@ -82,6 +82,12 @@ struct Topo {
     int ncp;
 };
 
+// The mixed path keeps no gradient operand for a leaf with exactly one sibling: the A accumulation forms it (the
+// outside pass's item lists leave such leaves out, by the same rule).
+__device__ __forceinline__ bool leaf_on_the_fly(const Topo& t, int b) {
+    return t.leaf[b] && t.ch_off[t.parent[b] + 1] - t.ch_off[t.parent[b]] == 2;
+}
+
 __device__ __forceinline__ int vslot(const Topo& t, int b) { return t.vidx ? t.vidx[b] : b; }
 
 struct Model {

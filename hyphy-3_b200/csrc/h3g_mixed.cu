@@ -613,21 +613,26 @@ __global__ void __launch_bounds__(kThreads, 2) k_outside_mx(Topo t, Model md, Wo
 //   acc3 += [lo; hi]  x D_lo                 (unused)            hi*lo
 // A[i][.] = acc0[i] + acc1[i] + acc2[i] + acc0[64+i] + acc1[64+i] + acc3[64+i].
 // Leaf branches have 0/1 leaf vectors (exact in BF16): only acc0 and acc2.
-// Every kADrain tiles (1024 patterns) the accumulators are drained into FP64 registers, so no
+// Every kADrain tiles of a group (1024 patterns) its accumulators are drained into FP64 registers, so no
 // FP32 accumulator takes more than 4 * kADrain = 64 additions: a truncation bias below 2e-6 relative
 // even if every addition truncated by half an ulp (gradient errors against FP64 measured 0.8-3e-6;
 // draining every 256 patterns kept them at 0.6-1e-6 and cost 11 % of the kernel in FP64 conversions).
 //
-// Pipeline (one CTA per SM, 16 warps): the FP32 V and D tiles of 64 patterns
-// stream into a kRing-deep shared-memory ring by 16-byte cp.async (one commit
-// group per tile); the threads split the oldest ring slot into one of two
-// BF16 MMA stages; one thread issues the MMAs of that stage asynchronously.
-// Copies for tiles k+1 .. k+3, the split of tile k and the MMAs of tile k-1 overlap.
-// grid (n, M, nchunk), block 512 (warp w: TMEM lane quadrant w % 4, column quarter w / 4).
+// A leaf with one sibling has no stored V: its U and the sibling's message (a stored tile, or rows of FP32 P^T by the
+// sibling's states) are multiplied as they are split, scaled by f 2^(EL - EV) in two factors so that no power of two
+// leaves the FP32 range.  Storing V for them was half of the outside pass's items and a third of its traffic:
+// with 1024 taxa x 5000 codons the outside pass went from 8.9 to 5.4 ms and this kernel stayed at 6.1 ms (the sibling
+// leaf's rows gathered into shared memory one tile ahead; gathered entry by entry in the split it took 8.0 ms).
+//
+// Pipeline (one CTA per SM): two groups of 8 warps take turns with the 64-pattern tiles, each with its own
+// two-slot FP32 ring (16-byte cp.async, one tile ahead), BF16 MMA stage, TMEM accumulators and barrier, so that one
+// group's waits are filled by the other's splits (all 16 warps on one tile at a time took 2660 cycles a tile, mostly
+// barriers and latencies).  grid (n, M, nchunk), block 512.
 constexpr int kAccThreads = 512;
 constexpr int kAT = 64;                                   // patterns per tile (MMA K per tile)
 constexpr int kADrain = 16;                               // tiles per FP32 accumulation group
-constexpr int kRing = 4;                                  // FP32 tiles in flight
+constexpr int kRing = 4;                                  // FP32 tiles: two for each group
+constexpr int kGT = kAccThreads / 2;                      // threads of a group
 constexpr uint32_t kVRows = 3 * SP;                       // stacked V terms
 constexpr uint32_t kVLbo = (kVRows / 8) * 128;            // K-chunk stride in the V stack
 constexpr uint32_t kDLbo = (SP / 8) * 128;                // K-chunk stride in a D term
@@ -639,9 +644,11 @@ constexpr size_t kStage = kVStage + 3 * kDTerm;           // 48 KB per BF16 MMA 
 constexpr uint32_t kRawRow = kAT * 4;
 constexpr size_t kRawOp = size_t(SP) * kRawRow;           // 16 KB per operand
 constexpr size_t kRawSlot = 2 * kRawOp;                   // V and D
-constexpr size_t kAccSmem = 2 * kStage + kRing * kRawSlot + 8 * 2 + 16;
-// Two TMEM accumulator sets of 4 x 64 columns (all 512 columns: the shared memory above admits one
-// CTA per SM), so one group's drain overlaps the next group's products.
+// per slot: the branch's leaf states and the two scale factors of the tile's patterns
+constexpr size_t kSide = 64 + 2 * kAT * 4;
+constexpr size_t kAccSmem = 2 * kStage + kRing * (kRawSlot + kSide) + 8 * 2 + 16;
+static_assert(kAccSmem <= 227 * 1024, "the accumulation's buffers must fit one CTA");
+// Each group's TMEM accumulators: 4 x 64 columns (all 512 columns in use: the shared memory admits one CTA per SM).
 constexpr uint32_t kAccSet = 256;
 
 struct Split8 { uint4 hi, mid, lo; };
@@ -652,34 +659,35 @@ __device__ __forceinline__ Split8 split8(const float (&x)[8]) {
     return {make_uint4(h[0], h[1], h[2], h[3]), make_uint4(md[0], md[1], md[2], md[3]), make_uint4(lo[0], lo[1], lo[2], lo[3])};
 }
 
-// The 8 patterns of state row j of a leaf's 0/1 vector, from the tile's states
-// (8 bytes at st) and masks (8 words at mk) staged in shared memory.
-__device__ __forceinline__ void leaf_row8_smem(const Topo& t, int tx, int j, const unsigned char* st, const uint64_t* mk,
-                                               float (&d)[8]) {
-    if (j >= t.S) {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) d[x] = 0.f;
-        return;
+// The 8 patterns p .. p + 7 of state row j of a leaf's 0/1 vector as BF16 pairs, from the tile's states (8 bytes at st).
+__device__ __forceinline__ uint4 leaf_row8(const Topo& t, int tx, int j, const unsigned char* st, size_t p) {
+    const uint32_t one = 0x3F803F80u;                          // 1.0, 1.0
+    if (j >= t.S) return make_uint4(0, 0, 0, 0);
+    if (tx < 0) return make_uint4(one, one, one, one);
+    const uint2 s = *reinterpret_cast<const uint2*>(st);
+    if (((s.x | s.y) & 0x80808080u) == 0) {
+        const uint32_t jj = uint32_t(j) * 0x01010101u, a = __vcmpeq4(s.x, jj), b = __vcmpeq4(s.y, jj);   // 0xFF where the state is j
+        return make_uint4(__byte_perm(a, 0, 0x1100) & one, __byte_perm(a, 0, 0x3322) & one, __byte_perm(b, 0, 0x1100) & one,
+                          __byte_perm(b, 0, 0x3322) & one);
     }
-    if (tx < 0) {
-#pragma unroll
-        for (int x = 0; x < 8; ++x) d[x] = 1.f;
-        return;
-    }
-    const uint64_t st8 = *reinterpret_cast<const uint64_t*>(st);
+    uint32_t w[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int x = 0; x < 8; ++x) {
-        const int s = int(int8_t(uint8_t(st8 >> (8 * x))));
+        const int v = int(int8_t(uint8_t((x < 4 ? s.x : s.y) >> (8 * (x & 3)))));
         bool on;
-        if (s >= 0) {
-            on = s == j;
+        if (v >= 0) {
+            on = v == j;
         } else {
-            const uint64_t m = mk[x];
+            const uint64_t m = __ldg(t.masks + size_t(tx) * t.Pp + p + x);
             on = m == 0 || (m & t.all_mask) == t.all_mask || ((m >> j) & 1);
         }
-        d[x] = on ? 1.f : 0.f;
+        if (on) w[x >> 1] |= (x & 1) ? 0x3F800000u : 0x3F80u;
     }
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
+// Where state row j of pattern x lies in a tile of leaf messages [64 patterns][64 states]: the 16-byte chunks of a
+// pattern are XOR-swizzled by its 8-pattern group, so a warp's 8 rows x 4 groups hit 32 banks.
+__device__ __forceinline__ uint32_t msg_chunk(int x, int c) { return uint32_t(x) * kRawRow + uint32_t((c ^ (2 * ((x >> 3) & 3))) << 4); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(tc::smem_u32(dst)), "l"(src) : "memory");
@@ -702,15 +710,25 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumA_mx(Topo t, Model md, 
     const int b = branches ? branches[blockIdx.x] : int(blockIdx.x), m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x;
     if (b == t.root) return;
     const int M = md.M, warp = tid >> 5, lane = tid & 31;
+    const int h = tid / kGT, gt = tid % kGT, gw = gt >> 5;       // group, thread and warp in it
     const size_t Pp = size_t(t.Pp);
     const int p_begin = ck * w.chunk, p_end = min(t.Pp, p_begin + w.chunk);
-    const int ntile = (p_end - p_begin) / kAT;
+    const int ntile = (p_end - p_begin) / kAT, nloc = (ntile - h + 1) / 2;      // tiles h, h + 2, ... are this group's
     const bool lf = t.leaf[b];
     const int tx = lf ? t.taxon[b] : -1;
-    const float* Vb = mw.Vf + part_off(vslot(t, b), m, M, t.Pp);
-    const float* Db = lf ? nullptr : mw.D + part_off(t.iidx[b], m, M, t.Pp);
+    // a leaf with one sibling: V from U and the sibling's message
+    const int u = t.parent[b], k0 = t.ch_off[u];
+    const bool fly = leaf_on_the_fly(t, b);
+    const int2 sb = fly ? t.kdesc[t.kdesc[k0].x == b ? k0 + 1 : k0] : make_int2(0, -1);
+    const bool sib_tile = fly && sb.y <= -2, sib_rows = fly && sb.y >= -1, at_root = u == t.root;
+    const float* PTs = mw.PT32 + mat_off_f(m, sb.x, t.n);
+    const int iu = t.iidx[u], is = sib_tile ? -(sb.y + 2) : 0;
+    const float* Vb = fly ? mw.U + part_off(at_root ? 0 : iu, m, M, t.Pp) : mw.Vf + part_off(vslot(t, b), m, M, t.Pp);
+    const float* Db = lf ? mw.Ms + part_off(is, m, M, t.Pp) : mw.D + part_off(t.iidx[b], m, M, t.Pp);
+    const bool load_v = !(fly && at_root), load_d = !lf || sib_tile;
     unsigned char* ring = smraw + 2 * kStage;
-    uint64_t* mma_bar = reinterpret_cast<uint64_t*>(ring + kRing * kRawSlot);   // [2]
+    unsigned char* side = ring + kRing * kRawSlot;
+    uint64_t* mma_bar = reinterpret_cast<uint64_t*>(side + kRing * kSide);   // [2]
     uint32_t* slot = reinterpret_cast<uint32_t*>(mma_bar + 2);
     if (tid == 0) {
         for (int q = 0; q < 2; ++q) tc::mbar_init(&mma_bar[q], 1);
@@ -721,102 +739,141 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumA_mx(Topo t, Model md, 
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *slot;
+    auto group_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + h), "n"(kGT) : "memory"); };
+    auto tile_p = [&](int j) { return size_t(p_begin) + size_t(2 * j + h) * kAT; };
 
-    // all threads stream tile `tile` into ring slot tile % kRing with 16-byte cp.async
-    // (256-byte state-row segments, two rows per warp instruction); one commit group per tile
-    auto produce = [&](int tile) {
-        if (tile < ntile) {
-            unsigned char* dst = ring + (tile % kRing) * kRawSlot;
-            const size_t p0 = size_t(p_begin) + size_t(tile) * kAT;
+    // the sibling leaf's states at this thread's four patterns of tile j (a byte each), loaded a tile before they are used
+    uint32_t sib_st = 0xFFFFFFFFu;
+    auto sib_states = [&](int j) {
+        if (!sib_rows || sb.y < 0 || j >= nloc) return;
+        sib_st = 0;
 #pragma unroll
-            for (int q = 0; q < 2; ++q) {
-                const int c = tid + kAccThreads * q, r = c >> 4, c16 = c & 15;
+        for (int q = 0; q < 4; ++q) sib_st |= uint32_t(uint8_t(__ldg(t.states + size_t(sb.y) * Pp + tile_p(j) + (gt >> 4) + 16 * q))) << (8 * q);
+    };
+
+    // the group streams its tile j into its ring slot j & 1 with 16-byte cp.async (256-byte state-row segments, two
+    // rows per warp instruction); one commit group per tile
+    auto produce = [&](int j) {
+        if (j < nloc) {
+            unsigned char* dst = ring + (2 * h + (j & 1)) * kRawSlot;
+            unsigned char* sd = side + (2 * h + (j & 1)) * kSide;
+            const size_t p0 = tile_p(j);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int c = gt + kGT * q, r = c >> 4, c16 = c & 15;
                 const int pc = (c16 ^ (r & 7)) * 16;
-                cp_async16(dst + r * kRawRow + pc, Vb + size_t(r) * Pp + p0 + 4 * c16);
-                if (!lf) cp_async16(dst + kRawOp + r * kRawRow + pc, Db + size_t(r) * Pp + p0 + 4 * c16);
+                if (load_v) cp_async16(dst + r * kRawRow + pc, Vb + size_t(r) * Pp + p0 + 4 * c16);
+                if (load_d) cp_async16(dst + kRawOp + r * kRawRow + pc, Db + size_t(r) * Pp + p0 + 4 * c16);
             }
-            if (lf && tx >= 0 && tid < 36) {
-                // a leaf's states (64 B) and masks (512 B) of the tile, in the unused D area of the slot
-                const size_t o = size_t(tx) * Pp + p0;
-                if (tid < 4) cp_async16(dst + kRawOp + tid * 16, t.states + o + 16 * tid);
-                else cp_async16(dst + kRawOp + 64 + (tid - 4) * 16, t.masks + o + 2 * (tid - 4));
+            if (lf && tx >= 0 && gt < 4) cp_async16(sd + 16 * gt, t.states + size_t(tx) * Pp + p0 + 16 * gt);
+            if (sib_rows) {
+                // the sibling leaf's message at each pattern: its row of FP32 P^T (or the row sums, or a masked sum)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int x = (gt >> 4) + 16 * q, c = gt & 15, st = int(int8_t(uint8_t(sib_st >> (8 * q))));
+                    unsigned char* to = dst + kRawOp + msg_chunk(x, c);
+                    const float* from = PTs + st * SP + 4 * c;
+                    if (st < 0) {
+                        const uint64_t mk = sb.y < 0 ? t.all_mask : __ldg(t.masks + size_t(sb.y) * Pp + p0 + x);
+                        if (mk == 0 || (mk & t.all_mask) == t.all_mask) {
+                            from = mw.rs32 + (size_t(m) * t.n + sb.x) * SP + 4 * c;
+                        } else {
+                            float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+                            for (uint64_t b2 = mk; b2; b2 &= b2 - 1) {
+                                const float4 r = __ldg(reinterpret_cast<const float4*>(PTs + (__ffsll((long long)b2) - 1) * SP + 4 * c));
+                                a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w;
+                            }
+                            *reinterpret_cast<float4*>(to) = a;
+                            continue;
+                        }
+                    }
+                    cp_async16(to, from);
+                }
+            }
+            if (fly && gt >= 64 && gt < 64 + kAT) {
+                // f V_true 2^-E: the scale f 2^(EL - EV) as two factors
+                const size_t p = p0 + (gt - 64);
+                const int EV = (at_root ? 0 : mw.EU[col_off(iu, m, M, t.Pp) + p]) + (sib_tile ? mw.EM[col_off(is, m, M, t.Pp) + p] : 0);
+                int fe = 0;
+                const double fm = frexp(w.f[size_t(m) * Pp + p], &fe);
+                const int e = max(-250, min(250, fe + mw.ED[col_off(t.iidx[t.root], m, M, t.Pp) + p] - EV));
+                float* sc = reinterpret_cast<float*>(sd + 64) + (gt - 64);
+                sc[0] = float(fm) * pow2f(e / 2);
+                sc[kAT] = pow2f(e - e / 2);
             }
         }
         cp_async_commit();
     };
 
-    // split item of this thread: state row 8 (tid / 64) + tid % 8, 8-pattern chunk (tid / 8) % 8
-    const int row = 8 * (tid >> 6) + (tid & 7), kc = (tid >> 3) & 7;
-    const int lq = warp & 3, cq = warp >> 2;
+    const int lq = warp & 3, cq = gw >> 2;                        // TMEM lane quadrant, half of the 64 columns
     const bool top = lq < 2;
-    double dacc[16];
+    const uint32_t set = tmem + kAccSet * uint32_t(h);            // the group's accumulators
+    double dacc[32];
 #pragma unroll
-    for (int x = 0; x < 16; ++x) dacc[x] = 0.0;
-
-    // Accumulator group G (tiles kADrain G .. kADrain G + kADrain - 1) runs on TMEM set G & 1; draining it
-    // waits for the commit of its last tile and adds the set into the FP64 registers.
-    auto drain = [&](int G) {
-        const int kl = min(ntile, (G + 1) * kADrain) - 1;
-        if (kl < 0) return;
-        if (!tc::mbar_wait(&mma_bar[kl & 1], uint32_t((kl >> 1) & 1)) && lane == 0) atomicOr(w.err, 8);
-        tc::tc_fence_after();
-        const uint32_t rowaddr = tmem + kAccSet * uint32_t(G & 1) + (uint32_t(32 * lq) << 16) + uint32_t(16 * cq);
-        // acc0, acc1 (internal branches) and acc2 (top rows) / acc3 (bottom rows, internal branches)
-        const uint32_t cols[3] = {0u, 64u, top ? 128u : 192u};
-        const bool use[3] = {true, !lf, top || !lf};
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (!use[a]) continue;
-            float v16[16];
-            tc::tmem_ld16(rowaddr + cols[a], v16);
-            tc::tmem_wait_ld();
-#pragma unroll
-            for (int x = 0; x < 16; ++x) dacc[x] += double(v16[x]);
-        }
-        tc::tc_fence_before();
-        __syncthreads();
-        tc::tc_fence_after();
-    };
-    for (int q = 0; q < kRing - 1; ++q) produce(q);
-    for (int kt = 0; kt < ntile; ++kt) {
-        const int st = kt & 1, sl = kt % kRing;
-        produce(kt + kRing - 1);                 // slot of tile kt-1, released by the barrier of iteration kt-1
-        cp_async_wait<kRing - 1>();              // this thread's copies of tile kt have landed
-        __syncthreads();                         // ... and everyone else's
-        unsigned char* VS = smraw + st * kStage;
+    for (int x = 0; x < 32; ++x) dacc[x] = 0.0;
+    sib_states(0);
+    produce(0);
+    sib_states(1);
+    for (int j = 0; j < nloc; ++j) {
+        produce(j + 1);                          // the slot of tile j - 1, whose split the last barrier ended
+        sib_states(j + 2);
+        cp_async_wait<1>();                      // this thread's copies of tile j have landed
+        group_sync();                            // ... and the group's
+        unsigned char* VS = smraw + h * kStage;
         unsigned char* DS = VS + kVStage;
-        const unsigned char* raw = ring + sl * kRawSlot;
-        if (kt >= 2 && !tc::mbar_wait(&mma_bar[st], uint32_t(((kt - 2) >> 1) & 1)) && lane == 0) atomicOr(w.err, 4);
-        {
+        const unsigned char* raw = ring + (2 * h + (j & 1)) * kRawSlot;
+        const unsigned char* sd = side + (2 * h + (j & 1)) * kSide;
+        if (j >= 1 && !tc::mbar_wait(&mma_bar[h], uint32_t((j - 1) & 1)) && lane == 0) atomicOr(w.err, 4);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            // split item: state row 8 (i / 64) + i % 8, 8-pattern chunk (i / 8) % 8
+            const int i = gt + kGT * q, row = 8 * (i >> 6) + (i & 7), kc = (i >> 3) & 7;
             const uint32_t rg = uint32_t(row >> 3) * 128 + uint32_t(row & 7) * 16;
             float x[8];
-            ld_row8(raw, row, kc, x);
+            if (load_v) {
+                ld_row8(raw, row, kc, x);
+            } else {
+                const float pi = float(md.pi[row]);
+#pragma unroll
+                for (int y = 0; y < 8; ++y) x[y] = pi;
+            }
+            if (fly) {
+                float o[8];
+                if (sib_tile) {
+                    ld_row8(raw + kRawOp, row, kc, o);
+                } else {
+#pragma unroll
+                    for (int y = 0; y < 8; ++y)
+                        o[y] = *reinterpret_cast<const float*>(raw + kRawOp + msg_chunk(8 * kc + y, row >> 2) + 4 * (row & 3));
+                }
+                const float4* sc = reinterpret_cast<const float4*>(sd + 64) + 2 * kc;
+                const float4 a0 = sc[0], a1 = sc[1], b0 = sc[kAT / 4], b1 = sc[kAT / 4 + 1];
+                const float sa[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+                const float se[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+#pragma unroll
+                for (int y = 0; y < 8; ++y) x[y] = (x[y] * sa[y]) * (o[y] * se[y]);
+            }
             const Split8 sv = split8(x);
             *reinterpret_cast<uint4*>(VS + kc * kVLbo + 0 * 1024 + rg) = sv.lo;
             *reinterpret_cast<uint4*>(VS + kc * kVLbo + 1 * 1024 + rg) = sv.hi;
             *reinterpret_cast<uint4*>(VS + kc * kVLbo + 2 * 1024 + rg) = sv.mid;
             if (lf) {
-                leaf_row8_smem(t, tx, row, raw + kRawOp + 8 * kc, reinterpret_cast<const uint64_t*>(raw + kRawOp + 64) + 8 * kc, x);
-                uint32_t h[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) h[e] = tc::bf16x2_bits(x[2 * e], x[2 * e + 1]);
-                *reinterpret_cast<uint4*>(DS + kc * kDLbo + rg) = make_uint4(h[0], h[1], h[2], h[3]);
+                *reinterpret_cast<uint4*>(DS + kc * kDLbo + rg) = leaf_row8(t, tx, row, sd + 8 * kc, tile_p(j) + 8 * kc);
             } else {
                 ld_row8(raw + kRawOp, row, kc, x);
-                const Split8 sd = split8(x);
-                *reinterpret_cast<uint4*>(DS + kc * kDLbo + rg) = sd.hi;
-                *reinterpret_cast<uint4*>(DS + kDTerm + kc * kDLbo + rg) = sd.mid;
-                *reinterpret_cast<uint4*>(DS + 2 * kDTerm + kc * kDLbo + rg) = sd.lo;
+                const Split8 sdv = split8(x);
+                *reinterpret_cast<uint4*>(DS + kc * kDLbo + rg) = sdv.hi;
+                *reinterpret_cast<uint4*>(DS + kDTerm + kc * kDLbo + rg) = sdv.mid;
+                *reinterpret_cast<uint4*>(DS + 2 * kDTerm + kc * kDLbo + rg) = sdv.lo;
             }
         }
         tc::fence_async_smem();
         tc::tc_fence_before();
-        __syncthreads();
+        group_sync();
         tc::tc_fence_after();
-        if (tid == 0) {
+        if (gt == 0) {
             const uint32_t vs = tc::smem_u32(VS), ds = tc::smem_u32(DS);
-            const bool first = (kt % kADrain) == 0;
-            const uint32_t set = tmem + kAccSet * uint32_t((kt / kADrain) & 1);     // this group's accumulators
+            const bool first = (j % kADrain) == 0;
 #pragma unroll
             for (int ks = 0; ks < kAT / 16; ++ks) {
                 const uint32_t acc = (first && ks == 0) ? 0u : 1u;
@@ -832,23 +889,44 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumA_mx(Topo t, Model md, 
                     tc::mma_bf16(set + 192, a2, bl, kIdesc, acc);
                 }
             }
-            tc::mma_commit(&mma_bar[st]);
+            tc::mma_commit(&mma_bar[h]);
         }
-        // the previous group's accumulators drain while this tile's products run on the other set
-        if ((kt % kADrain) == 0 && kt > 0) drain(kt / kADrain - 1);
+        if ((j + 1) % kADrain == 0 || j + 1 == nloc) {
+            // the accumulators into the FP64 registers; the next tile's first barrier orders the loads before its products
+            if (!tc::mbar_wait(&mma_bar[h], uint32_t(j & 1)) && lane == 0) atomicOr(w.err, 8);
+            tc::tc_fence_after();
+            const uint32_t rowaddr = set + (uint32_t(32 * lq) << 16) + uint32_t(32 * cq);
+            // acc0, acc1 (internal branches) and acc2 (top rows) / acc3 (bottom rows, internal branches)
+            const uint32_t cols[3] = {0u, 64u, top ? 128u : 192u};
+            const bool use[3] = {true, !lf, top || !lf};
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                if (!use[a]) continue;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    float v16[16];
+                    tc::tmem_ld16(rowaddr + cols[a] + 16 * q, v16);
+                    tc::tmem_wait_ld();
+#pragma unroll
+                    for (int x = 0; x < 16; ++x) dacc[16 * q + x] += double(v16[x]);
+                }
+            }
+            tc::tc_fence_before();
+        }
     }
-    drain((ntile - 1) / kADrain);
-    // combine the two halves of each state row in shared memory (stages are idle now), write coalesced
+    // combine the groups and the two halves of each state row in shared memory (stages are idle once both groups
+    // are here), in a fixed order, write coalesced
     double* sA = reinterpret_cast<double*>(smraw);              // [64][65]
     const int i = 32 * lq + lane - (top ? 0 : 64);
-    if (!top) {
 #pragma unroll
-        for (int x = 0; x < 16; ++x) sA[i * 65 + 16 * cq + x] = dacc[x];
-    }
-    __syncthreads();
-    if (top) {
+    for (int turn = 0; turn < 4; ++turn) {
+        __syncthreads();
+        if (turn != 2 * h + (top ? 1 : 0)) continue;
 #pragma unroll
-        for (int x = 0; x < 16; ++x) sA[i * 65 + 16 * cq + x] += dacc[x];
+        for (int x = 0; x < 32; ++x) {
+            double* c = sA + i * 65 + 32 * cq + x;
+            *c = turn == 0 ? dacc[x] : *c + dacc[x];
+        }
     }
     __syncthreads();
     double* dst = w.Apart + ((size_t(b) * M + m) * w.nchunk + ck) * SP2;
