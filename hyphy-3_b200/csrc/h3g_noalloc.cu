@@ -74,6 +74,7 @@ extern "C" h3g_status h3g_eval_from_P_noalloc(int device, void* cuda_stream, int
     int ch_off[kNoallocMaxNodes + 1], ch[kNoallocMaxNodes], iidx[kNoallocMaxNodes], taxon[kNoallocMaxNodes];
     int order[kNoallocMaxNodes], height[kNoallocMaxNodes], in_nodes[kNoallocMaxNodes], in_off[kNoallocMaxNodes + 1];
     int fill[kNoallocMaxNodes];
+    int2 kdesc[kNoallocMaxNodes];
     int root = -1, NI = 0;
     std::memset(ch_off, 0, sizeof(int) * (n + 1));
     for (int i = 0; i < n; ++i) {
@@ -109,6 +110,7 @@ extern "C" h3g_status h3g_eval_from_P_noalloc(int device, void* cuda_stream, int
             taxon[i] = leaf_taxon[i] < 0 ? -1 : leaf_taxon[i];
         }
     }
+    for (int k = 0; k < ch_off[n]; ++k) kdesc[k] = make_int2(ch[k], is_leaf[ch[k]] ? taxon[ch[k]] : -(2 + iidx[ch[k]]));
     int m = 0;
     in_off[0] = 0;
     for (int h = 1; h <= H; ++h) {
@@ -147,10 +149,8 @@ extern "C" h3g_status h3g_eval_from_P_noalloc(int device, void* cuda_stream, int
     t.n = n; t.root = root; t.NI = NI; t.T = T; t.P = n_patterns; t.Pp = Pp; t.S = S;
     t.all_mask = S >= 64 ? ~uint64_t(0) : ((uint64_t(1) << S) - 1);
     int* d_ch_off = c.take<int>(n + 1);
-    int* d_ch = c.take<int>(std::max(n, 1));
+    int2* d_kdesc = c.take<int2>(n);
     int* d_iidx = c.take<int>(n);
-    int* d_taxon = c.take<int>(n);
-    uint8_t* d_leaf = c.take<uint8_t>(n);
     int* d_in_nodes = c.take<int>(std::max(m, 1));
     int8_t* d_st_pm = c.take<int8_t>(std::max<size_t>(size_t(n_patterns) * T, 1));
     uint64_t* d_mk_pm = c.take<uint64_t>(std::max<size_t>(size_t(n_patterns) * T, 1));
@@ -176,10 +176,8 @@ extern "C" h3g_status h3g_eval_from_P_noalloc(int device, void* cuda_stream, int
     cudaError_t e = cudaSuccess;
     auto ok = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     ok(cudaMemcpyAsync(d_ch_off, ch_off, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
-    ok(cudaMemcpyAsync(d_ch, ch, sizeof(int) * std::max(ch_off[n], 1), cudaMemcpyHostToDevice, s));
+    ok(cudaMemcpyAsync(d_kdesc, kdesc, sizeof(int2) * ch_off[n], cudaMemcpyHostToDevice, s));
     ok(cudaMemcpyAsync(d_iidx, iidx, sizeof(int) * n, cudaMemcpyHostToDevice, s));
-    ok(cudaMemcpyAsync(d_taxon, taxon, sizeof(int) * n, cudaMemcpyHostToDevice, s));
-    ok(cudaMemcpyAsync(d_leaf, is_leaf, n, cudaMemcpyHostToDevice, s));
     if (m > 0) ok(cudaMemcpyAsync(d_in_nodes, in_nodes, sizeof(int) * m, cudaMemcpyHostToDevice, s));
     // the scratch keeps the previous call's contents: zero what is read before written
     ok(cudaMemsetAsync(d_w, 0, sizeof(double) * Pp, s));
@@ -200,7 +198,7 @@ extern "C" h3g_status h3g_eval_from_P_noalloc(int device, void* cuda_stream, int
         const size_t total = size_t(T) * Pp;
         k_noalloc_patterns<<<unsigned((total + 255) / 256), 256, 0, s>>>(d_st_pm, d_mk_pm, n_patterns, T, Pp, d_st, d_mk);
     }
-    t.ch_off = d_ch_off; t.ch = d_ch; t.iidx = d_iidx; t.leaf = d_leaf; t.taxon = d_taxon;
+    t.ch_off = d_ch_off; t.kdesc = d_kdesc; t.iidx = d_iidx;      // what the inside pass reads of the topology
     t.states = d_st; t.masks = d_mk; t.w = d_w;
     md.M = 1; md.K = 1; md.nmod = 1; md.sentinel = 1; md.pi = d_pi;
     launch_prep_given_P(t, w, s);
