@@ -27,7 +27,13 @@ struct h3g_ctx {
     int live_problems = 0;
     std::string err;
     void* compress = nullptr;      // alignment-compression scratch (h3g_compress.cu), kept between calls
+    // Pinned memory that h3g_model_set passes a model through, for every problem of the context (kept between calls up
+    // to kStageKeep): whoever fills it holds the mutex until the device has read it.
+    std::mutex stage_mu;
+    double* stage = nullptr;
+    size_t stage_count = 0;
 };
+constexpr size_t kStageKeep = size_t(8) << 20;     // doubles (64 MB)
 
 namespace h3g {
 void compress_scratch_free(void* p);     // h3g_compress.cu
@@ -209,6 +215,7 @@ extern "C" h3g_status h3g_ctx_destroy(h3g_ctx* ctx) {
     if (ctx->live_problems > 0) return fail(ctx, H3G_ERR_STATE, "destroy every problem before its context");
     cudaSetDevice(ctx->device);
     if (ctx->compress) h3g::compress_scratch_free(ctx->compress);
+    if (ctx->stage) cudaFreeHost(ctx->stage);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return H3G_OK;
@@ -881,15 +888,54 @@ static h3g_status ensure_workspace(h3g_problem* pr, int M, int K, int nmod, int 
 static uint64_t hash_bytes(uint64_t h, const void* p, size_t n) {
     const unsigned char* c = static_cast<const unsigned char*>(p);
     size_t i = 0;
-    for (; i + 8 <= n; i += 8) {
+    auto mix = [](uint64_t& l, const unsigned char* at) {
         uint64_t w;
-        std::memcpy(&w, c + i, 8);
-        h = (h ^ w) * 0x9E3779B97F4A7C15ull;
-        h ^= h >> 29;
+        std::memcpy(&w, at, 8);
+        l = (l ^ w) * 0x9E3779B97F4A7C15ull;
+        l ^= l >> 29;
+    };
+    if (n >= 64) {                   // four chains side by side: one is bound by the multiply's latency
+        uint64_t lane[4] = {h, h ^ 0x243F6A8885A308D3ull, h ^ 0x13198A2E03707344ull, h ^ 0xA4093822299F31D0ull};
+        for (; i + 32 <= n; i += 32)
+            for (int q = 0; q < 4; ++q) mix(lane[q], c + i + 8 * q);
+        for (const uint64_t l : lane) { h = (h ^ l) * 0x9E3779B97F4A7C15ull; h ^= h >> 29; }
     }
+    for (; i + 8 <= n; i += 8) mix(h, c + i);
     for (; i < n; ++i) { h ^= c[i]; h *= 1099511628211ull; }
     return h;
 }
+
+namespace {
+// The context's staging memory, grown to `count` doubles and held; the destructor waits for the device's reads.
+struct StageHold {
+    h3g_ctx* ctx;
+    cudaStream_t other;
+    std::unique_lock<std::mutex> lk;
+    StageHold(h3g_ctx* c, cudaStream_t s2) : ctx(c), other(s2), lk(c->stage_mu) {}
+    cudaError_t grow(size_t count) {
+        if (count <= ctx->stage_count) return cudaSuccess;
+        if (ctx->stage) cudaFreeHost(ctx->stage);
+        ctx->stage = nullptr;
+        ctx->stage_count = 0;
+        count = std::max(count, size_t(1) << 14);
+        const cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&ctx->stage), count * sizeof(double));
+        if (e == cudaSuccess) ctx->stage_count = count;
+        return e;
+    }
+    cudaError_t wait() {
+        const cudaError_t a = cudaStreamSynchronize(ctx->stream), b = cudaStreamSynchronize(other);
+        return a != cudaSuccess ? a : b;
+    }
+    ~StageHold() {
+        wait();
+        if (ctx->stage_count > kStageKeep) {
+            cudaFreeHost(ctx->stage);
+            ctx->stage = nullptr;
+            ctx->stage_count = 0;
+        }
+    }
+};
+}  // namespace
 
 extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
     if (!pr || !d) return H3G_ERR_ARG;
@@ -955,22 +1001,6 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
         pr->time_mode = d->time_mode; pr->sentinel = d->zero_l_sentinel;
         if (pr->precision != d->precision) { pr->drop_graphs(); pr->work_mem.release(); pr->w = Work{}; }
         pr->precision = d->precision;
-        std::vector<double> pi(SP, 0.0), Q(size_t(nm) * SP2), U(size_t(nm) * SP2), V(size_t(nm) * SP2), lam(size_t(nm) * SP, 0.0);
-        std::vector<double> UT(size_t(nm) * SP2), QT(size_t(nm) * SP2);
-        std::copy(d->pi, d->pi + S, pi.begin());
-        for (int k = 0; k < nm; ++k) {
-            pad_matrix(d->Q + size_t(k) * S * S, S, &Q[size_t(k) * SP2]);
-            if (!dev_eig) {
-                pad_matrix(d->U + size_t(k) * S * S, S, &U[size_t(k) * SP2]);
-                pad_matrix(d->V + size_t(k) * S * S, S, &V[size_t(k) * SP2]);
-                std::copy(d->lam + size_t(k) * S, d->lam + size_t(k) * S + S, &lam[size_t(k) * SP]);
-            }
-            for (int i = 0; i < SP; ++i)
-                for (int j = 0; j < SP; ++j) {
-                    UT[size_t(k) * SP2 + size_t(j) * SP + i] = U[size_t(k) * SP2 + size_t(i) * SP + j];
-                    QT[size_t(k) * SP2 + size_t(j) * SP + i] = Q[size_t(k) * SP2 + size_t(i) * SP + j];
-                }
-        }
         std::vector<double> mu(nm, 1.0);
         if (d->mu) {
             std::copy(d->mu, d->mu + nm, mu.begin());
@@ -983,14 +1013,6 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
             }
         }
         pr->h_mu = mu;
-        // dense directions [n_dirs][nm], then the per-model ones [nm]
-        std::vector<double> dQ((size_t(std::max(d->n_dirs, 1)) * nm + size_t(n_model_dirs)) * SP2, 0.0);
-        for (int x = 0; x < d->n_dirs; ++x)
-            for (int k = 0; k < nm; ++k) pad_matrix(d->dQ + (size_t(x) * nm + k) * S * S, S, &dQ[(size_t(x) * nm + k) * SP2]);
-        for (int k = 0; k < n_model_dirs; ++k)
-            pad_matrix(d->dQ_model + size_t(k) * S * S, S, &dQ[(size_t(d->n_dirs) * nm + k) * SP2]);
-        std::vector<uint8_t> it(pr->n, 1);
-        if (d->is_test) std::copy(d->is_test, d->is_test + pr->n, it.begin());
         // grow-only, like the workspace
         size_t mkey[5] = {size_t(nm), size_t(d->K), size_t(d->M), size_t(std::max(d->n_dirs, 1) + (n_model_dirs ? 1 : 0)),
                           size_t(pr->n)};
@@ -1016,37 +1038,63 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
             H3G_TRY_CUDA(ctx, A.alloc(&pr->m_rt, cM));
             H3G_TRY_CUDA(ctx, A.alloc(&pr->m_rw, cM));
             H3G_TRY_CUDA(ctx, A.alloc(&pr->m_dQ, cdirs * cnm * SP2));
-            H3G_TRY_CUDA(ctx, A.alloc(&pr->m_it, it.size()));
-            H3G_TRY_CUDA(ctx, A.alloc(&pr->m_br, size_t(pr->n) + 1));
+            H3G_TRY_CUDA(ctx, A.alloc(&pr->m_it, (size_t(pr->n) + 7) / 8 * 8));          // whole 8-byte words
+            H3G_TRY_CUDA(ctx, A.alloc(&pr->m_br, (size_t(pr->n) + 2) / 2 * 2));
             std::copy(mkey, mkey + 5, pr->model_key);
         }
+        // The caller's arrays go through pinned memory as they are and a kernel lays them out (padded, transposed):
+        // generators first, so that they are diagonalised while the host still stages the directions.
         cudaStream_t s = ctx->stream;
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_pi, pi.data(), SP * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_Q, Q.data(), Q.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_QT, QT.data(), QT.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        if (dev_eig) {
-            launch_model_eig(pr->m_Q, pr->m_pi, S, nm, pr->m_lam, pr->m_U, pr->m_UT, pr->m_V, s);
-            H3G_TRY_CUDA(ctx, cudaGetLastError());
-        } else {
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_lam, lam.data(), lam.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_U, U.data(), U.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_UT, UT.data(), UT.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_V, V.data(), V.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+        const size_t SS = size_t(S) * S, n_dq = size_t(d->n_dirs) * nm + size_t(n_model_dirs);
+        const size_t br_words = d->branch_classes ? (size_t(pr->n) + 2) / 2 : 0, it_words = d->is_test ? (size_t(pr->n) + 7) / 8 : 0;
+        StageHold hold(ctx, pr->s2);
+        H3G_TRY_CUDA(ctx, hold.grow(size_t(S) + 3 * nm * SS + size_t(nm) * (S + 2) + d->K + 2 * d->M + br_words + it_words + n_dq * SS));
+        double* st_at = ctx->stage;
+        auto stage = [&](const void* src, size_t bytes) {
+            double* at = st_at;
+            std::memcpy(at, src, bytes);
+            st_at += (bytes + 7) / 8;
+            return at;
+        };
+        auto vec = [&](ModelInstall& in, const void* src, size_t bytes, void* dst, int rows, int pad) {
+            const int words = int((bytes + 7) / 8);
+            in.vec[in.n_vec++] = {stage(src, bytes), static_cast<double*>(dst), rows, words / rows, pad ? pad : words / rows};
+        };
+        auto mats = [&](ModelInstall& in, const double* src, int count, double* dst, double* dst_t) {
+            in.mat[in.n_mat++] = {stage(src, size_t(count) * SS * sizeof(double)), dst, dst_t, count};
+        };
+        ModelInstall in{};
+        in.S = S;
+        vec(in, d->pi, S * sizeof(double), pr->m_pi, 1, SP);
+        mats(in, d->Q, nm, pr->m_Q, pr->m_QT);
+        if (!dev_eig) {
+            vec(in, d->lam, size_t(nm) * S * sizeof(double), pr->m_lam, nm, SP);
+            mats(in, d->U, nm, pr->m_U, pr->m_UT);
+            mats(in, d->V, nm, pr->m_V, nullptr);
         }
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_mu, mu.data(), mu.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_cw, d->class_w, d->K * sizeof(double), cudaMemcpyHostToDevice, s));
+        vec(in, mu.data(), mu.size() * sizeof(double), pr->m_mu, 1, 0);
+        vec(in, d->class_w, d->K * sizeof(double), pr->m_cw, 1, 0);
         if (d->has_bg > 0) {
             pr->h_bw.assign(size_t(d->has_bg), 1.0);
             if (d->bg_w) std::copy(d->bg_w, d->bg_w + d->has_bg, pr->h_bw.begin());
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_bw, pr->h_bw.data(), pr->h_bw.size() * sizeof(double), cudaMemcpyHostToDevice, s));
+            vec(in, pr->h_bw.data(), pr->h_bw.size() * sizeof(double), pr->m_bw, 1, 0);
         }
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_rt, d->rates, d->M * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_rw, d->rate_w, d->M * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_dQ, dQ.data(), dQ.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_it, it.data(), it.size(), cudaMemcpyHostToDevice, s));
-        if (d->branch_classes)
-            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->m_br, d->branch_classes, size_t(pr->n + 1) * sizeof(int32_t),
-                                              cudaMemcpyHostToDevice, s));
+        vec(in, d->rates, d->M * sizeof(double), pr->m_rt, 1, 0);
+        vec(in, d->rate_w, d->M * sizeof(double), pr->m_rw, 1, 0);
+        if (d->is_test) vec(in, d->is_test, size_t(pr->n), pr->m_it, 1, 0);
+        if (d->branch_classes) vec(in, d->branch_classes, size_t(pr->n + 1) * sizeof(int32_t), pr->m_br, 1, 0);
+        launch_model_install(in, s);
+        if (dev_eig) launch_model_eig(pr->m_Q, pr->m_pi, S, nm, pr->m_lam, pr->m_U, pr->m_UT, pr->m_V, s);
+        H3G_TRY_CUDA(ctx, cudaGetLastError());
+        if (n_dq > 0) {
+            // dense directions [n_dirs][nm], then the per-model ones [nm]
+            ModelInstall dq{};
+            dq.S = S;
+            if (d->n_dirs > 0) mats(dq, d->dQ, d->n_dirs * nm, pr->m_dQ, nullptr);
+            if (n_model_dirs > 0) mats(dq, d->dQ_model, n_model_dirs, pr->m_dQ + size_t(d->n_dirs) * nm * SP2, nullptr);
+            launch_model_install(dq, pr->s2);
+            H3G_TRY_CUDA(ctx, cudaGetLastError());
+        }
         Model md{};
         md.M = d->M; md.K = d->K; md.has_bg = d->has_bg; md.nmod = nm; md.time_mode = d->time_mode; md.ndirs = n_dirs_all;
         md.ndirs_dense = d->n_dirs;
@@ -1060,7 +1108,7 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
         pr->md = md;
         h3g_status st = ensure_workspace(pr, d->M, d->K, nm, n_dirs_all);
         if (st != H3G_OK) return st;
-        H3G_TRY_CUDA(ctx, cudaStreamSynchronize(s));
+        H3G_TRY_CUDA(ctx, hold.wait());
         pr->model_hash = h;
         pr->has_model = true;
         return H3G_OK;

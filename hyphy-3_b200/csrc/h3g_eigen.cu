@@ -67,7 +67,46 @@ __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q,
     }
 }
 
+// A model's arrays from the caller's layout in pinned host memory to the engine's: matrices S x S to 64 x 64, padded with
+// zeros, and transposed where asked (a CTA each), vectors and byte arrays by the last CTA.  Read over the bus once,
+// coalesced; padding and transposing on the host and copying from pageable memory took 350 us for 3 codon models with
+// 8 directions, and this kernel takes about the bus time of the unpadded arrays.
+__global__ void __launch_bounds__(256) k_model_install(ModelInstall in) {
+    pdl_enter();
+    const int tid = threadIdx.x, S = in.S;
+    int b = blockIdx.x;
+    for (int g = 0; g < in.n_mat; b -= in.mat[g].count, ++g) {
+        if (b >= in.mat[g].count) continue;
+        __shared__ double tile[SP * (SP + 1)];
+        const double* src = in.mat[g].src + size_t(b) * S * S;
+        double* dst = in.mat[g].dst + size_t(b) * SP2;
+        for (int e = tid; e < SP * (SP + 1); e += 256) tile[e] = 0.0;
+        __syncthreads();
+#pragma unroll 8
+        for (int e = tid; e < S * S; e += 256) tile[(e / S) * (SP + 1) + e % S] = src[e];
+        __syncthreads();
+        for (int e = tid; e < SP2; e += 256) dst[e] = tile[(e >> 6) * (SP + 1) + (e & 63)];
+        if (double* dt = in.mat[g].dst_t)
+            for (int e = tid; e < SP2; e += 256) dt[size_t(b) * SP2 + e] = tile[(e & 63) * (SP + 1) + (e >> 6)];
+        return;
+    }
+    for (int g = 0; g < in.n_vec; ++g) {
+        const auto& v = in.vec[g];
+        for (int e = tid; e < v.rows * v.pad; e += 256) {
+            const int r = e / v.pad, c = e % v.pad;
+            v.dst[e] = c < v.width ? v.src[r * v.width + c] : 0.0;
+        }
+    }
+}
+
 }  // namespace
+
+int launch_model_install(const ModelInstall& in, cudaStream_t s) {
+    int blocks = in.n_vec ? 1 : 0;
+    for (int g = 0; g < in.n_mat; ++g) blocks += in.mat[g].count;
+    launch_k(k_model_install, blocks, 256, 0, s, in);
+    return 1;
+}
 
 void eigen_configure() {
     cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem));

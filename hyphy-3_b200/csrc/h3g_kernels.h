@@ -5,6 +5,14 @@
 
 namespace h3g {
 
+// Arrays of a model in pinned host memory and where the engine wants them (k_model_install).
+struct ModelInstall {
+    struct Mat { const double* src; double* dst; double* dst_t; int count; } mat[3];       // [count][S][S] -> [count][64][64]
+    struct Vec { const double* src; double* dst; int rows, width, pad; } vec[9];           // [rows][width] -> [rows][pad], 8-byte words
+    int n_mat, n_vec, S;
+};
+int launch_model_install(const ModelInstall& in, cudaStream_t s);
+
 void fp64_configure();
 int launch_build_P(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 int launch_prep_given_P(const Topo& t, const Work& w, cudaStream_t s);
