@@ -368,7 +368,6 @@ __device__ __forceinline__ void tile_mm_store(const RowFrags& f, const double* _
 // Tried and slower: leaves' matrices staged in shared memory (2.92), columns fetched by cp.async two tiles ahead
 // (3.09), whole rows of P^T fetched for leaves (2.93).
 __global__ void __launch_bounds__(256, 2) k_inside(Topo t, Model md, Work w, const int* __restrict__ nodes, int tiles) {
-    pdl_enter();
     __shared__ __align__(16) double sD[SP * kDL];
     __shared__ double smax[kGroups * kTileP];
     const int u = nodes[blockIdx.y], m = blockIdx.z, tid = threadIdx.x;
@@ -382,6 +381,7 @@ __global__ void __launch_bounds__(256, 2) k_inside(Topo t, Model md, Work w, con
     double a0[8], a1[8];
     int p = t0 * kTileP + lane;
     int s0 = child_state(t, d0, p), s1 = child_state(t, d1, p);
+    pdl_enter();                                                   // above: the problem's tables and patterns only
 #pragma unroll
     for (int q = 0; q < 8; ++q) a0[q] = 8 * g + q < t.S ? 1.0 : 0.0;      // a node without children
     if (one) load_msg8(a0, t, w, m, M, d0, p, g, s0);
@@ -432,11 +432,11 @@ __global__ void __launch_bounds__(256, 2) k_inside(Topo t, Model md, Work w, con
 
 // --------------------------------------------------------------------- root
 __global__ void k_root(Topo t, Model md, Work w) {
-    pdl_enter();
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= t.Pp) return;
     const int ir = t.iidx[t.root], M = md.M;
     const double wt = t.w[p];
+    pdl_enter();
     double L[kMaxRateClasses], ll[kMaxRateClasses];
     for (int m = 0; m < M; ++m) {
         const double* D = w.D + part_off(ir, m, M, t.Pp) + p;
@@ -483,7 +483,6 @@ __global__ void k_root(Topo t, Model md, Work w) {
 // it (k_accumA_leaf): storing it for them was half of this kernel's CTAs and the gradient's largest stream
 // (1024 taxa x 1200 codons x 4 rates: 4.87 -> 2.81 ms).
 __global__ void __launch_bounds__(256, 2) k_outside(Topo t, Model md, Work w, const int* __restrict__ kids, int tiles) {
-    pdl_enter();
     __shared__ __align__(16) double sV[SP * kDL];
     __shared__ double smax[kGroups * kTileP];
     const int c = kids[blockIdx.y], m = blockIdx.z, g = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -505,7 +504,9 @@ __global__ void __launch_bounds__(256, 2) k_outside(Topo t, Model md, Work w, co
     };
     double a[8], b[8];
     int p = t0 * kTileP + lane;
-    int st = child_state(t, ds, p), nx = 0, e = eo[p];
+    int st = child_state(t, ds, p), nx = 0;
+    pdl_enter();                                                  // above: the problem's tables and patterns only
+    int e = eo[p];
     double f = fp[p];
     load_u(a, p);
     if (sib) load_msg8(b, t, w, m, M, ds, p, g, st);
@@ -560,7 +561,6 @@ constexpr size_t kAccStage = size_t(2) * SP * kAL;             // V and D tiles 
 static const size_t kAccIntSmem = 2 * kAccStage * sizeof(double);
 
 __global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, const int* __restrict__ branches) {
-    pdl_enter();
     extern __shared__ __align__(16) double smA[];
     const int b = branches[blockIdx.x], m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
     const size_t Pp = size_t(t.Pp);
@@ -583,6 +583,7 @@ __global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, co
     const int r0 = 16 * (wp >> 1), c0 = 32 * (wp & 1);
     Frag64 acc;
     frag_zero(acc);
+    pdl_enter();                                 // above: the problem's tables only
     stage(0);
     for (int st = 0; st < nst; ++st) {
         if (st + 1 < nst) stage(st + 1);
@@ -656,7 +657,6 @@ __device__ __forceinline__ void leaf_add(double* sA, const double* sV, int own, 
 }
 
 __global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w, const int2* __restrict__ leaves) {
-    pdl_enter();
     extern __shared__ __align__(16) double smA[];
     double* sA = smA + 2 * SP * kLV;
     double* smax = sA + 2 * kLCols * kLA;
@@ -684,7 +684,9 @@ __global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w
     for (int x = tid; x < (pair ? 2 : 1) * kLCols * kLA; x += 256) sA[x] = 0.0;
     double a[8], b[8], bx[8];
     int p = p_begin + lane;
-    int own_x = child_state(t, dx, p), own_s = child_state(t, ds, p), e = eo[p];
+    int own_x = child_state(t, dx, p), own_s = child_state(t, ds, p);
+    pdl_enter();                                                  // above: the problem's tables and patterns only
+    int e = eo[p];
     double f = fp[p];
     load_u(a, p);
     if (sib) load_msg8(b, t, w, m, M, ds, p, g, own_s);
