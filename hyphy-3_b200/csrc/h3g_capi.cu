@@ -74,6 +74,8 @@ struct h3g_problem {
     uint8_t* d_leaf = nullptr;
     int2* d_kdesc = nullptr;
     int4* d_in_info = nullptr;
+    int4* d_few = nullptr;             // Topo::few_in, then few_out
+    int* d_few_lv = nullptr;
     int4* d_out_info = nullptr;
     int* d_chains = nullptr;           // [in_next | in_heads | out_next | out_heads]
     int n_in_heads = 0, n_out_heads = 0;
@@ -157,6 +159,9 @@ struct h3g_problem {
         t.all_mask = S >= 64 ? ~uint64_t(0) : ((uint64_t(1) << S) - 1);
         t.vidx = nullptr;
         t.ncp = 0;
+        t.few_in = d_few; t.few_out = d_few ? d_few + 2 * in_nodes.size() : nullptr;
+        t.few_in_lv = d_few_lv; t.few_out_lv = d_few_lv + in_off.size();
+        t.few_in_levels = int(in_off.size()) - 1; t.few_out_levels = int(out_int_off.size()) - 1;
         return t;
     }
     // the topology an evaluation of this problem's own workspace runs on: checkpoint slots when planned
@@ -425,6 +430,29 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_kdesc, kdesc.data(), kdesc.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_in_info, in_info.data(), in_info.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_out_info, out_info.data(), out_info.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+        std::vector<int4> few;
+        std::vector<int> few_lv;
+        if (pr->max_state < kFewStates) {
+            for (int u : pr->in_nodes) {
+                const int k0 = pr->ch_off[u], k1 = pr->ch_off[u + 1];
+                const int2 none = make_int2(0, -1), a = k0 < k1 ? kdesc[k0] : none, b = k0 + 1 < k1 ? kdesc[k0 + 1] : none;
+                few.push_back(make_int4(u, pr->iidx[u], k0, k1));
+                few.push_back(make_int4(a.x, a.y, b.x, b.y));
+            }
+            for (int k = 0; k < pr->out_int_off.back(); ++k) {
+                const int c = pr->out_split[size_t(k)], u = parent[c], k0 = pr->ch_off[u], k1 = pr->ch_off[u + 1];
+                const int ks = pr->ch[size_t(k0)] == c ? k0 + 1 : k0;
+                const int2 d = ks < k1 ? kdesc[ks] : make_int2(0, -1);
+                few.push_back(make_int4(c, pr->iidx[u], pr->iidx[c], u == pr->root));
+                few.push_back(make_int4(d.x, d.y, ks, k1));
+            }
+            few_lv = pr->in_off;
+            few_lv.insert(few_lv.end(), pr->out_int_off.begin(), pr->out_int_off.end());
+            H3G_TRY_CUDA(ctx, A.alloc(&pr->d_few, few.size()));
+            H3G_TRY_CUDA(ctx, A.alloc(&pr->d_few_lv, few_lv.size()));
+            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_few, few.data(), few.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
+            H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_few_lv, few_lv.data(), few_lv.size() * sizeof(int), cudaMemcpyHostToDevice, s));
+        }
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_states, st.size()));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_masks, mk.size()));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_w, wt.size()));
@@ -1138,6 +1166,9 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
     const Topo t = pr->topo();
     const Model& md = pr->md;
     const bool mixed = pr->precision == H3G_PREC_MIXED;
+    // Up to four states, FP64: the walks of h3g_few.cu.  For 256 taxa x 3000 nucleotide patterns a call with gradients
+    // takes 610 us, with the 64-state passes 2130 us; these win at every size, they do a sixteenth of the work.
+    const bool few = !mixed && t.S <= kFewStates && t.few_in;
     const bool grads = (want & (H3G_WANT_GRAD_T | H3G_WANT_GRAD_GLOBAL)) != 0;
     const bool global = (want & H3G_WANT_GRAD_GLOBAL) != 0;
     int L = 0;
@@ -1161,6 +1192,8 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
     if (mixed) {
         // one persistent launch over every level, per-tile dependencies
         l = launch_inside_mixed(t, md, w, mwk, pr->n_in_heads, pr->wait, s);
+    } else if (few) {
+        l = launch_inside_few(t, md, w, s);
     } else {
         for (size_t lv = 0; lv + 1 < pr->in_off.size(); ++lv) {
             const int cnt = pr->in_off[lv + 1] - pr->in_off[lv];
@@ -1174,6 +1207,8 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
         l = 0;
         if (mixed) {
             l = launch_outside_mixed(t, md, w, mwk, pr->n_out_heads, pr->wait, s);
+        } else if (few) {
+            l = launch_outside_few(t, md, w, s);
         } else {
             for (size_t lv = 0; lv + 1 < pr->out_int_off.size(); ++lv) {
                 const int cnt = pr->out_int_off[lv + 1] - pr->out_int_off[lv];
@@ -1183,6 +1218,7 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
         }
         mark(ST_OUTSIDE, l);
         mark(ST_ACCUM_A, mixed ? launch_accumA_mixed(t, md, w, mwk, nullptr, 0, s)
+                         : few ? launch_accumA_few(t, md, w, s)
                                : launch_accumA_fp64(t, md, w, pr->d_out_split, pr->out_int_off.back(),
                                                     reinterpret_cast<const int2*>(pr->d_out_split + pr->pairs_at), pr->n_pairs, s));
         mark(ST_FRECHET, launch_frechet(t, md, w, global ? 1 : 0, s));

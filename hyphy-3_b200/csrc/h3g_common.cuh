@@ -84,7 +84,13 @@ struct Topo {
     // the nodes of other blocks reuse
     const int* vidx;
     int ncp;
+    // walks of the passes for models of at most kFewStates states (h3g_few.cu): item descriptors in level order, two
+    // each, and the levels' offsets.  NULL for problems with more states.
+    const int4 *few_in, *few_out;
+    const int *few_in_lv, *few_out_lv;
+    int few_in_levels, few_out_levels;
 };
+constexpr int kFewStates = 4;
 
 // The mixed path keeps no gradient operand for a leaf with exactly one sibling: the A accumulation forms it (the
 // outside pass's item lists leave such leaves out, by the same rule).

@@ -441,7 +441,11 @@ __global__ void k_root(Topo t, Model md, Work w) {
     for (int m = 0; m < M; ++m) {
         const double* D = w.D + part_off(ir, m, M, t.Pp) + p;
         double s = 0.0;
-        for (int i = 0; i < SP; ++i) s = fma(md.pi[i], D[size_t(i) * t.Pp], s);
+        if (t.S > kFewStates) {
+            for (int i = 0; i < SP; ++i) s = fma(md.pi[i], D[size_t(i) * t.Pp], s);
+        } else {                                   // h3g_few.cu leaves the other rows unwritten
+            for (int i = 0; i < kFewStates; ++i) s = fma(md.pi[i], D[size_t(i) * t.Pp], s);
+        }
         L[m] = s;
         ll[m] = s > 0.0 ? log(s) - double(w.Ecum[col_off(ir, m, M, t.Pp) + p]) * 0.69314718055994530942 : -1e20;
     }

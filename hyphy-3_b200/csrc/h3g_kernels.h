@@ -23,6 +23,10 @@ int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int
 // A of the listed internal branches, and of leaves: entries of one leaf (y = -1) or the two of a two-leaf node
 int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_internal, int n_internal, const int2* d_leaves,
                        int n_leaves, cudaStream_t s);
+// The same passes for t.S <= kFewStates, one launch each (h3g_few.cu)
+int launch_inside_few(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
+int launch_outside_few(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
+int launch_accumA_few(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 int launch_frechet(const Topo& t, const Model& md, const Work& w, int want_global, cudaStream_t s);
 int launch_global(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 int launch_dir(const Topo& t, const Model& md, const Work& w, cudaStream_t s);

@@ -12,9 +12,10 @@
 // log-likelihood log L - E ln 2, or the reference's -1e20 when L <= 0; the weighted sum
 // over patterns is a fixed-order Neumaier sum.  FP64 throughout.
 //
-// With fewer patterns than it takes to fill the GPU (kLevelBelow), the tree is walked
-// level by level instead: one launch per height, one thread per (internal node of the
-// level, pattern), partials stored per internal node.
+// With fewer patterns than it takes to fill the GPU (kLevelBelow), a CTA of 16 warps
+// walks the tree for 32 patterns level by level instead (h3g_few.cuh), a warp per
+// internal node of the level, partials stored per internal node.  A call for 256 taxa
+// x 3000 patterns (41 levels) takes 545 us, with a launch per level 684 us.
 #include <algorithm>
 #include <cmath>
 #include <new>
@@ -22,7 +23,7 @@
 #include <utility>
 #include <vector>
 
-#include "h3g_common.cuh"
+#include "h3g_few.cuh"
 #include "h3g_fel.h"
 
 namespace h3g {
@@ -35,7 +36,6 @@ int problem_max_state(h3g_problem* pr);
 namespace {
 
 constexpr int kNucT = 128;                                 // threads per block (patterns)
-constexpr int kLvlT = 256;
 constexpr int kSumT = 1024;
 constexpr int kLevelBelow = 131072;                        // patterns: below, the level-by-level walk
 
@@ -49,8 +49,6 @@ struct NucState {
     double4* d_stk = nullptr;                              // [depth][Pp]
     int* d_exp = nullptr;                                  // [depth][Pp]
     bool levels = false;                                   // level-by-level walk
-    std::vector<int> lv_off;                               // [H + 1] internal nodes by height
-    int* d_lv = nullptr;                                   // [NI]
     double4* d_part = nullptr;                             // [NI][Pp]
     int* d_pexp = nullptr;                                 // [NI][Pp]
     double* d_lnl = nullptr;
@@ -132,91 +130,102 @@ __global__ void __launch_bounds__(kNucT) k_nuc_lnl(Topo t, const int* __restrict
     site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
 }
 
-// leaf vector of taxon tx at pattern p (likelihood.hpp:54-87)
-__device__ __forceinline__ void nuc_leaf(const Topo& t, int tx, int p, double (&x)[4]) {
-    int st = -1;
-    uint64_t mk = 0xF;
-    if (tx >= 0) {
-        st = t.states[size_t(tx) * size_t(t.Pp) + p];
-        if (!(st >= 0 && st < 4)) mk = t.masks[size_t(tx) * size_t(t.Pp) + p];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-        x[i] = (st >= 0 && st < 4) ? (i == st ? 1.0 : 0.0) : ((mk == 0 || (mk & 0xF) == 0xF || ((mk >> i) & 1)) ? 1.0 : 0.0);
-}
-
-// one thread per (internal node of this level, pattern): the product of the children's messages
-__global__ void __launch_bounds__(kLvlT) k_nuc_level(Topo t, const int* __restrict__ nodes, int cnt, const double* __restrict__ P,
-                                                      const double* __restrict__ pi, double4* __restrict__ part,
-                                                      int* __restrict__ pexp, double* __restrict__ site) {
-    pdl_enter();                                           // the lower levels' partials are complete
-    const int i = int(blockIdx.x) * kLvlT + int(threadIdx.x);
-    if (i >= cnt * t.P) return;
-    const int u = nodes[i / t.P], p = i - (i / t.P) * t.P;
+// The product of the children's messages at every internal node, level by level; grid Pp / 32.
+__global__ void __launch_bounds__(32 * kFewWarps) k_nuc_walk(Topo t, const double* __restrict__ P, const double* __restrict__ pi,
+                                                             double4* part, int* pexp, double* __restrict__ site) {
+    const int lane = threadIdx.x & 31, p = 32 * int(blockIdx.x) + lane;
     const size_t Pp = size_t(t.Pp);
-    double d[4] = {1.0, 1.0, 1.0, 1.0};
-    int E = 0;
-    for (int e = t.ch_off[u]; e < t.ch_off[u + 1]; ++e) {
-        const int c = t.ch[e];
-        double x[4];
-        if (t.leaf[c]) {
-            nuc_leaf(t, t.taxon[c], p, x);
-        } else {
-            const size_t o = size_t(t.iidx[c]) * Pp + p;
-            const double4 v = part[o];
-            x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
-            E += pexp[o];
-        }
-        const double* Pn = P + size_t(c) * 16;
-        double mx = 0.0;
+    few_walk(
+        t.few_in_lv, t.few_in_levels, t.few_in, threadIdx.x >> 5,
+        [&](int4 d, int& s0, int& s1) { s0 = few_state(t, make_int2(d.x, d.y), p); s1 = few_state(t, make_int2(d.z, d.w), p); },
+        [] { pdl_enter(); },
+        [&](int4 a, int4 d4, int s0, int s1) {
+            const int u = a.x, k0 = a.z, k1 = a.w;
+            double d[4] = {1.0, 1.0, 1.0, 1.0};
+            int E = 0;
+            struct Child { double2 P[8]; double x[4]; int E; };
+            auto load = [&](int2 c, int st) {
+                Child o;
+                const double2* Pn = reinterpret_cast<const double2*>(P + size_t(c.x) * 16);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            d[k] *= __ldg(Pn + 4 * k) * x[0] + __ldg(Pn + 4 * k + 1) * x[1] + __ldg(Pn + 4 * k + 2) * x[2] +
-                    __ldg(Pn + 4 * k + 3) * x[3];
-            mx = fmax(mx, d[k]);
-        }
-        if (mx > 0.0 && mx < 0x1p-256) {
+                for (int i = 0; i < 8; ++i) o.P[i] = __ldg(Pn + i);
+                o.E = 0;
+                if (c.y <= -2) {
+                    const size_t at = size_t(-(c.y + 2)) * Pp + p;
+                    const double4 v = part[at];
+                    o.x[0] = v.x; o.x[1] = v.y; o.x[2] = v.z; o.x[3] = v.w;
+                    o.E = pexp[at];
+                } else {                                   // likelihood.hpp:54-87
+                    const uint64_t mk = st >= 0 ? uint64_t(1) << st : (c.y < 0 ? 0xF : t.masks[size_t(c.y) * Pp + p]);
+                    const bool any = st < 0 && (mk == 0 || (mk & 0xF) == 0xF);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) d[k] *= 0x1p256;
-            E += 256;
-        }
-    }
-    if (u == t.root) {
-        const double L = pi[0] * d[0] + pi[1] * d[1] + pi[2] * d[2] + pi[3] * d[3];
-        site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
-    } else {
-        const size_t o = size_t(t.iidx[u]) * Pp + p;
-        part[o] = make_double4(d[0], d[1], d[2], d[3]);
-        pexp[o] = E;
-    }
+                    for (int i = 0; i < 4; ++i) o.x[i] = any || ((mk >> i) & 1) ? 1.0 : 0.0;
+                }
+                return o;
+            };
+            auto take = [&](const Child& c) {
+                double mx = 0.0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double2 a01 = c.P[2 * i], a23 = c.P[2 * i + 1];
+                    d[i] *= a01.x * c.x[0] + a01.y * c.x[1] + a23.x * c.x[2] + a23.y * c.x[3];
+                    mx = fmax(mx, d[i]);
+                }
+                E += c.E;
+                if (mx > 0.0 && mx < 0x1p-256) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) d[i] *= 0x1p256;
+                    E += 256;
+                }
+            };
+            if (k0 + 1 < k1) {                             // two side by side: one trip to memory
+                const Child c0 = load(make_int2(d4.x, d4.y), s0), c1 = load(make_int2(d4.z, d4.w), s1);
+                take(c0);
+                take(c1);
+            } else if (k0 < k1) {
+                take(load(make_int2(d4.x, d4.y), s0));
+            }
+            for (int k = k0 + 2; k < k1; ++k) take(load(t.kdesc[k], few_state(t, t.kdesc[k], p)));
+            if (u == t.root) {
+                if (p >= t.P) return;
+                const double L = pi[0] * d[0] + pi[1] * d[1] + pi[2] * d[2] + pi[3] * d[3];
+                site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
+            } else {
+                const size_t o = size_t(a.y) * Pp + p;
+                part[o] = make_double4(d[0], d[1], d[2], d[3]);
+                pexp[o] = E;
+            }
+        });
 }
 
-// one block: weights x site log-likelihoods, Neumaier over contiguous chunks, then the chunk sums in order
+// One block: weights x site log-likelihoods, Neumaier over every 1024th pattern, then a fixed tree of two-sums (the
+// 1024 partial sums added up by one thread took 25 of this kernel's 27 us).
+__device__ __forceinline__ void two_sum(double& s, double& c, double x, double xc) {
+    const double t = s + x;
+    c += xc + (fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s);
+    s = t;
+}
 __global__ void __launch_bounds__(kSumT) k_nuc_sum(const double* __restrict__ site, const double* __restrict__ w, int P,
                                                    double* __restrict__ out) {
-    pdl_enter();                                           // k_nuc_lnl's site log-likelihoods are complete
-    __shared__ double hi[kSumT], lo[kSumT];
+    pdl_enter();                                           // the site log-likelihoods are complete
+    __shared__ double hi[kSumT / 32], lo[kSumT / 32];
     const int tid = threadIdx.x;
-    const int chunk = (P + kSumT - 1) / kSumT, b = tid * chunk, e = min(P, b + chunk);
     double s = 0.0, c = 0.0;
-    for (int i = b; i < e; ++i) {
-        const double x = w[i] * site[i], t = s + x;
-        c += fabs(s) >= fabs(x) ? (s - t) + x : (x - t) + s;
-        s = t;
-    }
-    hi[tid] = s;
-    lo[tid] = c;
+    for (int i = tid; i < P; i += kSumT) two_sum(s, c, w[i] * site[i], 0.0);
+    auto warp_sum = [&] {
+        for (int o = 16; o > 0; o >>= 1) {
+            const double x = __shfl_down_sync(0xffffffffu, s, o), xc = __shfl_down_sync(0xffffffffu, c, o);
+            two_sum(s, c, x, xc);
+        }
+    };
+    warp_sum();
+    if ((tid & 31) == 0) { hi[tid >> 5] = s; lo[tid >> 5] = c; }
     __syncthreads();
-    if (tid == 0) {
-        double S = 0.0, Cc = 0.0;
-        for (int k = 0; k < kSumT; ++k)
-            for (double x : {hi[k], lo[k]}) {
-                const double t = S + x;
-                Cc += fabs(S) >= fabs(x) ? (S - t) + x : (x - t) + S;
-                S = t;
-            }
-        *out = S + Cc;
-    }
+    if (tid >= 32) return;
+    s = hi[tid];
+    c = lo[tid];
+    warp_sum();
+    if (tid == 0) *out = s + c;
 }
 
 // depth-first events (2 node + 1 opens an internal node, 2 node closes a node) and the
@@ -261,25 +270,6 @@ NucState* nuc_state(h3g_problem* pr, const FelProblemView& v, std::string* err) 
     s->P = t.P;
     s->Pp = size_t(t.Pp);
     s->levels = t.P < kLevelBelow;
-    std::vector<int> lv;
-    if (s->levels) {                                       // internal nodes by height, children first
-        std::vector<int> h(size_t(v.n), 0);
-        for (int e : ev)
-            if (!(e & 1)) {                                // a node closes after its descendants
-                const int u = e >> 1;
-                for (int c = v.ch_off[u]; c < v.ch_off[u + 1]; ++c) h[size_t(u)] = std::max(h[size_t(u)], h[size_t(v.ch[c])] + 1);
-            }
-        for (int c = v.ch_off[v.root]; c < v.ch_off[v.root + 1]; ++c) h[size_t(v.root)] = std::max(h[size_t(v.root)], h[size_t(v.ch[c])] + 1);
-        const int H = h[size_t(v.root)];
-        s->lv_off.assign(size_t(H) + 1, 0);
-        for (int u = 0; u < v.n; ++u)
-            if (!v.leaf[u]) ++s->lv_off[size_t(h[size_t(u)])];
-        for (int k = 1; k <= H; ++k) s->lv_off[size_t(k)] += s->lv_off[size_t(k) - 1];
-        lv.resize(size_t(s->lv_off[size_t(H)]));
-        std::vector<int> fill(s->lv_off.begin(), s->lv_off.end() - 1);
-        for (int u = 0; u < v.n; ++u)
-            if (!v.leaf[u]) lv[size_t(fill[size_t(h[size_t(u)]) - 1]++)] = u;
-    }
     auto take = [&](auto** p, size_t count) {
         void* q = nullptr;
         if (cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(**p)) != cudaSuccess) return false;
@@ -292,8 +282,7 @@ NucState* nuc_state(h3g_problem* pr, const FelProblemView& v, std::string* err) 
               cudaMallocHost(reinterpret_cast<void**>(&s->h_pin), sizeof(double)) == cudaSuccess &&
               cudaMemcpy(s->d_ev, ev.data(), ev.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess;
     if (ok && s->levels)
-        ok = take(&s->d_lv, lv.size()) && take(&s->d_part, size_t(t.NI) * s->Pp) && take(&s->d_pexp, size_t(t.NI) * s->Pp) &&
-             cudaMemcpy(s->d_lv, lv.data(), lv.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess;
+        ok = take(&s->d_part, size_t(t.NI) * s->Pp) && take(&s->d_pexp, size_t(t.NI) * s->Pp);
     else if (ok)
         ok = take(&s->d_stk, size_t(deepest) * s->Pp) && take(&s->d_exp, size_t(deepest) * s->Pp);
     // the copies above come from pageable memory on the default stream, which the evaluator's
@@ -338,13 +327,8 @@ extern "C" h3g_status h3g_nuc_eval_from_P(h3g_problem* pr, const double* P, cons
               cudaMemcpyAsync(s->d_pi, pi, 4 * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess;
     if (ok && s->P > 0) {
         if (s->levels) {
-            for (size_t k = 0; k + 1 < s->lv_off.size(); ++k) {
-                const int cnt = s->lv_off[k + 1] - s->lv_off[k];
-                if (cnt == 0) continue;
-                launch_k(k_nuc_level, int((size_t(cnt) * size_t(s->P) + kLvlT - 1) / kLvlT), kLvlT, 0, st, t,
-                         static_cast<const int*>(s->d_lv + s->lv_off[k]), cnt, static_cast<const double*>(s->d_P),
-                         static_cast<const double*>(s->d_pi), s->d_part, s->d_pexp, s->d_site);
-            }
+            launch_k(k_nuc_walk, (s->P + 31) / 32, 32 * kFewWarps, 0, st, t, static_cast<const double*>(s->d_P),
+                     static_cast<const double*>(s->d_pi), s->d_part, s->d_pexp, s->d_site);
         } else {
             launch_k(k_nuc_lnl, (s->P + kNucT - 1) / kNucT, kNucT, 0, st, t, static_cast<const int*>(s->d_ev), s->n_ev,
                      static_cast<const double*>(s->d_P), static_cast<const double*>(s->d_pi), s->d_stk, s->d_exp, s->d_site);
