@@ -353,20 +353,29 @@ __device__ void prune(const Spectral<NC>& sp, double* sL, const Topo& t, const d
 // over the tree).  With BG, a branch flagged in f.bg uses the request's
 // background eigensystem alone (weight 1) instead of the NC tested ones.
 // Persistent: CTA b evaluates requests b, b + grid, ...
+//
+// A level costs a warp two dependent 64-term sums (kept in order: the fits compare likelihoods bit for bit) and, before
+// this layout, four dependent loads; three CTAs of 8 warps to an SM hide more of that chain than two of 16, the
+// descriptors come a level ahead, and a wide level's rows of U and V are read once for two nodes.  A FEL run on
+// 256 taxa x 400 codons: 115 -> 98 ms (one node at a time 103; two CTAs with four nodes 129, 384 threads 120).
 struct LevelPlan {
     int H;                    // levels: 0 = leaves ... H - 1 = the root alone
     const int* off;           // [H + 1]
-    const int* nodes;         // [n] nodes ordered by level
+    const int4* nodes;        // [n] in level order: {node, taxon (-1: missing) of a leaf or -2, first two children or -1}
 };
 
-constexpr int kLvT = 512;
-constexpr int kLvW = kLvT / 32;
-
-// nc tested components, plus the background's eigensystem when bg
-constexpr size_t lv_smem(int nc, bool bg) {
-    return (size_t(nc + (bg ? 1 : 0)) * (2 * SP * LD + SP) + size_t(kLvW) * (nc + 1) * SP) * sizeof(double);
-}
-static_assert(lv_smem(2, true) <= 227 * 1024, "three eigensystems must fit one CTA");
+// CTA shape by the eigensystems of a request (nc tested components, plus the background's when bg): threads, CTAs to an
+// SM, and the nodes of a level that a warp takes at once (a row of U or V is then read once for all of them; the
+// nodes of a background branch use other matrices, so with a background it is one).
+template <int NC, bool BG>
+struct LevelShape {
+    static constexpr int kThreads = NC == 1 && !BG ? 256 : 512, kPerSm = NC == 1 && !BG ? 3 : 1;
+    static constexpr int kGroup = BG ? 1 : 2, kWarps = kThreads / 32;
+    // eigensystems, and the group's vectors per warp
+    static constexpr size_t kSmem = (size_t(NC + (BG ? 1 : 0)) * (2 * SP * LD + SP) + size_t(kWarps) * kGroup * NC * SP) * sizeof(double);
+    static_assert(kPerSm * (kSmem + 1024 + 64) <= 228 * 1024, "the CTAs of an SM share its memory");
+};
+constexpr int kLevelCtas = 3;             // most CTAs to an SM of any shape
 
 __device__ __forceinline__ double warp_max(double v) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -378,162 +387,249 @@ __device__ __forceinline__ double warp_sum(double v) {
     return v;
 }
 
+// One request's matrices and scalars, as every warp of its CTA sees them.
 template <int NC, bool BG>
-__global__ void __launch_bounds__(kLvT) k_site_lnl(FelModel f, Topo t, const double* __restrict__ bl, LevelPlan lp,
+struct LevelRequest {
+    static constexpr int NT = NC + (BG ? 1 : 0);          // eigensystems per request; the last is the background's
+    double *U[NT], *V[NT], *lam[NT];                      // shared
+    double w[NC];
+    double *msg, *vec;                                     // the CTA's messages; this warp's vectors (shared)
+    double* L;                                             // shared: the root's value and exponent
+    int* E;
+    int p;
+};
+
+// a[k] = rows lane and lane + 32 of mat (shared, stride LD) times the vectors vec + k * stride; every sum runs over j
+// in order, whatever G is
+template <int G>
+__device__ __forceinline__ void rows_times(double (&a)[G][2], const double* mat, const double* vec, int stride, int lane) {
+    const double *r0 = mat + lane * LD, *r1 = r0 + 32 * LD;
+#pragma unroll
+    for (int k = 0; k < G; ++k) a[k][0] = a[k][1] = 0.0;
+#pragma unroll 4
+    for (int j = 0; j < SP; j += 2) {
+        const double x0 = r0[j], x1 = r0[j + 1], y0 = r1[j], y1 = r1[j + 1];
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            const double2 v = *reinterpret_cast<const double2*>(vec + k * stride + j);
+            a[k][0] = fma(x1, v.y, fma(x0, v.x, a[k][0]));
+            a[k][1] = fma(y1, v.y, fma(y0, v.x, a[k][1]));
+        }
+    }
+}
+
+// Nodes d[0 .. count), count <= G, of one level by one warp (LevelPlan::nodes; d[count ..] repeat a node).
+template <int NC, bool BG, int G>
+__device__ __forceinline__ void level_nodes(const LevelRequest<NC, BG>& q, const FelModel& f, const Topo& t, const double* __restrict__ bl,
+                                            const int4 (&d)[LevelShape<NC, BG>::kGroup], int count, int lane) {
+    constexpr int NT = LevelRequest<NC, BG>::NT;
+    const int s0 = lane, s1 = lane + 32, S = t.S;
+    double m[G][2][2];                                     // the first two children's messages, all loaded side by side
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int c = e ? d[k].w : d[k].z;
+            if (c >= 0) {
+                m[k][e][0] = q.msg[size_t(c) * SP + s0];
+                m[k][e][1] = q.msg[size_t(c) * SP + s1];
+            }
+        }
+    // the branch above u: the tested components, or the background one alone
+    const bool bgn = BG && f.bg[d[0].x] != 0;
+    const int ncu = bgn ? 1 : NC;
+    double ex[NC][G][2];                                   // e^{lambda a t_b}, before the sums that it scales
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+        const double tb = bl[d[k].x];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (c >= ncu) break;
+            const double* lc = bgn ? q.lam[NT - 1] : q.lam[c];
+            ex[c][k][0] = exp(lc[s0] * tb);
+            ex[c][k][1] = exp(lc[s1] * tb);
+        }
+    }
+    double x[NC][G][2];
+    bool inner = false;
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+        if (d[k].y > -2) {                                 // x_c = V_c * leaf vector
+            const int tx = d[k].y;
+            int st = -1;
+            uint64_t mk = t.all_mask;
+            if (tx >= 0) {
+                st = t.states[size_t(tx) * t.Pp + q.p];
+                if (st < 0) mk = t.masks[size_t(tx) * t.Pp + q.p];
+            }
+            const bool all = mk == 0 || (mk & t.all_mask) == t.all_mask;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                if (c >= ncu) break;
+                const double* Vc = bgn ? q.V[NT - 1] : q.V[c];
+                double a0 = 0.0, a1 = 0.0;
+                if (st >= 0) {
+                    a0 = Vc[s0 * LD + st];
+                    a1 = Vc[s1 * LD + st];
+                } else {
+                    for (int j = 0; j < S; ++j)
+                        if (all || ((mk >> j) & 1)) { a0 += Vc[s0 * LD + j]; a1 += Vc[s1 * LD + j]; }
+                }
+                x[c][k][0] = a0;
+                x[c][k][1] = a1;
+            }
+        } else {                                           // D = product of the children's messages
+            double d0 = s0 < S ? 1.0 : 0.0, d1 = s1 < S ? 1.0 : 0.0;
+            int E = 0;
+            auto take = [&](double c0, double c1) {
+                d0 *= c0;
+                d1 *= c1;
+                const double mx = warp_max(fmax(d0, d1));
+                if (mx > 0.0 && mx < 0x1p-256) {
+                    d0 *= 0x1p256;
+                    d1 *= 0x1p256;
+                    E += 256;
+                }
+            };
+            if (d[k].z >= 0) take(m[k][0][0], m[k][0][1]);
+            if (d[k].w >= 0) {
+                take(m[k][1][0], m[k][1][1]);
+                const int end = t.ch_off[d[k].x + 1];
+                for (int e = t.ch_off[d[k].x] + 2; e < end; ++e) {
+                    const double* mc = q.msg + size_t(t.ch[e]) * SP;
+                    take(mc[s0], mc[s1]);
+                }
+            }
+            if (lane == 0 && E && k < count) atomicAdd(q.E, E);
+            if (d[k].x == t.root) {                          // L = pi . D; the root is alone on its level
+                const double v = warp_sum((s0 < S ? f.pi[s0] * d0 : 0.0) + (s1 < S ? f.pi[s1] * d1 : 0.0));
+                if (lane == 0) *q.L = v;
+                return;
+            }
+            q.vec[k * SP + s0] = d0;
+            q.vec[k * SP + s1] = d1;
+            inner = true;
+        }
+    }
+    if (inner) {                                           // x_c = V_c D
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (c >= ncu) break;
+            double a[G][2];
+            rows_times<G>(a, bgn ? q.V[NT - 1] : q.V[c], q.vec, SP, lane);
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (d[k].y <= -2) { x[c][k][0] = a[k][0]; x[c][k][1] = a[k][1]; }
+        }
+        __syncwarp();                                      // every lane has read the partials
+    }
+#pragma unroll
+    for (int k = 0; k < G; ++k)
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+            if (c >= ncu) break;
+            q.vec[(c * G + k) * SP + s0] = x[c][k][0] * ex[c][k][0];
+            q.vec[(c * G + k) * SP + s1] = x[c][k][1] * ex[c][k][1];
+        }
+    __syncwarp();
+    double m0[G], m1[G];
+#pragma unroll
+    for (int k = 0; k < G; ++k) m0[k] = m1[k] = 0.0;
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+        if (c >= ncu) break;
+        double a[G][2];
+        rows_times<G>(a, bgn ? q.U[NT - 1] : q.U[c], q.vec + c * G * SP, SP, lane);
+        const double wc = bgn ? 1.0 : q.w[c];
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            m0[k] += wc * a[k][0];
+            m1[k] += wc * a[k][1];
+        }
+    }
+    __syncwarp();                                          // the vectors are reused by this warp's next nodes
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+        if (k >= count) break;
+        q.msg[size_t(d[k].x) * SP + s0] = s0 < S ? fmax(m0[k], 0.0) : 0.0;
+        q.msg[size_t(d[k].x) * SP + s1] = s1 < S ? fmax(m1[k], 0.0) : 0.0;
+    }
+}
+
+template <int NC, bool BG>
+__global__ void __launch_bounds__(LevelShape<NC, BG>::kThreads, LevelShape<NC, BG>::kPerSm) k_site_lnl(FelModel f, Topo t, const double* __restrict__ bl, LevelPlan lp,
                                                    double* __restrict__ work, FelReqs q, int n_req, double* __restrict__ out) {
-    constexpr int NT = NC + (BG ? 1 : 0);                 // eigensystems per request; the last is the background's
+    using Shape = LevelShape<NC, BG>;
+    constexpr int NT = NC + (BG ? 1 : 0), W = Shape::kWarps, GM = Shape::kGroup;
     pdl_enter();
     extern __shared__ __align__(16) double sm[];
     __shared__ int sE;
     __shared__ double sL;
-    double* U[NT];
-    double* V[NT];
-    double* lam[NT];
-    double* z = sm;
+    LevelRequest<NC, BG> rq;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    rq.vec = sm + size_t(warp) * GM * NC * SP;             // first: its pairs are read as 16 bytes
+    double* z = sm + size_t(W) * GM * NC * SP;
 #pragma unroll
     for (int c = 0; c < NT; ++c) {
-        U[c] = z; z += SP * LD;
-        V[c] = z; z += SP * LD;
-        lam[c] = z; z += SP;
+        rq.U[c] = z; z += SP * LD;
+        rq.V[c] = z; z += SP * LD;
+        rq.lam[c] = z; z += SP;
     }
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, S = t.S;
-    double* dv = z + size_t(warp) * (NC + 1) * SP;        // this warp's partial
-    double* xv = dv + SP;                                  // [NC][64] spectral coordinates
-    double* msg = work + size_t(blockIdx.x) * t.n * SP;
-    const int s0 = lane, s1 = lane + 32;
+    rq.msg = work + size_t(blockIdx.x) * t.n * SP;
+    rq.L = &sL;
+    rq.E = &sE;
     for (int r = blockIdx.x; r < n_req; r += gridDim.x) {
         int sl[NT];
-        double w[NC];
         sl[0] = q.slot[r];
         if constexpr (NC == 2) {
             sl[1] = q.slot2[r];
-            w[0] = q.w1[r];
-            w[1] = 1.0 - q.w1[r];
+            rq.w[0] = q.w1[r];
+            rq.w[1] = 1.0 - q.w1[r];
         } else {
-            w[0] = 1.0;
+            rq.w[0] = 1.0;
         }
         if constexpr (BG) sl[NT - 1] = q.slot_bg[r];
         const double a = q.a[r];
-        const int p = q.pattern[r];
+        rq.p = q.pattern[r];
         __syncthreads();                                   // the previous request is done with shared memory
 #pragma unroll
         for (int c = 0; c < NT; ++c) {
             const double* gU = f.U + size_t(sl[c]) * SP2;
             const double* gV = f.V + size_t(sl[c]) * SP2;
-            for (int e = tid; e < SP2; e += kLvT) {
+            for (int e = tid; e < SP2; e += Shape::kThreads) {
                 const int i = e >> 6, j = e & 63;
-                U[c][i * LD + j] = gU[e];
-                V[c][i * LD + j] = gV[e];
+                rq.U[c][i * LD + j] = gU[e];
+                rq.V[c][i * LD + j] = gV[e];
             }
-            if (tid < SP) lam[c][tid] = f.lam[size_t(sl[c]) * SP + tid] * a;
+            if (tid < SP) rq.lam[c][tid] = f.lam[size_t(sl[c]) * SP + tid] * a;
         }
         if (tid == 0) { sE = 0; sL = 0.0; }
         __syncthreads();
+        // as many nodes at once as leaves no warp idle
+        auto group = [](int nodes) { return min(GM, nodes <= W ? 1 : (nodes <= 2 * W ? 2 : 4)); };
+        auto load = [&](int4 (&d)[GM], int i, int g, int end) {
+#pragma unroll
+            for (int k = 0; k < GM; ++k)
+                if (k < g && i < end) d[k] = lp.nodes[min(i + k, end - 1)];
+        };
+        int b0 = lp.off[0], b1 = lp.off[1], b2 = lp.off[min(2, lp.H)];
+        int4 d[GM], nx[GM];                                // this warp's first nodes of the level and of the next
+        load(d, b0 + warp * group(b1 - b0), group(b1 - b0), b1);
         for (int h = 0; h < lp.H; ++h) {
-            const int b1 = lp.off[h + 1];
-            for (int i = lp.off[h] + warp; i < b1; i += kLvW) {
-                const int u = lp.nodes[i];
-                // the branch above u: the tested components, or the background one alone
-                const bool bgn = BG && f.bg[u] != 0;
-                const int ncu = bgn ? 1 : NC;
-                double x[NC][2];
-                if (t.leaf[u]) {                           // x_c = V_c * leaf vector
-                    const int tx = t.taxon[u];
-                    int st = -1;
-                    uint64_t mk = t.all_mask;
-                    if (tx >= 0) {
-                        st = t.states[size_t(tx) * t.Pp + p];
-                        if (st < 0) mk = t.masks[size_t(tx) * t.Pp + p];
-                    }
-                    const bool all = mk == 0 || (mk & t.all_mask) == t.all_mask;
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        if (c >= ncu) break;
-                        const double* Vc = bgn ? V[NT - 1] : V[c];
-                        double a0 = 0.0, a1 = 0.0;
-                        if (st >= 0) {
-                            a0 = Vc[s0 * LD + st];
-                            a1 = Vc[s1 * LD + st];
-                        } else {
-                            for (int j = 0; j < S; ++j)
-                                if (all || ((mk >> j) & 1)) { a0 += Vc[s0 * LD + j]; a1 += Vc[s1 * LD + j]; }
-                        }
-                        x[c][0] = a0;
-                        x[c][1] = a1;
-                    }
-                } else {                                   // D = product of the children's messages
-                    double d0 = s0 < S ? 1.0 : 0.0, d1 = s1 < S ? 1.0 : 0.0;
-                    int E = 0;
-                    const int e1 = t.ch_off[u + 1];
-                    for (int e = t.ch_off[u]; e < e1; ++e) {
-                        const double* mc = msg + size_t(t.ch[e]) * SP;
-                        d0 *= mc[s0];
-                        d1 *= mc[s1];
-                        const double mx = warp_max(fmax(d0, d1));
-                        if (mx > 0.0 && mx < 0x1p-256) {
-                            d0 *= 0x1p256;
-                            d1 *= 0x1p256;
-                            E += 256;
-                        }
-                    }
-                    if (lane == 0 && E) atomicAdd(&sE, E);
-                    if (u == t.root) {                     // L = pi . D
-                        const double v = warp_sum((s0 < S ? f.pi[s0] * d0 : 0.0) + (s1 < S ? f.pi[s1] * d1 : 0.0));
-                        if (lane == 0) sL = v;
-                        continue;
-                    }
-                    dv[s0] = d0;
-                    dv[s1] = d1;
-                    __syncwarp();
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) {
-                        if (c >= ncu) break;
-                        const double* Vc = bgn ? V[NT - 1] : V[c];
-                        double a0 = 0.0, a1 = 0.0;
-                        const double* v0 = Vc + s0 * LD;
-                        const double* v1 = Vc + s1 * LD;
-#pragma unroll 16
-                        for (int j = 0; j < SP; ++j) {
-                            const double dj = dv[j];
-                            a0 = fma(v0[j], dj, a0);
-                            a1 = fma(v1[j], dj, a1);
-                        }
-                        x[c][0] = a0;
-                        x[c][1] = a1;
-                    }
-                }
-                const double tb = bl[u];
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if (c >= ncu) break;
-                    const double* lc = bgn ? lam[NT - 1] : lam[c];
-                    xv[c * SP + s0] = x[c][0] * exp(lc[s0] * tb);
-                    xv[c * SP + s1] = x[c][1] * exp(lc[s1] * tb);
-                }
-                __syncwarp();
-                double m0 = 0.0, m1 = 0.0;
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    if (c >= ncu) break;
-                    double a0 = 0.0, a1 = 0.0;
-                    const double* u0 = (bgn ? U[NT - 1] : U[c]) + s0 * LD;
-                    const double* u1 = (bgn ? U[NT - 1] : U[c]) + s1 * LD;
-                    const double* xc = xv + c * SP;
-#pragma unroll 16
-                    for (int j = 0; j < SP; ++j) {
-                        const double xj = xc[j];
-                        a0 = fma(u0[j], xj, a0);
-                        a1 = fma(u1[j], xj, a1);
-                    }
-                    const double wc = bgn ? 1.0 : w[c];
-                    m0 += wc * a0;
-                    m1 += wc * a1;
-                }
-                __syncwarp();                              // dv / xv are reused by this warp's next node
-                msg[size_t(u) * SP + s0] = s0 < S ? fmax(m0, 0.0) : 0.0;
-                msg[size_t(u) * SP + s1] = s1 < S ? fmax(m1, 0.0) : 0.0;
+            const int g = group(b1 - b0), gn = group(b2 - b1), b3 = lp.off[min(h + 3, lp.H)];
+            load(nx, b1 + warp * gn, gn, b2);
+            for (int i = b0 + warp * g; i < b1; i += W * g) {
+                const int count = min(g, b1 - i);
+                if (i >= b0 + W * g) load(d, i, g, b1);
+                if (g == 1) level_nodes<NC, BG, 1>(rq, f, t, bl, d, count, lane);
+                else if (GM == 2 || g == 2) level_nodes<NC, BG, GM < 2 ? 1 : 2>(rq, f, t, bl, d, count, lane);
+                else level_nodes<NC, BG, GM < 4 ? 1 : 4>(rq, f, t, bl, d, count, lane);
             }
             __syncthreads();                               // this level's messages are visible to the next
+#pragma unroll
+            for (int k = 0; k < GM; ++k) d[k] = nx[k];
+            b0 = b1; b1 = b2; b2 = b3;
         }
         if (tid == 0) out[r] = sL > 0.0 ? log(sL) - double(sE) * 0.69314718055994530942 : -1e20;
     }
@@ -668,7 +764,8 @@ struct FelDevice {
     uint8_t* d_bg = nullptr;              // [n] background flags of the run
     int* d_ev = nullptr;
     double* d_stack = nullptr;            // EBF pass: [kEbfChunk][depth][64] open partials
-    int* d_lv = nullptr;                  // level plan: [H + 1] offsets, then [n] nodes
+    int* d_lv = nullptr;                  // level plan: [H + 1] offsets
+    int4* d_lvn = nullptr;                // and its [n] nodes
     int H = 0;
     double* d_work = nullptr;             // level-synchronous pruning: [grid][n][64] messages
     int grid[2][2] = {{1, 1}, {1, 1}};    // persistent CTAs per [tested components - 1][background]
@@ -743,12 +840,17 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
     }
     for (int c = v.ch_off[v.root]; c < v.ch_off[v.root + 1]; ++c) height[v.root] = std::max(height[v.root], height[v.ch[c]] + 1);
     d->H = height[v.root] + 1;
-    std::vector<int> lv(size_t(d->H) + 1 + v.n, 0);
+    std::vector<int> lv(size_t(d->H) + 1, 0);
+    std::vector<int4> lvn(size_t(v.n));
     for (int u = 0; u < v.n; ++u) ++lv[size_t(height[u]) + 1];
     for (int h = 0; h < d->H; ++h) lv[size_t(h) + 1] += lv[size_t(h)];
     {
         std::vector<int> fill(lv.begin(), lv.begin() + d->H);
-        for (int u = 0; u < v.n; ++u) lv[size_t(d->H) + 1 + size_t(fill[size_t(height[u])]++)] = u;
+        for (int u = 0; u < v.n; ++u) {
+            const int c0 = v.ch_off[u], nc = v.ch_off[u + 1] - c0;
+            lvn[size_t(fill[size_t(height[u])]++)] =
+                make_int4(u, v.leaf[u] ? std::max(v.taxon[u], -1) : -2, nc > 0 ? v.ch[c0] : -1, nc > 1 ? v.ch[c0 + 1] : -1);
+        }
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, v.device);
@@ -765,7 +867,7 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
               take(&d->f.V, size_t(d->n_slots) * SP2) && take(&d->d_bl, v.n) && take(&d->d_bg, v.n) &&
               take(&d->d_ev, ev.size()) &&
               take(&d->d_stack, size_t(kEbfChunk) * d->depth * SP) && take(&d->d_out, d->max_req) &&
-              take(&d->d_lv, lv.size()) && take(&d->d_work, size_t(2) * std::max(sms, 1) * v.n * SP);
+              take(&d->d_lv, lv.size()) && take(&d->d_lvn, lvn.size());
     void* rq = nullptr;
     ok = ok && cudaMalloc(&rq, d->req_bytes()) == cudaSuccess;
     if (rq) d->owned.push_back(rq);
@@ -776,27 +878,34 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
     d->f.Qs = qs; d->f.Qn = qn; d->f.sq = dsq; d->f.isq = disq; d->f.pi = dpi; d->f.bg = d->d_bg;
     ok = cudaMemcpyAsync(d->d_ev, ev.data(), ev.size() * sizeof(int), cudaMemcpyHostToDevice, d->s) == cudaSuccess &&
          cudaMemcpyAsync(d->d_lv, lv.data(), lv.size() * sizeof(int), cudaMemcpyHostToDevice, d->s) == cudaSuccess &&
+         cudaMemcpyAsync(d->d_lvn, lvn.data(), lvn.size() * sizeof(int4), cudaMemcpyHostToDevice, d->s) == cudaSuccess &&
          cudaStreamSynchronize(d->s) == cudaSuccess;
     static bool configured = false;
     if (ok && !configured) {
         ok = cudaFuncSetAttribute(k_fel_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem)) == cudaSuccess &&
-             cudaFuncSetAttribute(k_site_lnl<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(1, false))) == cudaSuccess &&
-             cudaFuncSetAttribute(k_site_lnl<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(2, false))) == cudaSuccess &&
-             cudaFuncSetAttribute(k_site_lnl<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(1, true))) == cudaSuccess &&
-             cudaFuncSetAttribute(k_site_lnl<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(lv_smem(2, true))) == cudaSuccess &&
+             cudaFuncSetAttribute(k_site_lnl<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<1, false>::kSmem)) == cudaSuccess &&
+             cudaFuncSetAttribute(k_site_lnl<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<2, false>::kSmem)) == cudaSuccess &&
+             cudaFuncSetAttribute(k_site_lnl<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<1, true>::kSmem)) == cudaSuccess &&
+             cudaFuncSetAttribute(k_site_lnl<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<2, true>::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_meme_ebf<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ebf_smem(2))) == cudaSuccess &&
              cudaFuncSetAttribute(k_meme_ebf<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(ebf_smem(3))) == cudaSuccess;
         configured = ok;
     }
     int per[2][2] = {{0, 0}, {0, 0}};
-    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0][0], k_site_lnl<1, false>, kLvT, lv_smem(1, false)) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1][0], k_site_lnl<2, false>, kLvT, lv_smem(2, false)) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0][1], k_site_lnl<1, true>, kLvT, lv_smem(1, true)) == cudaSuccess &&
-         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1][1], k_site_lnl<2, true>, kLvT, lv_smem(2, true)) == cudaSuccess;
+    ok = ok && cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0][0], k_site_lnl<1, false>, LevelShape<1, false>::kThreads, LevelShape<1, false>::kSmem) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1][0], k_site_lnl<2, false>, LevelShape<2, false>::kThreads, LevelShape<2, false>::kSmem) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[0][1], k_site_lnl<1, true>, LevelShape<1, true>::kThreads, LevelShape<1, true>::kSmem) == cudaSuccess &&
+         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per[1][1], k_site_lnl<2, true>, LevelShape<2, true>::kThreads, LevelShape<2, true>::kSmem) == cudaSuccess;
     if (!ok) { *err = std::string("FEL set-up: ") + cudaGetErrorString(cudaGetLastError()); delete d; return nullptr; }
+    // the messages of kLevelCtas CTAs to an SM; of two, as before, where there is no memory for them
+    int ctas = kLevelCtas;
+    while (ctas > 1 && !take(&d->d_work, size_t(ctas) * std::max(sms, 1) * v.n * SP)) {
+        cudaGetLastError();
+        --ctas;
+    }
+    if (!d->d_work) { *err = "device allocation failed"; delete d; return nullptr; }
     for (int c = 0; c < 2; ++c)
-        for (int b = 0; b < 2; ++b)       // the workspace holds 2 x SMs CTAs
-            d->grid[c][b] = std::max(1, std::min(per[c][b], 2) * std::max(sms, 1));
+        for (int b = 0; b < 2; ++b) d->grid[c][b] = std::max(1, std::min(per[c][b], ctas) * std::max(sms, 1));
     return d;
 }
 
@@ -932,7 +1041,7 @@ bool fel_device_eval(FelDevice* d, int n_eig, const double* eig_omega, const int
                      req_slot_bg, order, &q, err))
         return false;
     cudaStream_t s = d->s;
-    const LevelPlan lp{d->H, d->d_lv, d->d_lv + d->H + 1};
+    const LevelPlan lp{d->H, d->d_lv, d->d_lvn};
     const double* bl = d->d_bl;
     for (int g = 0; g < 4; ++g) {
         const int k0 = start[g], cnt = start[g + 1] - start[g];
@@ -941,10 +1050,10 @@ bool fel_device_eval(FelDevice* d, int n_eig, const double* eig_omega, const int
         double* o = d->d_out + k0;
         const int grid = std::min(cnt, d->grid[g & 1][g >> 1]);
         switch (g) {
-            case 0: launch_k(k_site_lnl<1, false>, grid, kLvT, lv_smem(1, false), s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
-            case 1: launch_k(k_site_lnl<2, false>, grid, kLvT, lv_smem(2, false), s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
-            case 2: launch_k(k_site_lnl<1, true>, grid, kLvT, lv_smem(1, true), s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
-            default: launch_k(k_site_lnl<2, true>, grid, kLvT, lv_smem(2, true), s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
+            case 0: launch_k(k_site_lnl<1, false>, grid, LevelShape<1, false>::kThreads, LevelShape<1, false>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
+            case 1: launch_k(k_site_lnl<2, false>, grid, LevelShape<2, false>::kThreads, LevelShape<2, false>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
+            case 2: launch_k(k_site_lnl<1, true>, grid, LevelShape<1, true>::kThreads, LevelShape<1, true>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
+            default: launch_k(k_site_lnl<2, true>, grid, LevelShape<2, true>::kThreads, LevelShape<2, true>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
         }
         ++d->launches;
     }
