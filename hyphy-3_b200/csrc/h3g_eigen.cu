@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q,
         }
     }
     __syncthreads();
-    jac::sweeps(sm, js, kEigMaxSweeps);
+    jac::sweeps_sym(sm, js, kEigMaxSweeps);
     double* lk = lam + size_t(k) * SP;
     double* Uk = U + size_t(k) * SP2;
     double* UTk = UT + size_t(k) * SP2;
@@ -109,12 +109,12 @@ int launch_model_install(const ModelInstall& in, cudaStream_t s) {
 }
 
 void eigen_configure() {
-    cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem));
+    cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSymSmem));
 }
 
 int launch_model_eig(const double* Q, const double* pi, int S, int nmod, double* lam, double* U, double* UT, double* V,
                      cudaStream_t s) {
-    launch_k(k_model_eig, nmod, kET, jac::kSmem, s, Q, pi, S, lam, U, UT, V);
+    launch_k(k_model_eig, nmod, kET, jac::kSymSmem, s, Q, pi, S, lam, U, UT, V);
     return 1;
 }
 

@@ -1,6 +1,6 @@
 // h3g_jacobi.cuh — parallel cyclic Jacobi for a symmetric 64x64 FP64 matrix held in shared
-// memory by one CTA, shared by the per-site fits' eigensystems (h3g_fel.cu) and the main
-// engine's model eigensystems (h3g_eigen.cu).
+// memory by one CTA: sweeps() for the per-site fits' eigensystems (h3g_fel.cu), whose searches compare
+// likelihoods bit for bit, and sweeps_sym(), on half of the matrix, for the main engine's (h3g_eigen.cu).
 //
 // Golub & Van Loan, "Matrix Computations" (Alg. 8.5.1 / 8.5.3): one sweep = 63 rounds of 32
 // disjoint rotations (p_k, q_k), p < q, covering all 64 indices (circle schedule: seat k of round r
@@ -309,6 +309,214 @@ __device__ __forceinline__ void sweeps(double* sm, Scratch& js, int max_sweeps) 
             E[index_at(kSeats * eh + k)] = w.ex[k];
             E[index_at(32 + kSeats * eh + k)] = w.ey[k];
         }
+    __syncthreads();
+}
+
+// ------------------------------------------------------------------ symmetric form
+// The same sweeps on half of A, for callers that do not need the bits of the form above: an entry between two
+// occupants is kept once.  Entries are stored by the distance of their seats, S[kind][d][J] between seats I = J + d mod 32
+// and J, d = 1 .. 16 (16: J < 16), kind = 2 (y at I) + (y at J), so a warp's loads are 32 consecutive entries; where an
+// entry moves with its occupants is fixed, and looked up once.  The pivot of the next round, the entry of two
+// occupants of one seat, goes to S[0][0][seat].  The x of a seat is always the p of its rotation.
+// A round then moves about 600 wavefronts through shared memory instead of 1060, and the chain of the rotations bounds it:
+// 1000 cycles instead of 1540.  61 states, 2 to 3 matrices: 398 -> 265 us (with rotation() 279; with the worker's loads
+// all ahead of E 310, the rotation warp's wait behind them).  Codon generators, 400 drawn: departure from orthogonality
+// 3.3e-15 on average (worst 5.5e-15), residual 2.5e-15 (5.6e-15) of the largest entry; with sweeps() 4.0e-15 (6.2e-15)
+// and 2.8e-15 (6.1e-15).
+constexpr int kSymKind = 17 * 32;                      // entries of one kind
+constexpr int kSymBuf = 4 * kSymKind;
+constexpr size_t kSymSmem = (size_t(2) * SP * LD + 2 * kSymBuf) * sizeof(double);     // the callers' A and E, two buffers of S
+constexpr int kSymBlocks = 16 / kWarps;                // distances a worker warp updates
+
+// an occupant's place: 2 seat + (is y); where it goes after a round
+__device__ __forceinline__ int sym_next(int at) {
+    const int k = at >> 1;
+    if (at & 1) return k == 31 ? 2 * 31 : at + 2;
+    return k == 0 ? 0 : (k == 1 ? 1 : at - 2);
+}
+// where the entry between two places is kept
+__device__ __forceinline__ int sym_slot(int a, int b) {
+    int I = a >> 1, J = b >> 1, d = (I - J) & 31;
+    if (d == 0) return I;
+    if (d > 16 || (d == 16 && J >= 16)) {
+        const int x = a; a = b; b = x;
+        J = I;
+        d = 32 - d;
+    }
+    return (2 * (a & 1) + (b & 1)) * kSymKind + 32 * d + J;
+}
+
+// The rotation that annihilates a_pq, by the double angle: with h = d^2 + 4 a_pq^2, d = a_qq - a_pp, cos 2theta = |d| / sqrt(h),
+// c^2 = (1 + cos 2theta) / 2 and s = a_pq sign(d) / (c sqrt(h)); two reciprocal square roots in a row where
+// rotation() has a square root, a divide and a reciprocal square root.  One Newton step makes c^2 + s^2 = 1 to the
+// last bits.  Entries below 1e-150 (squares that the sweeps' test cannot see) count as zero.
+__device__ __forceinline__ double2 rotation_sym(double apq, double app, double aqq, double& t) {
+    const double d = aqq - app, h = fma(4.0 * apq, apq, d * d);
+    double c = 1.0, s = 0.0;
+    t = 0.0;
+    if (fabs(apq) >= 1e-150 && h <= 1e300) {
+        const double r = rsqrt(h), c2 = fma(0.5 * fabs(d), r, 0.5), rc = rsqrt(c2);
+        const double sa = (d >= 0.0 ? apq : -apq) * r;
+        c = c2 * rc;
+        s = sa * rc;
+        t = s * rc;
+        const double n = 0.5 * fma(s, s, fma(c, c, -1.0));
+        c = fma(-n, c, c);
+        s = fma(-n, s, s);
+    }
+    return make_double2(c, s);
+}
+
+// sm (kSymSmem bytes) holds A and E as for sweeps(), the results are the same: js.lam and E in place.
+__device__ __forceinline__ void sweeps_sym(double* sm, Scratch& js, int max_sweeps) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int wp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const bool worker = wp < kWarps;
+    double* S = sm + 2 * SP * LD;
+    const int eh = (wp >> 1) & (kGroups - 1), er = 32 * (wp & 1) + lane, xe = SP * eh + er;
+    double* E = sm + SP * LD + er * LD;
+    double ex[kSeats], ey[kSeats];
+#pragma unroll
+    for (int k = 0; k < kSeats; ++k) {
+        ex[k] = E[index_at(kSeats * eh + k)];
+        ey[k] = E[index_at(32 + kSeats * eh + k)];
+    }
+    // a place's index in round 0
+    auto index_of = [](int at) { return index_at((at & 1) * 32 + (at >> 1)); };
+    for (int e = tid; e < 2 * kSymBuf; e += kThreads) S[e] = 0.0;
+    __syncthreads();
+    double tot = 0.0;
+    for (int e = tid; e < SP * SP; e += kThreads) {
+        const int a = e >> 6, b = e & 63;
+        if (a >= b) continue;
+        const double v = sm[index_of(a) * LD + index_of(b)];
+        S[sym_slot(a, b)] = v;
+        tot += 2.0 * v * v;
+    }
+    if (tid < SP) { const double v = sm[tid * LD + tid]; tot = fma(v, v, tot); }
+    // workers: the slots that their blocks' entries move to; the rotation warp: its next pivot's block and where a zero goes
+    int to[kSymBlocks][4], from[kSymBlocks], zero = 0, ahead[4];
+    double gx = 0.0, gy = 0.0, dx = 0.0, dy = 0.0;     // rotation warp: the seat's diagonal before and after the round to come
+    bool xa = true, xb = false;                        // the next pivot is between an x and a y
+#pragma unroll
+    for (int i = 0; i < kSymBlocks; ++i) {
+        const int d = 1 + (wp & (kWarps - 1)) + kWarps * i, I = (lane + d) & 31;
+        from[i] = 32 * d + lane;
+#pragma unroll
+        for (int e = 0; e < 4; ++e)                    // (distance 16, J >= 16: zeros, kept where they are)
+            to[i][e] = d == 16 && lane >= 16 ? e * kSymKind + from[i] : sym_slot(sym_next(2 * I + (e >> 1)), sym_next(2 * lane + (e & 1)));
+#pragma unroll
+        for (int e = 0; e < 4; ++e) pin(to[i][e]);
+    }
+    {
+        const int k = lane, sa = k == 0 ? 0 : (k == 31 ? 31 : k + 1), sb = k == 0 ? 1 : k - 1;
+        xa = k != 31;
+        xb = k == 0;
+        for (int e = 0; e < 4; ++e) ahead[e] = sym_slot(2 * sa + (e >> 1), 2 * sb + (e & 1));
+        zero = sym_slot(sym_next(2 * k), sym_next(2 * k + 1));
+        if (!worker) {
+            gx = sm[index_at(k) * (LD + 1)];
+            gy = sm[index_at(32 + k) * (LD + 1)];
+        }
+    }
+    double part = worker ? tot : 0.0, rest = worker ? 0.0 : tot;
+    for (int o = 16; o > 0; o >>= 1) rest += __shfl_xor_sync(0xffffffffu, rest, o);
+    if (!worker && lane == 0) js.up[0][0] = rest;      // the rotation warp's share of the total
+    tot = block_sum(part, js.red);
+    tot += js.up[0][0];
+    __syncthreads();
+    int par = 0;                                       // parity of the round to apply: the buffer that holds it
+    bool moved = false;
+    for (int sweep = 0; sweep < max_sweeps; ++sweep) {
+        const double* cur = S + (par ? kSymBuf : 0);
+        double off = 0.0;
+        if (worker)
+            for (int e = tid; e < kSymBuf; e += kWorkers) off = fma(cur[e], cur[e], off);
+        off = 2.0 * block_sum(off, js.red);
+        if (off <= 1e-30 * tot || off == 0.0) break;
+        if (!moved && !worker) {
+            double t;
+            const double a = cur[lane];
+            js.cs[par][lane] = rotation_sym(a, gx, gy, t);
+            dx = fma(-t, a, gx);
+            dy = fma(t, a, gy);
+        }
+        for (int r = 0; r < SP - 1; ++r) {
+            __syncthreads();                           // this round's entries and rotations, and the other buffer, are ready
+            const double* A = S + (par ? kSymBuf : 0);
+            double* B = S + (par ? 0 : kSymBuf);
+            const double2* cs = js.cs[par];
+            if (worker) {
+                {   // E first: the rotation warp's few loads then go ahead of the workers' many
+                    const double2* ce = cs + kSeats * eh;
+                    if (moved) {                       // the entries of E that the last round passed on
+                        if (eh < kGroups - 1) ex[kSeats - 1] = js.up[par][xe];
+                        if (eh > 0) ey[0] = js.down[par][xe];
+                    }
+#pragma unroll
+                    for (int k = 0; k < kSeats; ++k) {
+                        const double2 q = ce[k];
+                        const double x = ex[k], y = ey[k];
+                        ex[k] = rot_p(q, x, y);
+                        ey[k] = rot_q(q, x, y);
+                    }
+                    if (eh > 0) js.up[par ^ 1][xe - SP] = ex[0];
+                    if (eh < kGroups - 1) js.down[par ^ 1][xe + SP] = ey[kSeats - 1];
+                    const double x0 = ex[0], x1 = ex[1], y_last = ey[kSeats - 1];
+#pragma unroll
+                    for (int k = 0; k < kSeats - 1; ++k) ex[k] = ex[k + 1];
+                    if (eh == 0) ex[0] = x0;
+                    ex[kSeats - 1] = y_last;
+#pragma unroll
+                    for (int k = kSeats - 1; k > 0; --k) ey[k] = ey[k - 1];
+                    ey[0] = x1;
+                }
+                const double2 rJ = cs[lane];
+#pragma unroll
+                for (int i = 0; i < kSymBlocks; ++i) {
+                    const double2 rI = cs[(lane + 1 + wp + kWarps * i) & 31];
+                    const double a = A[from[i]], b = A[from[i] + kSymKind], c = A[from[i] + 2 * kSymKind], d = A[from[i] + 3 * kSymKind];
+                    const double m0 = rot_p(rJ, a, b), m1 = rot_q(rJ, a, b);
+                    const double m2 = rot_p(rJ, c, d), m3 = rot_q(rJ, c, d);
+                    B[to[i][0]] = rot_p(rI, m0, m2);
+                    B[to[i][1]] = rot_p(rI, m1, m3);
+                    B[to[i][2]] = rot_q(rI, m0, m2);
+                    B[to[i][3]] = rot_q(rI, m1, m3);
+                }
+            } else {
+                const int k = lane;
+                const double2 ra = cs[k == 0 ? 0 : (k == 31 ? 31 : k + 1)], rb = cs[k == 0 ? 1 : k - 1];
+                const double v0 = A[ahead[0]], v1 = A[ahead[1]], v2 = A[ahead[2]], v3 = A[ahead[3]];
+                const double up = __shfl_down_sync(0xffffffffu, dx, 1), down = __shfl_up_sync(0xffffffffu, dy, 1);
+                gx = k == 0 ? dx : (k == 31 ? dy : up);
+                gy = k == 0 ? up : down;
+                const double a0 = xa ? ra.x : ra.y, a1 = xa ? -ra.y : ra.x, b0 = xb ? rb.x : rb.y, b1 = xb ? -rb.y : rb.x;
+                const double apq = fma(a0, fma(b0, v0, __dmul_rn(b1, v1)), __dmul_rn(a1, fma(b0, v2, __dmul_rn(b1, v3))));
+                double t;
+                js.cs[par ^ 1][k] = rotation_sym(apq, gx, gy, t);
+                B[zero] = 0.0;
+                dx = fma(-t, apq, gx);
+                dy = fma(t, apq, gy);
+            }
+            moved = true;
+            par ^= 1;
+        }
+        __syncthreads();                               // the sweep's last round is complete
+    }
+    if (!worker) {
+        js.lam[index_at(lane)] = gx;
+        js.lam[index_at(32 + lane)] = gy;
+    } else {
+        if (moved) {
+            if (eh < kGroups - 1) ex[kSeats - 1] = js.up[par][xe];
+            if (eh > 0) ey[0] = js.down[par][xe];
+        }
+#pragma unroll
+        for (int k = 0; k < kSeats; ++k) {             // a whole number of sweeps: the seats of round 0 again
+            E[index_at(kSeats * eh + k)] = ex[k];
+            E[index_at(32 + kSeats * eh + k)] = ey[k];
+        }
+    }
     __syncthreads();
 }
 
