@@ -1969,6 +1969,7 @@ static h3g_status batch_prepare(h3g_batch* b) {
 // The workspace view gene g evaluates in: its slot's buffers, its own branch lengths, chunking and groups.
 static Work batch_view(const h3g_batch* b, const h3g_batch::Slot& sl, int g) {
     Work w = sl.w;
+    w.share = int(b->slots.size());
     w.bl = b->probs[g]->d_bl;
     w.nchunk = b->gene_layout[g].nchunk;
     w.chunk = b->gene_layout[g].chunk;

@@ -122,6 +122,7 @@ struct Model {
 };
 
 struct Work {
+    int share = 1;           // evaluations that run side by side (a batch's slots): none has to fill the GPU by itself
     const double* bl;        // [n]
     double* P;               // [M][n][64*64]
     double* PT;              // [M][n][64*64]

@@ -1025,13 +1025,15 @@ int launch_prep_given_P(const Topo& t, const Work& w, cudaStream_t s) {
     return 1;
 }
 // Tiles per CTA of the pruning kernels: one while the level leaves SMs without a CTA to spare, up to 8 (four waves of
-// two CTAs per SM are left then, so an uneven last wave costs little).
-static int tiles_per_cta(int ntile, int nodes, int M) {
-    const long items = long(ntile) * nodes * M;
-    return int(std::max(1L, std::min({8L, long(ntile), items / (4 * 2 * 148)})));
+// two CTAs per SM are left then, so an uneven last wave costs little).  In a batch the other slots fill those waves, so
+// a launch keeps its share of them: 24 genes of 8 to 512 taxa in 8 slots, two evaluations, 44.0 -> 40.4 ms (twice the
+// tiles 40.4, half the CTAs 42.3, twice the CTAs 41.6).
+static int tiles_per_cta(int ntile, int nodes, int M, int share) {
+    const long items = long(ntile) * nodes * M, ctas = std::max(148L, 4L * 2 * 148 / share);
+    return int(std::max(1L, std::min({8L, long(ntile), items / ctas})));
 }
 int launch_inside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_nodes, int count, cudaStream_t s) {
-    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M);
+    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M, w.share);
     launch_k(k_inside, dim3((nt + k - 1) / k, count, md.M), 256, 0, s, t, md, w, d_nodes, k);
     return 1;
 }
@@ -1040,7 +1042,7 @@ int launch_root(const Topo& t, const Model& md, const Work& w, cudaStream_t s) {
     return 1;
 }
 int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_kids, int count, cudaStream_t s) {
-    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M);
+    const int nt = t.Pp / kTileP, k = tiles_per_cta(nt, count, md.M, w.share);
     launch_k(k_outside, dim3((nt + k - 1) / k, count, md.M), 256, 0, s, t, md, w, d_kids, k);
     return 1;
 }
