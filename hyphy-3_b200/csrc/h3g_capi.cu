@@ -1112,7 +1112,7 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
         if (d->is_test) vec(in, d->is_test, size_t(pr->n), pr->m_it, 1, 0);
         if (d->branch_classes) vec(in, d->branch_classes, size_t(pr->n + 1) * sizeof(int32_t), pr->m_br, 1, 0);
         launch_model_install(in, s);
-        if (dev_eig) launch_model_eig(pr->m_Q, pr->m_pi, S, nm, pr->m_lam, pr->m_U, pr->m_UT, pr->m_V, s);
+        if (dev_eig) launch_model_eig(pr->m_Q, pr->m_pi, S, nm, pr->m_lam, pr->m_U, pr->m_UT, pr->m_V, d->precision == H3G_PREC_MIXED, s);
         H3G_TRY_CUDA(ctx, cudaGetLastError());
         if (n_dq > 0) {
             // dense directions [n_dirs][nm], then the per-model ones [nm]

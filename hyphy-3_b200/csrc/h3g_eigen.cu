@@ -18,7 +18,11 @@ namespace {
 constexpr int kET = jac::kThreads;
 constexpr int kEigMaxSweeps = 30;
 
-// grid (nmod), block kET: one model per CTA.
+// grid (nmod), block kET: one model per CTA.  kSym: by the sweeps on half of the matrix (265 us instead of 398 us).  They are
+// as accurate, but not the same bits, and a gradient over branches far shorter than the changes on them amplifies the last bits
+// of an eigensystem by up to 1e6; so the FP64 path keeps the rotations it has always had, and the mixed path, whose
+// own rounding is 1e-7, takes the faster ones.
+template <bool kSym>
 __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q, const double* __restrict__ pi, int S,
                                                    double* lam, double* U, double* UT, double* V) {
     pdl_enter();
@@ -51,7 +55,8 @@ __global__ void __launch_bounds__(kET) k_model_eig(const double* __restrict__ Q,
         }
     }
     __syncthreads();
-    jac::sweeps_sym(sm, js, kEigMaxSweeps);
+    if constexpr (kSym) jac::sweeps_sym(sm, js, kEigMaxSweeps);
+    else jac::sweeps(sm, js, kEigMaxSweeps);
     double* lk = lam + size_t(k) * SP;
     double* Uk = U + size_t(k) * SP2;
     double* UTk = UT + size_t(k) * SP2;
@@ -109,12 +114,14 @@ int launch_model_install(const ModelInstall& in, cudaStream_t s) {
 }
 
 void eigen_configure() {
-    cudaFuncSetAttribute(k_model_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSymSmem));
+    cudaFuncSetAttribute(k_model_eig<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem));
+    cudaFuncSetAttribute(k_model_eig<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSymSmem));
 }
 
 int launch_model_eig(const double* Q, const double* pi, int S, int nmod, double* lam, double* U, double* UT, double* V,
-                     cudaStream_t s) {
-    launch_k(k_model_eig, nmod, kET, jac::kSymSmem, s, Q, pi, S, lam, U, UT, V);
+                     bool mixed, cudaStream_t s) {
+    if (mixed) launch_k(k_model_eig<true>, nmod, kET, jac::kSymSmem, s, Q, pi, S, lam, U, UT, V);
+    else launch_k(k_model_eig<false>, nmod, kET, jac::kSmem, s, Q, pi, S, lam, U, UT, V);
     return 1;
 }
 

@@ -8,9 +8,9 @@
 //                  rescaling, then the message P_u D_u for the parent (likelihood.hpp:500-597)
 //   k_root         L = pi . D_root, log-sum-exp over rate classes, per-pattern scale
 //                  factors f = w * post / L (likelihood.hpp:599-610, busted.hpp:1346-1375)
-//   k_outside      one launch per depth level: V_c = 2^{e_u} U_u o prod_{s != c} P_s D_s,
+//   k_outside      one launch per depth level, internal children: V_c = 2^{e_u} U_u o prod_{s != c} P_s D_s,
 //                  U_c = P_c^T V_c (likelihood.hpp:612-761)
-//   k_accumA       A_{m,b} = sum_p f V D^T  (likelihood.hpp:1435 generalised)
+//   k_accumA_int, k_accumA_leaf   A_{m,b} = sum_p f V D^T  (likelihood.hpp:1435 generalised)
 //   k_frechet      dlnL/dt_b = <A, dP>; spectral Frechet pieces U^T A V^T o E
 //                  (likelihood.hpp:1428-1471)
 //   k_hsum, k_dir, k_small   fixed-order reductions -> lnL, gradients

@@ -1,6 +1,7 @@
 // h3g_jacobi.cuh — parallel cyclic Jacobi for a symmetric 64x64 FP64 matrix held in shared
 // memory by one CTA: sweeps() for the per-site fits' eigensystems (h3g_fel.cu), whose searches compare
-// likelihoods bit for bit, and sweeps_sym(), on half of the matrix, for the main engine's (h3g_eigen.cu).
+// likelihoods bit for bit, and for the main engine's FP64 models (h3g_eigen.cu); sweeps_sym(), on half of the
+// matrix, for its mixed-precision models.
 //
 // Golub & Van Loan, "Matrix Computations" (Alg. 8.5.1 / 8.5.3): one sweep = 63 rounds of 32
 // disjoint rotations (p_k, q_k), p < q, covering all 64 indices (circle schedule: seat k of round r
