@@ -62,10 +62,8 @@ WORKLOADS = {
 # the padded pattern count (5120 / 512): these stages stream per-pattern partials, so their traffic is
 # proportional to the patterns processed.
 MEASURED_TRAFFIC = {
-    (1, "mixed"): {"inside": 19.5e6, "outside": 36.2e6, "accum_A": 49.4e6},
-    (1, "fp64"): {"inside": 36.5e6, "outside": 68.7e6, "accum_A": 98.3e6},
-    (3, "mixed"): {"inside": 14.724e9, "outside": 28.220e9, "accum_A": 18.835e9},
-    (3, "fp64"): {"inside": 29.259e9, "outside": 48.234e9, "accum_A": 34.790e9},
+    (1, "mixed"): {"inside": 19.5e6},
+    (3, "mixed"): {"inside": 14.724e9},
     # alignment compression, 1024 taxa x 100000 codons, captured at full size (one pass:
     # dram__bytes_read.sum + dram__bytes_write.sum of the call's launch)
     ("compress", "translate"): 479.30e6,
@@ -176,7 +174,9 @@ def stage_work(aln_P: int, tree, M: int, elem_bytes: int = 8) -> dict:
     reads the messages of internal children, writes D and (non-root) the
     message P*D; the outside stage reads U of the parent and the sibling
     messages, writes the scaled outside vector of every child and U of
-    internal children; accum_A reads V and D of every branch.
+    internal children; accum_A reads V and D of every branch.  No outside vector is
+    stored for a leaf (FP64) or a leaf with one sibling (mixed): accum_A reads the
+    parent's U and the siblings' messages for it.
     """
     S = 61
     nodes = tree.nodes
@@ -189,18 +189,20 @@ def stage_work(aln_P: int, tree, M: int, elem_bytes: int = 8) -> dict:
         int_kids = [c for c in nd.children if not nodes[c].is_leaf]
         ins_b += vec * (len(int_kids) + 1 + (nd.id != root))
         ins_f += 2 * S * S * (nd.id != root)
-        k = len(nd.children)
-        out_b += vec * (1 + k)
-        for c in nd.children:
-            out_b += vec * sum(1 for s in nd.children if s != c and not nodes[s].is_leaf)
+        kids = nd.children
+        stored = [c for c in kids if not nodes[c].is_leaf or (elem_bytes == 4 and len(kids) != 2)]
+        out_b += vec * (1 + len(stored)) if stored else 0
+        for c in kids:
+            siblings = sum(1 for s in kids if s != c and not nodes[s].is_leaf)
+            if c in stored:
+                out_b += vec * siblings
+                acc_b += vec * (1 if nodes[c].is_leaf else 2)
+            else:
+                acc_b += vec * (siblings + (nd.id != root))
+            acc_f += 2 * S * S if elem_bytes == 4 or not nodes[c].is_leaf else S     # FP64: leaf columns are sums
             if not nodes[c].is_leaf:
                 out_b += vec
                 out_f += 2 * S * S
-    for nd in nodes:
-        if nd.id == root:
-            continue
-        acc_b += vec * (2 if not nd.is_leaf else 1)
-        acc_f += 2 * S * S
     return {"inside": (ins_b * cols, ins_f * cols), "outside": (out_b * cols, out_f * cols),
             "accum_A": (acc_b * cols, acc_f * cols)}
 

@@ -621,7 +621,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_outside_mx(Topo t, Model md, Wo
 // A leaf with one sibling has no stored V: its U and the sibling's message (a stored tile, or rows of FP32 P^T by the
 // sibling's states) are multiplied as they are split, scaled by f 2^(EL - EV) in two factors so that no power of two
 // leaves the FP32 range.  Storing V for them was half of the outside pass's items and a third of its traffic:
-// with 1024 taxa x 5000 codons the outside pass went from 8.9 to 5.4 ms and this kernel stayed at 6.1 ms (the sibling
+// with 1024 taxa x 5000 codons the outside pass went from 8.9 to 5.4 ms and this kernel from 6.0 to 6.5 ms (the sibling
 // leaf's rows gathered into shared memory one tile ahead; gathered entry by entry in the split it took 8.0 ms).
 //
 // Pipeline (one CTA per SM): two groups of 8 warps take turns with the 64-pattern tiles, each with its own
