@@ -51,15 +51,22 @@ __device__ __forceinline__ void few_msg(double (&x)[kFewStates], const Topo& t, 
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
-// v *= x, kept away from underflow by powers of two; returns the shift applied
-__device__ __forceinline__ int few_mul(double (&v)[kFewStates], const double (&x)[kFewStates]) {
+// v away from underflow by a power of two, as the 64-state passes scale a column; returns the shift applied
+__device__ __forceinline__ int few_scale(double (&v)[kFewStates]) {
     double mx = 0.0;
 #pragma unroll
-    for (int q = 0; q < kFewStates; ++q) { v[q] *= x[q]; mx = fmax(mx, v[q]); }
+    for (int q = 0; q < kFewStates; ++q) mx = fmax(mx, v[q]);
     if (mx <= 0.0 || mx >= 0x1p-256) return 0;
+    const int sh = -ilogb(mx) - 1;
 #pragma unroll
-    for (int q = 0; q < kFewStates; ++q) v[q] *= 0x1p256;
-    return 256;
+    for (int q = 0; q < kFewStates; ++q) v[q] = ldexp(v[q], sh);
+    return sh;
+}
+// v *= x; returns the shift applied
+__device__ __forceinline__ int few_mul(double (&v)[kFewStates], const double (&x)[kFewStates]) {
+#pragma unroll
+    for (int q = 0; q < kFewStates; ++q) v[q] *= x[q];
+    return few_scale(v);
 }
 
 // The upper left corner of a padded 64 x 64 matrix (the same for the whole warp), and its product with x.  Loaded
@@ -96,7 +103,7 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_inside_few(Topo t, Model md,
             const int e0 = d.y <= -2 ? w.Ecum[col_off(-(d.y + 2), m, M, t.Pp) + p] : 0;
             const int e1 = d.w <= -2 ? w.Ecum[col_off(-(d.w + 2), m, M, t.Pp) + p] : 0;
             if (k0 < k1) few_msg(v, t, w, m, M, make_int2(d.x, d.y), p, s0);
-            int eown = 0, ecum = e0 + e1;
+            int eown = few_scale(v), ecum = e0 + e1;
             if (k0 + 1 < k1) {
                 few_msg(x, t, w, m, M, make_int2(d.z, d.w), p, s1);
                 eown += few_mul(v, x);
