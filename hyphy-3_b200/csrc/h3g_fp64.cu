@@ -305,17 +305,20 @@ __device__ __forceinline__ int renorm_cols(double (&v)[8], double* smax, int g, 
     }
     return 0;
 }
-// The same unless every thread's eight states reach 2^-340: one barrier instead of the exchange.  A column is then
-// left with a maximum of 2^-340 at least; the product of two such stays far from the end of the range, and
+// One barrier, a vote: does every thread have a state of 2^-340 or more among its eight?  A column then has a maximum
+// of 2^-340 at least and needs no scaling: the product of two such stays far from the end of the range, and
 // scaling by powers of two changes no result.  (At 2^-256, the bound of the exchange itself, states 60 powers of
 // two below their column's maximum sent most tiles through it.)  Doubles >= 0 compare like the integers of their
 // upper words.  S: states; a group beyond them does not count.
-__device__ __forceinline__ int renorm_if_small(double (&v)[8], double* smax, int g, int lane, int S) {
+__device__ __forceinline__ bool none_small(const double (&v)[8], int g, int S) {
     int hi = 8 * g >= S ? INT_MAX : 0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) hi = max(hi, __double2hiint(v[q]));
-    if (__syncthreads_and(hi >= ((1023 - 340) << 20))) return 0;
-    return renorm_cols(v, smax, g, lane);
+    return __syncthreads_and(hi >= ((1023 - 340) << 20));
+}
+// The vote, and the exchange unless it passes.
+__device__ __forceinline__ int renorm_if_small(double (&v)[8], double* smax, int g, int lane, int S) {
+    return none_small(v, g, S) ? 0 : renorm_cols(v, smax, g, lane);
 }
 
 // Partial tiles of the FP64 pruning CTAs in shared memory: [64 states][32 patterns] with a row
@@ -394,7 +397,19 @@ __global__ void __launch_bounds__(256, 2) k_inside(Topo t, Model md, Work w, con
         double v[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) v[q] = two ? a0[q] * a1[q] : a0[q];
-        int eown = renorm_if_small(v, smax, g, lane, t.S);  // (its barrier: the last tile's products are done with sD)
+        int eown = 0;
+        if (!none_small(v, g, t.S)) {                      // (its barrier: the last tile's products are done with sD)
+            // the first message by itself, then the product: two columns of a matrix's tiny entries, 2^-537 and
+            // below, have a product that is no double
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v[q] = a0[q];
+            eown = renorm_cols(v, smax, g, lane);
+            if (two) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) v[q] *= a1[q];
+                eown += renorm_cols(v, smax, g, lane);
+            }
+        }
         for (int k = k0 + 2; k < k1; ++k) {
             const int2 d = t.kdesc[k];
             double x[8];

@@ -34,7 +34,7 @@ def _site_lnl(parent, states, P, pi):
 
 
 @pytest.mark.parametrize("tree", sorted(TREES))
-@pytest.mark.parametrize("S", [2, 4])
+@pytest.mark.parametrize("S", [2, 4, 5, 61])
 @pytest.mark.parametrize("mag,rare", [(1e-20, False), (1e-120, False), (1e-150, False), (1e-150, True), (1e-250, True)])
 def test_transition_probabilities_near_the_range_ends(tree, S, mag, rare):
     from hyphy3 import _capi
