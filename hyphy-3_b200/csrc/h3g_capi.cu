@@ -58,6 +58,9 @@ struct DevArena {
 
 }  // namespace
 
+// Leaf entries of a children list (split_kids): where they start, how many, and how many more of large nodes.
+struct h3g_leaf_pairs { int at = 0, n = 0, n_many = 0; };
+
 struct h3g_problem {
     h3g_ctx* ctx = nullptr;
     h3g_batch* batch = nullptr;        // the batch this problem evaluates in (its workspace lives there)
@@ -69,7 +72,7 @@ struct h3g_problem {
     DevArena topo_mem, model_mem, work_mem;
     int *d_ch_off = nullptr, *d_ch = nullptr, *d_iidx = nullptr, *d_taxon = nullptr, *d_in_nodes = nullptr;
     int* d_out_split = nullptr;        // out_nodes: the internal ones (levels out_int_off), then leaf pairs (split_kids)
-    int pairs_at = 0, n_pairs = 0;
+    h3g_leaf_pairs pairs;
     int* d_parent = nullptr;
     uint8_t* d_leaf = nullptr;
     int2* d_kdesc = nullptr;
@@ -145,7 +148,7 @@ struct h3g_problem {
     int *d_ck_iidx = nullptr, *d_ck_vidx = nullptr, *d_ck_lists = nullptr;
     int2* d_ck_kdesc = nullptr;
     int4* d_ck_info = nullptr;
-    struct CkOffsets { int in, out, pairs_at, n_pairs, acc; std::vector<int> out_int_off; int in_info, out_info, in_next, in_heads, n_in_heads, out_next, out_heads, n_out_heads; };
+    struct CkOffsets { int in, out, acc; h3g_leaf_pairs pairs; std::vector<int> out_int_off; int in_info, out_info, in_next, in_heads, n_in_heads, out_next, out_heads, n_out_heads; };
     std::vector<CkOffsets> ck_off;
     uint64_t ws_bytes = 0, full_bytes = 0;
     Topo topo() const {
@@ -227,9 +230,10 @@ extern "C" h3g_status h3g_ctx_destroy(h3g_ctx* ctx) {
 }
 
 // kids (children grouped by parent, levels off): the internal ones by level (int_off) and after them, from an even
-// position on, the leaves as pairs: the two of a node with just these, else (leaf, -1).
-static void split_kids(const std::vector<int>& kids, const std::vector<int>& off, const uint8_t* leaf, const int* parent,
-                       const std::vector<int>& n_kids, std::vector<int>& split, std::vector<int>& int_off, int& pairs_at, int& n_pairs) {
+// position on, the leaves as pairs: the two of a node with just these, else (leaf, -1).  The n_many leaves of nodes with
+// more than kFewKids children come last.
+static h3g_leaf_pairs split_kids(const std::vector<int>& kids, const std::vector<int>& off, const uint8_t* leaf, const int* parent,
+                            const std::vector<int>& n_kids, std::vector<int>& split, std::vector<int>& int_off) {
     split.clear();
     int_off.assign(1, 0);
     for (size_t l = 0; l + 1 < off.size(); ++l) {
@@ -238,16 +242,21 @@ static void split_kids(const std::vector<int>& kids, const std::vector<int>& off
         int_off.push_back(int(split.size()));
     }
     if (split.size() % 2) split.push_back(-1);
-    pairs_at = int(split.size());
-    for (size_t k = 0; k < kids.size(); ++k) {
-        const int c = kids[k];
-        if (!leaf[c]) continue;
-        const bool pair = n_kids[size_t(parent[c])] == 2 && k + 1 < kids.size() && parent[kids[k + 1]] == parent[c] && leaf[kids[k + 1]];
-        split.push_back(c);
-        split.push_back(pair ? kids[k + 1] : -1);
-        k += pair ? 1 : 0;
+    h3g_leaf_pairs lp;
+    lp.at = int(split.size());
+    for (const bool many : {false, true}) {
+        const size_t from = split.size();
+        for (size_t k = 0; k < kids.size(); ++k) {
+            const int c = kids[k], nk = n_kids[size_t(parent[c])];
+            if (!leaf[c] || (nk > kFewKids) != many) continue;
+            const bool pair = nk == 2 && k + 1 < kids.size() && parent[kids[k + 1]] == parent[c] && leaf[kids[k + 1]];
+            split.push_back(c);
+            split.push_back(pair ? kids[k + 1] : -1);
+            k += pair ? 1 : 0;
+        }
+        (many ? lp.n_many : lp.n) = int(split.size() - from) / 2;
     }
-    n_pairs = (int(split.size()) - pairs_at) / 2;
+    return lp;
 }
 
 extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_t* parent, const uint8_t* is_leaf,
@@ -330,7 +339,7 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         }
         std::vector<int> n_kids(n);
         for (int i = 0; i < n; ++i) n_kids[i] = int(kids[i].size());
-        split_kids(pr->out_nodes, pr->out_off, is_leaf, parent, n_kids, pr->out_split, pr->out_int_off, pr->pairs_at, pr->n_pairs);
+        pr->pairs = split_kids(pr->out_nodes, pr->out_off, is_leaf, parent, n_kids, pr->out_split, pr->out_int_off);
         pr->parent_h.assign(parent, parent + n);
         if (n_patterns > 0) pr->states_pm.assign(states, states + size_t(n_patterns) * n_taxa);
         // patterns, taxon-major with padding (missing data, weight 0)
@@ -746,7 +755,7 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
         o.in = int(lists.size());
         lists.insert(lists.end(), B.in_nodes.begin(), B.in_nodes.end());
         std::vector<int> split;
-        split_kids(B.out_kids, B.out_lv, pr->leaf.data(), pr->parent_h.data(), n_kids, split, o.out_int_off, o.pairs_at, o.n_pairs);
+        o.pairs = split_kids(B.out_kids, B.out_lv, pr->leaf.data(), pr->parent_h.data(), n_kids, split, o.out_int_off);
         if (lists.size() % 2) lists.push_back(-1);              // the pairs are read as int2
         o.out = int(lists.size());
         lists.insert(lists.end(), split.begin(), split.end());
@@ -1220,7 +1229,7 @@ static int enqueue_eval_on(h3g_problem* pr, unsigned want, bool from_given_P, cu
         mark(ST_ACCUM_A, mixed ? launch_accumA_mixed(t, md, w, mwk, nullptr, 0, s)
                          : few ? launch_accumA_few(t, md, w, s)
                                : launch_accumA_fp64(t, md, w, pr->d_out_split, pr->out_int_off.back(),
-                                                    reinterpret_cast<const int2*>(pr->d_out_split + pr->pairs_at), pr->n_pairs, s));
+                                                    reinterpret_cast<const int2*>(pr->d_out_split + pr->pairs.at), pr->pairs.n, pr->pairs.n_many, s));
         mark(ST_FRECHET, launch_frechet(t, md, w, global ? 1 : 0, s));
         if (side) cudaStreamWaitEvent(s, pr->ev_join, 0);
         if (global) mark(ST_HSUM, launch_global(t, md, w, s));
@@ -1304,7 +1313,7 @@ static int enqueue_eval_ck(h3g_problem* pr, unsigned want, bool from_given_P, cu
                         l += launch_outside_fp64(t, md, w, lists + o.out + o.out_int_off[lv], cnt, s);
                 // the branches below this block's nodes: V or the parents' U and the siblings' messages, and their own D, are here
                 l += launch_accumA_fp64(t, md, w, lists + o.out, o.out_int_off.back(),
-                                        reinterpret_cast<const int2*>(lists + o.out + o.pairs_at), o.n_pairs, s);
+                                        reinterpret_cast<const int2*>(lists + o.out + o.pairs.at), o.pairs.n, o.pairs.n_many, s);
             }
         }
         mark(ST_OUTSIDE, l);

@@ -20,9 +20,11 @@ int launch_inside_fp64(const Topo& t, const Model& md, const Work& w, const int*
 int launch_root(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 // d_kids: internal children of one depth's nodes
 int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int* d_kids, int count, cudaStream_t s);
-// A of the listed internal branches, and of leaves: entries of one leaf (y = -1) or the two of a two-leaf node
+// A of the listed internal branches, and of leaves: n_leaves entries of one leaf (y = -1) or the two of a two-leaf node,
+// then n_many leaves of nodes with more than kFewKids children
+constexpr int kFewKids = 9;
 int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_internal, int n_internal, const int2* d_leaves,
-                       int n_leaves, cudaStream_t s);
+                       int n_leaves, int n_many, cudaStream_t s);
 // The same passes for t.S <= kFewStates, one launch each (h3g_few.cu)
 int launch_inside_few(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
 int launch_outside_few(const Topo& t, const Model& md, const Work& w, cudaStream_t s);
