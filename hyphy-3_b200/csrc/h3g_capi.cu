@@ -602,6 +602,9 @@ struct WsLayout {
     }
 };
 
+// Patterns per A-accumulation chunk come in multiples of this: two stages of the FP64 kernels, one tile of the mixed one.
+constexpr int kChunkGrain = 64;
+
 // part_nodes / vf_nodes: partial slots of internal nodes and gradient-operand slots (NI and n, or
 // fewer under a checkpoint plan).
 static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, int K, int nmod, int ndirs, const h3g_tuning& tu,
@@ -618,11 +621,10 @@ static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, 
     L.gt = size_t(M) * n;
     // enough A chunks for ~600 CTAs, never below 64 patterns per chunk (two stages: a chunk of 256 left the smallest
     // genes with 8 stages in a row on a handful of CTAs)
-    constexpr size_t kGrain = 64;
     const int want_chunks = std::max<int>(1, int((600 + n * M - 1) / (n * M)));
-    L.nchunk = std::min<int>(want_chunks, int(Pp / kGrain));
-    L.chunk = int((Pp / kGrain + L.nchunk - 1) / L.nchunk * kGrain);
-    if (tu.a_chunk > 0) L.chunk = int(std::min<size_t>(Pp, size_t(std::max(2 * TP, tu.a_chunk / TP * TP))));
+    L.nchunk = std::min<int>(want_chunks, int(Pp / kChunkGrain));
+    L.chunk = int((Pp / kChunkGrain + L.nchunk - 1) / L.nchunk * kChunkGrain);
+    if (tu.a_chunk > 0) L.chunk = int(std::min<size_t>(Pp, std::max(kChunkGrain, tu.a_chunk / kChunkGrain * kChunkGrain)));
     L.nchunk = int((Pp + L.chunk - 1) / L.chunk);
     L.apart = n * M * size_t(L.nchunk) * SP2;
     L.afull = n * M * SP2;
@@ -1496,8 +1498,8 @@ extern "C" h3g_status h3g_model_get_eigensystem(h3g_problem* pr, int k, double* 
 
 extern "C" h3g_status h3g_problem_set_tuning(h3g_problem* pr, const h3g_tuning* tu) {
     if (!pr || !tu) return H3G_ERR_ARG;
-    if (tu->a_chunk < 0 || (tu->a_chunk > 0 && (tu->a_chunk % TP != 0 || tu->a_chunk < 2 * TP)))
-        return fail(pr->ctx, H3G_ERR_ARG, "a_chunk must be 0 or a multiple of 128 that is at least 256");
+    if (tu->a_chunk < 0 || tu->a_chunk % kChunkGrain != 0)
+        return fail(pr->ctx, H3G_ERR_ARG, "a_chunk must be 0 or a multiple of 64");
     if (tu->ctas_per_sm < 0 || tu->ctas_per_sm > 2) return fail(pr->ctx, H3G_ERR_ARG, "ctas_per_sm must be 0, 1 or 2");
     if (tu->frechet_groups < 0) return fail(pr->ctx, H3G_ERR_ARG, "frechet_groups must be >= 0");
     pr->tuning = *tu;
@@ -1506,16 +1508,19 @@ extern "C" h3g_status h3g_problem_set_tuning(h3g_problem* pr, const h3g_tuning* 
     return H3G_OK;
 }
 
-// A chunk as a tuning can ask for it (the heuristic also takes smaller ones, for the smallest problems).
-static int tunable_chunk(int chunk) { return std::max(2 * TP, (chunk + TP - 1) / TP * TP); }
-
+// What runs: the workspace's shapes (sized for the largest model installed so far), or what a workspace would get.
 extern "C" h3g_status h3g_problem_get_tuning(const h3g_problem* pr, h3g_tuning* tu) {
     if (!pr || !tu) return H3G_ERR_ARG;
-    const WsLayout L = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), std::max(pr->M, 1), pr->K,
-                                 std::max(pr->nmod, 1), pr->ndirs, effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
-    tu->a_chunk = tunable_chunk(L.chunk);
+    if (pr->has_model && pr->w.P) {
+        tu->a_chunk = pr->w.chunk;
+        tu->frechet_groups = pr->w.ngroups;
+    } else {
+        const WsLayout L = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), std::max(pr->M, 1), pr->K,
+                                     std::max(pr->nmod, 1), pr->ndirs, effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
+        tu->a_chunk = L.chunk;
+        tu->frechet_groups = L.ngroups;
+    }
     tu->ctas_per_sm = pr->wait.ctas_per_sm;
-    tu->frechet_groups = L.ngroups;
     return H3G_OK;
 }
 
@@ -1547,15 +1552,14 @@ extern "C" h3g_status h3g_autotune(h3g_problem* pr, const double* bl, unsigned w
         return H3G_OK;
     };
     const WsLayout L0 = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs, h3g_tuning{});
-    const h3g_tuning heuristic{tunable_chunk(L0.chunk), 2, L0.ngroups};
-    h3g_tuning cur = heuristic;
-    double cur_ms = 0.0, untuned_ms = 0.0;
-    if (h3g_status st = measure(h3g_tuning{}, &untuned_ms); st != H3G_OK) return st;
+    // the heuristics' shapes, spelled out: zero fields would stand for the recorded tuning
+    h3g_tuning cur{L0.chunk, 2, L0.ngroups};
+    double cur_ms = 0.0;
     if (h3g_status st = measure(cur, &cur_ms); st != H3G_OK) return st;
     auto uniq = [](std::vector<int> v) { std::sort(v.begin(), v.end()); v.erase(std::unique(v.begin(), v.end()), v.end()); return v; };
     const int Pp = pr->Pp;
-    auto chunk_of = [&](int c) { return std::max(2 * TP, std::min(Pp, c / TP * TP)); };
-    std::vector<int> chunks = uniq({chunk_of(L0.chunk), chunk_of(Pp), chunk_of(Pp / 2), chunk_of(Pp / 4), chunk_of(Pp / 8),
+    auto chunk_of = [&](int c) { return std::min(Pp, std::max(2 * TP, c / TP * TP)); };
+    std::vector<int> chunks = uniq({L0.chunk, chunk_of(Pp), chunk_of(Pp / 2), chunk_of(Pp / 4), chunk_of(Pp / 8),
                                     chunk_of(1024), chunk_of(512), chunk_of(256)});
     std::vector<int> groups = uniq({L0.ngroups, std::max(1, L0.ngroups / 2), std::min(pr->n, 2 * L0.ngroups),
                                     std::min(pr->n, 4 * L0.ngroups)});
@@ -1572,20 +1576,11 @@ extern "C" h3g_status h3g_autotune(h3g_problem* pr, const double* bl, unsigned w
             if (ms < cur_ms) { cur = tu; cur_ms = ms; }
         }
     }
-    // nothing better than the heuristic's own chunk, below the smallest a tuning can ask for: stay with it
-    const bool keep = L0.chunk < heuristic.a_chunk && untuned_ms <= cur_ms;
-    if (keep) {
-        cur = heuristic;
-        cur_ms = untuned_ms;
-    }
-    const h3g_tuning install = keep ? h3g_tuning{} : cur;
+    if (h3g_status st = h3g_problem_set_tuning(pr, &cur); st != H3G_OK) return st;
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        const auto key = tune_key(pr, pr->M, pr->K, pr->nmod, pr->ndirs);
-        if (keep) g_tunings.erase(key);
-        else g_tunings[key] = cur;
+        g_tunings[tune_key(pr, pr->M, pr->K, pr->nmod, pr->ndirs)] = cur;
     }
-    if (h3g_status st = h3g_problem_set_tuning(pr, &install); st != H3G_OK) return st;
     if (best) *best = cur;
     if (best_ms) *best_ms = cur_ms;
     return H3G_OK;

@@ -222,7 +222,7 @@ h3g_status h3g_model_get_eigensystem(h3g_problem* prob, int k, double* lam, doub
  * device): later problems of that shape start from it.  Results are
  * deterministic for a given tuning; tunings differ only in summation order. */
 typedef struct {
-    int a_chunk;          /* patterns per A-accumulation chunk: a multiple of 128, >= 256 */
+    int a_chunk;          /* patterns per A-accumulation chunk: a multiple of 64 */
     int ctas_per_sm;      /* mixed persistent passes: 1 or 2 resident CTAs per SM */
     int frechet_groups;   /* branch groups of the Frechet kernel: >= 1 */
 } h3g_tuning;
