@@ -619,11 +619,15 @@ static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, 
     L.pcols = size_t(M) * Pp;
     L.ecols = part_nodes * M * Pp;
     L.gt = size_t(M) * n;
-    // enough A chunks for ~600 CTAs, never below 64 patterns per chunk (two stages: a chunk of 256 left the smallest
-    // genes with 8 stages in a row on a handful of CTAs)
+    // enough A chunks for ~600 CTAs, never below kGrain patterns per chunk.  FP64: 64 (two stages: a chunk of 256 left the
+    // smallest genes with 8 stages in a row on a handful of CTAs; 8 taxa x 1000 codons 114 us an evaluation, with 64
+    // patterns 100).  Mixed: 256, two 64-pattern tiles for each half of an accumulation CTA, which has its SM to itself:
+    // 64 patterns leave one half without a tile (8 taxa x 2000 codons 154 us an evaluation, with 256 patterns 117;
+    // 16 x 1000 154 and 129, 32 x 600 208 and 178, 256 x 300 403 and 381).
+    const int kGrain = precision == H3G_PREC_MIXED ? 256 : kChunkGrain, unit = std::min(kGrain, TP);
     const int want_chunks = std::max<int>(1, int((600 + n * M - 1) / (n * M)));
-    L.nchunk = std::min<int>(want_chunks, int(Pp / kChunkGrain));
-    L.chunk = int((Pp / kChunkGrain + L.nchunk - 1) / L.nchunk * kChunkGrain);
+    L.nchunk = std::min<int>(want_chunks, std::max<int>(1, int(Pp / kGrain)));
+    L.chunk = int((Pp / unit + L.nchunk - 1) / L.nchunk * unit);
     if (tu.a_chunk > 0) L.chunk = int(std::min<size_t>(Pp, std::max(kChunkGrain, tu.a_chunk / kChunkGrain * kChunkGrain)));
     L.nchunk = int((Pp + L.chunk - 1) / L.chunk);
     L.apart = n * M * size_t(L.nchunk) * SP2;

@@ -69,3 +69,18 @@ def test_chunks_that_a_tuning_can_ask_for(oracle):
             pr.set_tuning(a_chunk=chunk)
     pr.close()
     ctx.close()
+
+
+@pytest.mark.parametrize("sites,least", [(90, 128), (300, 256), (700, 256), (1500, 256)])
+def test_mixed_chunks_keep_both_halves_of_a_cta_busy(oracle, sites, least):
+    # four 64-pattern tiles in a chunk, or all there are
+    from hyphy3 import _capi
+    tree = oracle.Tree.parse(SHAPES["cherries"])
+    aln = _alignment(oracle, tree, sites, np.random.default_rng(sites))
+    e = oracle.mg94(aln, PAR)
+    ctx = _capi.Context(0)
+    pr = problem_from_oracle(ctx, oracle, tree, aln)
+    pr.set_model(pi=aln.pi, Q=e["Q"], lam=e["lam"], U=e["U"], V=e["V"], precision=_capi.PREC_MIXED)
+    assert pr.get_tuning()["a_chunk"] >= least
+    pr.close()
+    ctx.close()
