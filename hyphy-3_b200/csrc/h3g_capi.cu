@@ -606,9 +606,9 @@ struct WsLayout {
 constexpr int kChunkGrain = 64;
 
 // part_nodes / vf_nodes: partial slots of internal nodes and gradient-operand slots (NI and n, or
-// fewer under a checkpoint plan).
+// fewer under a checkpoint plan).  coarse: A chunks of 256 patterns and more also for FP64.
 static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, int K, int nmod, int ndirs, const h3g_tuning& tu,
-                          size_t part_nodes = 0, size_t vf_nodes = 0) {
+                          size_t part_nodes = 0, size_t vf_nodes = 0, bool coarse = false) {
     (void)K;
     if (!part_nodes) part_nodes = NI;
     if (!vf_nodes) vf_nodes = n;
@@ -624,7 +624,7 @@ static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, 
     // patterns 100).  Mixed: 256, two 64-pattern tiles for each half of an accumulation CTA, which has its SM to itself:
     // 64 patterns leave one half without a tile (8 taxa x 2000 codons 154 us an evaluation, with 256 patterns 117;
     // 16 x 1000 154 and 129, 32 x 600 208 and 178, 256 x 300 403 and 381).
-    const int kGrain = precision == H3G_PREC_MIXED ? 256 : kChunkGrain, unit = std::min(kGrain, TP);
+    const int kGrain = precision == H3G_PREC_MIXED || coarse ? 256 : kChunkGrain, unit = std::min(kGrain, TP);
     const int want_chunks = std::max<int>(1, int((600 + n * M - 1) / (n * M)));
     L.nchunk = std::min<int>(want_chunks, std::max<int>(1, int(Pp / kGrain)));
     L.chunk = int((Pp / unit + L.nchunk - 1) / L.nchunk * unit);
@@ -865,9 +865,10 @@ static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndi
     auto make = [&](int target) {
         return h3g::plan_checkpoints(pr->n, pr->root, kids, pr->leaf.data(), pr->bfs_order, pr->depth_h, pr->height_h, target);
     };
+    bool coarse = false;
     auto layout_of = [&](const h3g::CkPlan& p) {
         return ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu, size_t(p.ncp + p.scratch_int),
-                         size_t(p.ncp + p.scratch_all));
+                         size_t(p.ncp + p.scratch_all), coarse);
     };
     if (pr->ck_target_req > 0) {
         pr->ck_plan = make(pr->ck_target_req);
@@ -875,17 +876,23 @@ static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndi
         pr->ck = true;
         return H3G_OK;
     }
-    for (int target = pr->n;; target = std::max(2, target * 4 / 5)) {
-        h3g::CkPlan p = make(target);
-        const WsLayout Lc = layout_of(p);
-        if (ws_bytes(Lc, pr->precision) <= budget) {
-            pr->ck_plan = std::move(p);
-            L = Lc;
-            pr->ck = true;
-            return H3G_OK;
+    auto fitting = [&] {
+        for (int target = pr->n;; target = std::max(2, target * 4 / 5)) {
+            h3g::CkPlan p = make(target);
+            L = layout_of(p);
+            if (ws_bytes(L, pr->precision) <= budget) {
+                pr->ck_plan = std::move(p);
+                pr->ck = true;
+                return true;
+            }
+            if (target == 2) return false;
         }
-        if (target == 2) break;
-    }
+    };
+    if (fitting()) return H3G_OK;
+    // A small problem's fine A chunks are partial sums for every branch, whatever the plan (15 nodes x 300 codons: 2.9 MB,
+    // in one chunk 0.5 MB): the last resort gives up their order of summation for the room.
+    coarse = true;
+    if (fitting()) return H3G_OK;
     return fail(pr->ctx, H3G_ERR_OOM, "the evaluation workspace does not fit the memory budget even with subtree checkpoints");
 }
 

@@ -263,7 +263,9 @@ h3g_status h3g_problem_set_wait_limit(h3g_problem* prob, uint32_t polls, int unm
  * inside pass keeps only the checkpoint nodes' partials, and the outside pass
  * recomputes each block's inside partials from its checkpointed children before
  * walking it.  Results are bit-identical to the unbudgeted evaluation (same
- * kernels, same summation order).  Budget 0 = none, but a workspace larger than
+ * kernels, same summation order), but for a budget that only holds an FP64
+ * problem with larger A-accumulation chunks than its own: its gradients are
+ * then the same to rounding.  Budget 0 = none, but a workspace larger than
  * the device's free memory checkpoints by itself.  target > 0 forces that block
  * size (0 = the largest that fits the budget).  FP64 and mixed precision; not for
  * batch members (their workspaces are the batch's slots). */
