@@ -27,13 +27,13 @@ struct h3g_ctx {
     int live_problems = 0;
     std::string err;
     void* compress = nullptr;      // alignment-compression scratch (h3g_compress.cu), kept between calls
-    // Pinned memory that h3g_model_set passes a model through, for every problem of the context (kept between calls up
-    // to kStageKeep): whoever fills it holds the mutex until the device has read it.
+    // Pinned memory that h3g_model_set passes a model through, for every problem of the context (kept between calls,
+    // kStageMost at most): whoever fills it holds the mutex until the device has read it.
     std::mutex stage_mu;
     double* stage = nullptr;
     size_t stage_count = 0;
 };
-constexpr size_t kStageKeep = size_t(8) << 20;     // doubles (64 MB)
+constexpr size_t kStageLeast = size_t(1) << 14, kStageMost = size_t(2) << 20;     // doubles (16 MB at most)
 
 namespace h3g {
 void compress_scratch_free(void* p);     // h3g_compress.cu
@@ -956,32 +956,101 @@ static uint64_t hash_bytes(uint64_t h, const void* p, size_t n) {
 }
 
 namespace {
-// The context's staging memory, grown to `count` doubles and held; the destructor waits for the device's reads.
-struct StageHold {
+// A model's arrays on their way to the device: copied as they are into the context's staging memory, from which a kernel
+// lays them out (padded, transposed; k_model_install).  A model larger than that memory goes in pieces, each when the
+// device has read the one before: installs of hundreds of MB (a model for every branch and class, with directions) would
+// otherwise pin and release that much each time, and fail where it is refused.  510 models of 61 states with 6 directions
+// each, 107 MB: 29 ms, with one block for all of it 90 to 105 (the copies from pageable memory before that: 120).
+struct ModelStager {
     h3g_ctx* ctx;
-    cudaStream_t other;
+    cudaStream_t s[2];                 // the context's stream and the problem's side stream
+    int S;
     std::unique_lock<std::mutex> lk;
-    StageHold(h3g_ctx* c, cudaStream_t s2) : ctx(c), other(s2), lk(c->stage_mu) {}
-    cudaError_t grow(size_t count) {
-        if (count <= ctx->stage_count) return cudaSuccess;
+    cudaError_t err = cudaSuccess;     // the first one
+    int on = 0;                        // the stream that takes what is staged now
+    bool reads[2] = {false, false};    // the streams that read the staging memory's present contents
+    size_t at = 0;
+    ModelInstall in{};
+
+    ModelStager(h3g_ctx* c, cudaStream_t side, int S_, size_t total) : ctx(c), s{c->stream, side}, S(S_), lk(c->stage_mu) {
+        in.S = S;
+        size_t count = std::min(std::max(total, kStageLeast), kStageMost);
+        if (count <= ctx->stage_count) return;
         if (ctx->stage) cudaFreeHost(ctx->stage);
         ctx->stage = nullptr;
         ctx->stage_count = 0;
-        count = std::max(count, size_t(1) << 14);
-        const cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&ctx->stage), count * sizeof(double));
-        if (e == cudaSuccess) ctx->stage_count = count;
-        return e;
-    }
-    cudaError_t wait() {
-        const cudaError_t a = cudaStreamSynchronize(ctx->stream), b = cudaStreamSynchronize(other);
-        return a != cudaSuccess ? a : b;
-    }
-    ~StageHold() {
-        wait();
-        if (ctx->stage_count > kStageKeep) {
-            cudaFreeHost(ctx->stage);
+        for (;; count = std::max(count / 2, kStageLeast)) {
+            const cudaError_t e = cudaMallocHost(reinterpret_cast<void**>(&ctx->stage), count * sizeof(double));
+            if (e == cudaSuccess) { ctx->stage_count = count; return; }
+            cudaGetLastError();
             ctx->stage = nullptr;
-            ctx->stage_count = 0;
+            if (count == kStageLeast) { err = e; return; }
+        }
+    }
+    ~ModelStager() { wait(); }
+    void note(cudaError_t e) { if (err == cudaSuccess) err = e; }
+    // the device has read everything that was staged
+    void wait() {
+        for (int q = 0; q < 2; ++q)
+            if (reads[q]) { note(cudaStreamSynchronize(s[q])); reads[q] = false; }
+        at = 0;
+    }
+    // ... and what was launched behind it is done (a batch's slots run on streams of their own)
+    cudaError_t finish() {
+        reads[0] = reads[1] = true;
+        wait();
+        return err;
+    }
+    void flush() {
+        if (in.n_mat || in.n_vec) {
+            launch_model_install(in, s[on]);
+            note(cudaGetLastError());
+            reads[on] = true;
+        }
+        in = ModelInstall{};
+        in.S = S;
+    }
+    void side_stream() { flush(); on = 1; }
+    // `words` doubles' worth of staging memory at most, at least one unit of `unit`
+    size_t room(size_t words, size_t unit) {
+        if (ctx->stage_count - at < unit) { flush(); wait(); }
+        return std::min(words, (ctx->stage_count - at) / unit * unit);
+    }
+    double* put(const void* src, size_t bytes) {
+        double* to = ctx->stage + at;
+        std::memcpy(to, src, bytes);
+        at += (bytes + 7) / 8;
+        return to;
+    }
+    void add_vec(const double* from, void* dst, int rows, int width, int pad) {
+        if (in.n_vec == int(sizeof(in.vec) / sizeof(in.vec[0]))) flush();
+        in.vec[in.n_vec++] = {from, static_cast<double*>(dst), rows, width, pad};
+    }
+    // bytes as they are, in whole 8-byte words
+    void flat(const void* src, size_t bytes, void* dst) {
+        for (size_t done = 0; err == cudaSuccess && done < bytes;) {
+            const size_t words = room((bytes - done + 7) / 8, 1), take = std::min(words * 8, bytes - done);
+            add_vec(put(static_cast<const char*>(src) + done, take), static_cast<char*>(dst) + done, 1, int(words), int(words));
+            done += take;
+        }
+    }
+    // [rows][S] to [rows][64]
+    void rows(const double* src, size_t n_rows, double* dst) {
+        for (size_t done = 0; err == cudaSuccess && done < n_rows;) {
+            const size_t take = room((n_rows - done) * S, size_t(S)) / S;
+            add_vec(put(src + done * S, take * S * sizeof(double)), dst + done * SP, int(take), S, SP);
+            done += take;
+        }
+    }
+    // [count][S][S] to [count][64][64], and transposed to dst_t if given
+    void mats(const double* src, size_t count, double* dst, double* dst_t) {
+        const size_t SS = size_t(S) * S;
+        for (size_t done = 0; err == cudaSuccess && done < count;) {
+            const size_t take = room((count - done) * SS, SS) / SS;
+            if (in.n_mat == int(sizeof(in.mat) / sizeof(in.mat[0]))) flush();
+            in.mat[in.n_mat++] = {put(src + done * SS, take * SS * sizeof(double)), dst + done * SP2,
+                                  dst_t ? dst_t + done * SP2 : nullptr, int(take)};
+            done += take;
         }
     }
 };
@@ -1092,59 +1161,38 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
             H3G_TRY_CUDA(ctx, A.alloc(&pr->m_br, (size_t(pr->n) + 2) / 2 * 2));
             std::copy(mkey, mkey + 5, pr->model_key);
         }
-        // The caller's arrays go through pinned memory as they are and a kernel lays them out (padded, transposed):
-        // generators first, so that they are diagonalised while the host still stages the directions.
+        // generators first, so that they are diagonalised while the host still stages the directions
         cudaStream_t s = ctx->stream;
         const size_t SS = size_t(S) * S, n_dq = size_t(d->n_dirs) * nm + size_t(n_model_dirs);
-        const size_t br_words = d->branch_classes ? (size_t(pr->n) + 2) / 2 : 0, it_words = d->is_test ? (size_t(pr->n) + 7) / 8 : 0;
-        StageHold hold(ctx, pr->s2);
-        H3G_TRY_CUDA(ctx, hold.grow(size_t(S) + 3 * nm * SS + size_t(nm) * (S + 2) + d->K + 2 * d->M + br_words + it_words + n_dq * SS));
-        double* st_at = ctx->stage;
-        auto stage = [&](const void* src, size_t bytes) {
-            double* at = st_at;
-            std::memcpy(at, src, bytes);
-            st_at += (bytes + 7) / 8;
-            return at;
-        };
-        auto vec = [&](ModelInstall& in, const void* src, size_t bytes, void* dst, int rows, int pad) {
-            const int words = int((bytes + 7) / 8);
-            in.vec[in.n_vec++] = {stage(src, bytes), static_cast<double*>(dst), rows, words / rows, pad ? pad : words / rows};
-        };
-        auto mats = [&](ModelInstall& in, const double* src, int count, double* dst, double* dst_t) {
-            in.mat[in.n_mat++] = {stage(src, size_t(count) * SS * sizeof(double)), dst, dst_t, count};
-        };
-        ModelInstall in{};
-        in.S = S;
-        vec(in, d->pi, S * sizeof(double), pr->m_pi, 1, SP);
-        mats(in, d->Q, nm, pr->m_Q, pr->m_QT);
+        const size_t n_words = d->branch_classes || d->is_test ? (size_t(pr->n) + 2) / 2 : 0;
+        ModelStager st(ctx, pr->s2, S, size_t(S) + (dev_eig ? 1 : 3) * nm * SS + size_t(nm) * (S + 2) + d->K + 2 * d->M + n_words + n_dq * SS);
+        st.rows(d->pi, 1, pr->m_pi);
+        st.mats(d->Q, size_t(nm), pr->m_Q, pr->m_QT);
         if (!dev_eig) {
-            vec(in, d->lam, size_t(nm) * S * sizeof(double), pr->m_lam, nm, SP);
-            mats(in, d->U, nm, pr->m_U, pr->m_UT);
-            mats(in, d->V, nm, pr->m_V, nullptr);
+            st.rows(d->lam, size_t(nm), pr->m_lam);
+            st.mats(d->U, size_t(nm), pr->m_U, pr->m_UT);
+            st.mats(d->V, size_t(nm), pr->m_V, nullptr);
         }
-        vec(in, mu.data(), mu.size() * sizeof(double), pr->m_mu, 1, 0);
-        vec(in, d->class_w, d->K * sizeof(double), pr->m_cw, 1, 0);
+        st.flat(mu.data(), mu.size() * sizeof(double), pr->m_mu);
+        st.flat(d->class_w, d->K * sizeof(double), pr->m_cw);
         if (d->has_bg > 0) {
             pr->h_bw.assign(size_t(d->has_bg), 1.0);
             if (d->bg_w) std::copy(d->bg_w, d->bg_w + d->has_bg, pr->h_bw.begin());
-            vec(in, pr->h_bw.data(), pr->h_bw.size() * sizeof(double), pr->m_bw, 1, 0);
+            st.flat(pr->h_bw.data(), pr->h_bw.size() * sizeof(double), pr->m_bw);
         }
-        vec(in, d->rates, d->M * sizeof(double), pr->m_rt, 1, 0);
-        vec(in, d->rate_w, d->M * sizeof(double), pr->m_rw, 1, 0);
-        if (d->is_test) vec(in, d->is_test, size_t(pr->n), pr->m_it, 1, 0);
-        if (d->branch_classes) vec(in, d->branch_classes, size_t(pr->n + 1) * sizeof(int32_t), pr->m_br, 1, 0);
-        launch_model_install(in, s);
+        st.flat(d->rates, d->M * sizeof(double), pr->m_rt);
+        st.flat(d->rate_w, d->M * sizeof(double), pr->m_rw);
+        if (d->is_test) st.flat(d->is_test, size_t(pr->n), pr->m_it);
+        if (d->branch_classes) st.flat(d->branch_classes, size_t(pr->n + 1) * sizeof(int32_t), pr->m_br);
+        st.side_stream();
+        H3G_TRY_CUDA(ctx, st.err);
         if (dev_eig) launch_model_eig(pr->m_Q, pr->m_pi, S, nm, pr->m_lam, pr->m_U, pr->m_UT, pr->m_V, d->precision == H3G_PREC_MIXED, s);
         H3G_TRY_CUDA(ctx, cudaGetLastError());
-        if (n_dq > 0) {
-            // dense directions [n_dirs][nm], then the per-model ones [nm]
-            ModelInstall dq{};
-            dq.S = S;
-            if (d->n_dirs > 0) mats(dq, d->dQ, d->n_dirs * nm, pr->m_dQ, nullptr);
-            if (n_model_dirs > 0) mats(dq, d->dQ_model, n_model_dirs, pr->m_dQ + size_t(d->n_dirs) * nm * SP2, nullptr);
-            launch_model_install(dq, pr->s2);
-            H3G_TRY_CUDA(ctx, cudaGetLastError());
-        }
+        // dense directions [n_dirs][nm], then the per-model ones [nm]
+        if (d->n_dirs > 0) st.mats(d->dQ, size_t(d->n_dirs) * nm, pr->m_dQ, nullptr);
+        if (n_model_dirs > 0) st.mats(d->dQ_model, size_t(n_model_dirs), pr->m_dQ + size_t(d->n_dirs) * nm * SP2, nullptr);
+        st.flush();
+        H3G_TRY_CUDA(ctx, st.err);
         Model md{};
         md.M = d->M; md.K = d->K; md.has_bg = d->has_bg; md.nmod = nm; md.time_mode = d->time_mode; md.ndirs = n_dirs_all;
         md.ndirs_dense = d->n_dirs;
@@ -1156,9 +1204,8 @@ extern "C" h3g_status h3g_model_set(h3g_problem* pr, const h3g_model_desc* d) {
         md.dQ = pr->m_dQ;
         if (std::memcmp(&md, &pr->md, sizeof(Model)) != 0) pr->drop_graphs();
         pr->md = md;
-        h3g_status st = ensure_workspace(pr, d->M, d->K, nm, n_dirs_all);
-        if (st != H3G_OK) return st;
-        H3G_TRY_CUDA(ctx, hold.wait());
+        if (h3g_status ws = ensure_workspace(pr, d->M, d->K, nm, n_dirs_all); ws != H3G_OK) return ws;
+        H3G_TRY_CUDA(ctx, st.finish());
         pr->model_hash = h;
         pr->has_model = true;
         return H3G_OK;
