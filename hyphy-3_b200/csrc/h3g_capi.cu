@@ -527,6 +527,11 @@ void fel_set_error(h3g_problem* pr, const std::string& msg) {
 FelDevice*& problem_fel_device(h3g_problem* pr) { return pr->fel_dev; }
 void*& problem_nuc_state(h3g_problem* pr) { return pr->nuc; }
 int problem_max_state(h3g_problem* pr) { return pr->max_state; }
+// internal nodes by increasing height, and where each height starts
+void problem_levels(h3g_problem* pr, const std::vector<int>** nodes, const std::vector<int>** off) {
+    *nodes = &pr->in_nodes;
+    *off = &pr->in_off;
+}
 
 void fel_record_transfer(h3g_problem* pr, size_t h2d, size_t d2h, int launches, double ms) {
     pr->last_h2d = h2d;

@@ -12,10 +12,10 @@
 // log-likelihood log L - E ln 2, or the reference's -1e20 when L <= 0; the weighted sum
 // over patterns is a fixed-order Neumaier sum.  FP64 throughout.
 //
-// With fewer patterns than it takes to fill the GPU (kLevelBelow), a CTA of 16 warps
-// walks the tree for 32 patterns level by level instead (h3g_few.cuh), a warp per
-// internal node of the level, partials stored per internal node.  A call for 256 taxa
-// x 3000 patterns (41 levels) takes 545 us, with a launch per level 684 us.
+// With fewer patterns than it takes to fill the GPU (kLevelBelow), the tree is walked
+// level by level instead, partials stored per internal node: by one launch, in which a
+// CTA of 16 warps takes 32 patterns through all levels (h3g_few.cuh), a warp per internal
+// node of the level, or by a launch per level, a thread per node and pattern (walk_wins).
 #include <algorithm>
 #include <cmath>
 #include <new>
@@ -32,10 +32,16 @@ Topo problem_topo(h3g_problem* pr, int S);                // h3g_capi.cu
 cudaStream_t problem_stream(h3g_problem* pr);
 void*& problem_nuc_state(h3g_problem* pr);
 int problem_max_state(h3g_problem* pr);
+void problem_levels(h3g_problem* pr, const std::vector<int>** nodes, const std::vector<int>** off);
 
 namespace {
 
 constexpr int kNucT = 128;                                 // threads per block (patterns)
+constexpr int kLvlT = 256;
+// Nodes x patterns of a level below which a thread loads two children side by side: at its 96 registers two CTAs fit an SM, so
+// that is one wave.  Above, one at a time and twice the CTAs: 256 taxa at random x 131000 patterns 824 us, in pairs 1239; below,
+// a chain of 256 taxa x 16000 758 us, one at a time 1344.
+constexpr size_t kPairBelow = size_t(148) * 2 * kLvlT;
 constexpr int kSumT = 1024;
 constexpr int kLevelBelow = 131072;                        // patterns: below, the level-by-level walk
 
@@ -48,7 +54,8 @@ struct NucState {
     double* d_site = nullptr;                              // [P]
     double4* d_stk = nullptr;                              // [depth][Pp]
     int* d_exp = nullptr;                                  // [depth][Pp]
-    bool levels = false;                                   // level-by-level walk
+    bool levels = false;                                   // level by level ...
+    bool walk = false;                                     // ... in one launch
     double4* d_part = nullptr;                             // [NI][Pp]
     int* d_pexp = nullptr;                                 // [NI][Pp]
     double* d_lnl = nullptr;
@@ -130,72 +137,97 @@ __global__ void __launch_bounds__(kNucT) k_nuc_lnl(Topo t, const int* __restrict
     site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
 }
 
-// The product of the children's messages at every internal node, level by level; grid Pp / 32.
+// A child at pattern p (c: Topo::kdesc entry, st: its observed state if a leaf): its matrix, partial and exponent.
+struct NucChild { double2 P[8]; double x[4]; int E; };
+__device__ __forceinline__ NucChild nuc_child(const Topo& t, const double* __restrict__ P, const double4* part, const int* pexp, int2 c,
+                                              int st, int p) {
+    NucChild o;
+    const double2* Pn = reinterpret_cast<const double2*>(P + size_t(c.x) * 16);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o.P[i] = __ldg(Pn + i);
+    o.E = 0;
+    if (c.y <= -2) {
+        const size_t at = size_t(-(c.y + 2)) * size_t(t.Pp) + p;
+        const double4 v = part[at];
+        o.x[0] = v.x; o.x[1] = v.y; o.x[2] = v.z; o.x[3] = v.w;
+        o.E = pexp[at];
+    } else {                                               // likelihood.hpp:54-87
+        const uint64_t mk = st >= 0 ? uint64_t(1) << st : (c.y < 0 ? 0xF : t.masks[size_t(c.y) * size_t(t.Pp) + p]);
+        const bool any = st < 0 && (mk == 0 || (mk & 0xF) == 0xF);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o.x[i] = any || ((mk >> i) & 1) ? 1.0 : 0.0;
+    }
+    return o;
+}
+__device__ __forceinline__ void nuc_take(double (&d)[4], int& E, const NucChild& c) {
+    double mx = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const double2 a01 = c.P[2 * i], a23 = c.P[2 * i + 1];
+        d[i] *= a01.x * c.x[0] + a01.y * c.x[1] + a23.x * c.x[2] + a23.y * c.x[3];
+        mx = fmax(mx, d[i]);
+    }
+    E += c.E;
+    if (mx > 0.0 && mx < 0x1p-256) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[i] *= 0x1p256;
+        E += 256;
+    }
+}
+// One internal node at one pattern: the product of its children's messages.  a, d4: its two few_in descriptors; s0, s1: the
+// observed states of its first two children.
+template <bool kPair>
+__device__ __forceinline__ void nuc_node(const Topo& t, const double* __restrict__ P, const double* __restrict__ pi, double4* part,
+                                         int* pexp, double* __restrict__ site, int4 a, int4 d4, int s0, int s1, int p) {
+    const int k0 = a.z, k1 = a.w;
+    double d[4] = {1.0, 1.0, 1.0, 1.0};
+    int E = 0;
+    if (kPair && k0 + 1 < k1) {                            // two side by side: one trip to memory
+        const NucChild c0 = nuc_child(t, P, part, pexp, make_int2(d4.x, d4.y), s0, p);
+        const NucChild c1 = nuc_child(t, P, part, pexp, make_int2(d4.z, d4.w), s1, p);
+        nuc_take(d, E, c0);
+        nuc_take(d, E, c1);
+    } else if (k0 < k1) {
+        nuc_take(d, E, nuc_child(t, P, part, pexp, make_int2(d4.x, d4.y), s0, p));
+    }
+    if (!kPair && k0 + 1 < k1) nuc_take(d, E, nuc_child(t, P, part, pexp, make_int2(d4.z, d4.w), s1, p));
+    for (int k = k0 + 2; k < k1; ++k) {
+        const int2 c = t.kdesc[k];
+        nuc_take(d, E, nuc_child(t, P, part, pexp, c, few_state(t, c, p), p));
+    }
+    if (a.x == t.root) {
+        if (p >= t.P) return;
+        const double L = pi[0] * d[0] + pi[1] * d[1] + pi[2] * d[2] + pi[3] * d[3];
+        site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
+    } else {
+        const size_t o = size_t(a.y) * size_t(t.Pp) + p;
+        part[o] = make_double4(d[0], d[1], d[2], d[3]);
+        pexp[o] = E;
+    }
+}
+
+// The whole tree, level by level; grid ceil(P / 32).
 __global__ void __launch_bounds__(32 * kFewWarps) k_nuc_walk(Topo t, const double* __restrict__ P, const double* __restrict__ pi,
                                                              double4* part, int* pexp, double* __restrict__ site) {
     const int lane = threadIdx.x & 31, p = 32 * int(blockIdx.x) + lane;
-    const size_t Pp = size_t(t.Pp);
     few_walk(
         t.few_in_lv, t.few_in_levels, t.few_in, threadIdx.x >> 5,
         [&](int4 d, int& s0, int& s1) { s0 = few_state(t, make_int2(d.x, d.y), p); s1 = few_state(t, make_int2(d.z, d.w), p); },
         [] { pdl_enter(); },
-        [&](int4 a, int4 d4, int s0, int s1) {
-            const int u = a.x, k0 = a.z, k1 = a.w;
-            double d[4] = {1.0, 1.0, 1.0, 1.0};
-            int E = 0;
-            struct Child { double2 P[8]; double x[4]; int E; };
-            auto load = [&](int2 c, int st) {
-                Child o;
-                const double2* Pn = reinterpret_cast<const double2*>(P + size_t(c.x) * 16);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o.P[i] = __ldg(Pn + i);
-                o.E = 0;
-                if (c.y <= -2) {
-                    const size_t at = size_t(-(c.y + 2)) * Pp + p;
-                    const double4 v = part[at];
-                    o.x[0] = v.x; o.x[1] = v.y; o.x[2] = v.z; o.x[3] = v.w;
-                    o.E = pexp[at];
-                } else {                                   // likelihood.hpp:54-87
-                    const uint64_t mk = st >= 0 ? uint64_t(1) << st : (c.y < 0 ? 0xF : t.masks[size_t(c.y) * Pp + p]);
-                    const bool any = st < 0 && (mk == 0 || (mk & 0xF) == 0xF);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) o.x[i] = any || ((mk >> i) & 1) ? 1.0 : 0.0;
-                }
-                return o;
-            };
-            auto take = [&](const Child& c) {
-                double mx = 0.0;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const double2 a01 = c.P[2 * i], a23 = c.P[2 * i + 1];
-                    d[i] *= a01.x * c.x[0] + a01.y * c.x[1] + a23.x * c.x[2] + a23.y * c.x[3];
-                    mx = fmax(mx, d[i]);
-                }
-                E += c.E;
-                if (mx > 0.0 && mx < 0x1p-256) {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) d[i] *= 0x1p256;
-                    E += 256;
-                }
-            };
-            if (k0 + 1 < k1) {                             // two side by side: one trip to memory
-                const Child c0 = load(make_int2(d4.x, d4.y), s0), c1 = load(make_int2(d4.z, d4.w), s1);
-                take(c0);
-                take(c1);
-            } else if (k0 < k1) {
-                take(load(make_int2(d4.x, d4.y), s0));
-            }
-            for (int k = k0 + 2; k < k1; ++k) take(load(t.kdesc[k], few_state(t, t.kdesc[k], p)));
-            if (u == t.root) {
-                if (p >= t.P) return;
-                const double L = pi[0] * d[0] + pi[1] * d[1] + pi[2] * d[2] + pi[3] * d[3];
-                site[p] = L > 0.0 ? log(L) - double(E) * 0.69314718055994530942 : -1e20;
-            } else {
-                const size_t o = size_t(a.y) * Pp + p;
-                part[o] = make_double4(d[0], d[1], d[2], d[3]);
-                pexp[o] = E;
-            }
-        });
+        [&](int4 a, int4 d, int s0, int s1) { nuc_node<true>(t, P, pi, part, pexp, site, a, d, s0, s1, p); });
+}
+
+// Nodes first .. first + cnt of one level, a thread per (node, pattern).
+template <bool kPair>
+__global__ void __launch_bounds__(kLvlT, kPair ? 1 : 4) k_nuc_level(Topo t, int first, int cnt, const double* __restrict__ P, const double* __restrict__ pi,
+                                                     double4* part, int* pexp, double* __restrict__ site) {
+    const size_t i = size_t(blockIdx.x) * kLvlT + threadIdx.x, P_ = size_t(t.P);
+    if (i >= cnt * P_) return;
+    const int node = first + int(i / P_), p = int(i % P_);
+    const int4 a = t.few_in[2 * node], d = t.few_in[2 * node + 1];
+    const int s0 = few_state(t, make_int2(d.x, d.y), p), s1 = few_state(t, make_int2(d.z, d.w), p);
+    pdl_enter();                                           // the lower levels' partials are complete
+    nuc_node<kPair>(t, P, pi, part, pexp, site, a, d, s0, s1, p);
 }
 
 // One block: weights x site log-likelihoods, Neumaier over every 1024th pattern, then a fixed tree of two-sums (the
@@ -226,6 +258,27 @@ __global__ void __launch_bounds__(kSumT) k_nuc_sum(const double* __restrict__ si
     c = lo[tid];
     warp_sum();
     if (tid == 0) *out = s + c;
+}
+
+// Whether the walk takes less time than a launch per level, by the time of each in microseconds.  The walk's CTAs have an
+// SM to themselves (registers), so beyond 32 patterns an SM they run in waves, each as long as its chain of items: 1.25 a
+// binary node, 0.75 each further child, every 16 nodes of a level one item; 28e-6 a node and pattern at least.  A launch per
+// level costs 25 in all and for each level its launch and one node's chain, 2.9 and 0.65 each further child, or 22e-6
+// a node and pattern if that is more.  Fits whole calls to 20 % where the two are far apart.  Walk / levels in us: a chain of
+// 256 taxa x 16000 patterns 1397 / 759, x 64000 4728 / 871; a star of 100 x 8000 161 / 87, x 64000 764 / 102; 256 taxa at
+// random x 16000 207 / 160, x 64000 610 / 440; 1024 taxa x 8000 306 / 281, x 64000 1795 / 1529.  (The walk is taken for the
+// chain up to x 8000, 686; for the star at x 3000, 88; for the 256 taxa at x 8000, 117.)
+bool walk_wins(const std::vector<int>& nodes, const std::vector<int>& off, const FelProblemView& v, int P, int sms) {
+    const int waves = ((P + 31) / 32 + sms - 1) / sms;
+    double chain = 0.0, levels = 25.0;
+    for (size_t l = 0; l + 1 < off.size(); ++l) {
+        const int width = off[l + 1] - off[l];
+        int more = 0;
+        for (int k = off[l]; k < off[l + 1]; ++k) more = std::max(more, v.ch_off[nodes[size_t(k)] + 1] - v.ch_off[nodes[size_t(k)]] - 2);
+        chain += (width + kFewWarps - 1) / kFewWarps * (1.25 + 0.75 * more);
+        levels += std::max(2.9 + 0.65 * more, 22e-6 * width * P);
+    }
+    return std::max(28e-6 * double(nodes.size()) * P, waves * chain) < levels;
 }
 
 // depth-first events (2 node + 1 opens an internal node, 2 node closes a node) and the
@@ -270,6 +323,11 @@ NucState* nuc_state(h3g_problem* pr, const FelProblemView& v, std::string* err) 
     s->P = t.P;
     s->Pp = size_t(t.Pp);
     s->levels = t.P < kLevelBelow;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, v.device);
+    const std::vector<int>*nodes, *off;
+    problem_levels(pr, &nodes, &off);
+    s->walk = walk_wins(*nodes, *off, v, t.P, sms);
     auto take = [&](auto** p, size_t count) {
         void* q = nullptr;
         if (cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(**p)) != cudaSuccess) return false;
@@ -326,7 +384,17 @@ extern "C" h3g_status h3g_nuc_eval_from_P(h3g_problem* pr, const double* P, cons
     bool ok = cudaMemcpyAsync(s->d_P, P, size_t(v.n) * 16 * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
               cudaMemcpyAsync(s->d_pi, pi, 4 * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess;
     if (ok && s->P > 0) {
-        if (s->levels) {
+        if (s->levels && !s->walk) {
+            const std::vector<int>*nodes, *off;
+            problem_levels(pr, &nodes, &off);
+            for (size_t l = 0; l + 1 < off->size(); ++l) {
+                const int first = (*off)[l], cnt = (*off)[l + 1] - first;
+                if (cnt == 0) continue;
+                const bool pair = size_t(cnt) * size_t(s->P) < kPairBelow;
+                launch_k(pair ? k_nuc_level<true> : k_nuc_level<false>, int((size_t(cnt) * size_t(s->P) + kLvlT - 1) / kLvlT), kLvlT, 0, st, t, first, cnt,
+                         static_cast<const double*>(s->d_P), static_cast<const double*>(s->d_pi), s->d_part, s->d_pexp, s->d_site);
+            }
+        } else if (s->levels) {
             launch_k(k_nuc_walk, (s->P + 31) / 32, 32 * kFewWarps, 0, st, t, static_cast<const double*>(s->d_P),
                      static_cast<const double*>(s->d_pi), s->d_part, s->d_pexp, s->d_site);
         } else {
