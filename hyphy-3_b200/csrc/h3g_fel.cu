@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(LevelShape<NC, BG>::kThreads, LevelShape<NC, B
         if (tid == 0) { sE = 0; sL = 0.0; }
         __syncthreads();
         // as many nodes at once as leaves no warp idle
-        auto group = [](int nodes) { return min(GM, nodes <= W ? 1 : (nodes <= 2 * W ? 2 : 4)); };
+        auto group = [](int nodes) { return nodes <= W ? 1 : GM; };
         auto load = [&](int4 (&d)[GM], int i, int g, int end) {
 #pragma unroll
             for (int k = 0; k < GM; ++k)
@@ -623,8 +623,7 @@ __global__ void __launch_bounds__(LevelShape<NC, BG>::kThreads, LevelShape<NC, B
                 const int count = min(g, b1 - i);
                 if (i >= b0 + W * g) load(d, i, g, b1);
                 if (g == 1) level_nodes<NC, BG, 1>(rq, f, t, bl, d, count, lane);
-                else if (GM == 2 || g == 2) level_nodes<NC, BG, GM < 2 ? 1 : 2>(rq, f, t, bl, d, count, lane);
-                else level_nodes<NC, BG, GM < 4 ? 1 : 4>(rq, f, t, bl, d, count, lane);
+                else level_nodes<NC, BG, GM>(rq, f, t, bl, d, count, lane);
             }
             __syncthreads();                               // this level's messages are visible to the next
 #pragma unroll

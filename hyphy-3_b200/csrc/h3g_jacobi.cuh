@@ -103,7 +103,7 @@ __device__ __forceinline__ double2 rotation(double apq, double app, double aqq, 
     return make_double2(c, s);
 }
 
-// A worker's four seats of one row of E through their rotations.  kRole: x is the p of 0 no seat, 1 every seat,
+// A worker's eight seats (kSeats) of one row of E through their rotations.  kRole: x is the p of 0 no seat, 1 every seat,
 // 2 the seats k >= first.
 template <int kRole>
 __device__ __forceinline__ void rotate_seats(double (&ex)[kSeats], double (&ey)[kSeats], const double2* cs, int first) {
