@@ -66,7 +66,7 @@ struct h3g_problem {
     h3g_batch* batch = nullptr;        // the batch this problem evaluates in (its workspace lives there)
     int n = 0, root = -1, T = 0, P = 0, Pp = 0, NI = 0, max_state = -1;
     std::vector<int> ch_off, ch, iidx, taxon, in_off, out_off, in_nodes, out_nodes, out_split, out_int_off, parent_h;
-    std::vector<uint8_t> leaf;
+    std::vector<uint8_t> leaf, no_operand;           // no_operand: leaves with one sibling (leaf_on_the_fly)
     std::vector<int> bfs_order, depth_h, height_h;   // BFS order from the root, node depths and heights
     std::vector<int8_t> states_pm;     // [P][T] as uploaded (per-pattern checks on the host)
     DevArena topo_mem, model_mem, work_mem;
@@ -74,6 +74,8 @@ struct h3g_problem {
     int* d_out_split = nullptr;        // out_nodes: the internal ones (levels out_int_off), then leaf pairs (split_kids)
     h3g_leaf_pairs pairs;
     int* d_parent = nullptr;
+    int* d_vidx = nullptr;             // Topo::vidx of the full workspace
+    int n_stored = 1;                  // its gradient-operand slots
     uint8_t* d_leaf = nullptr;
     int2* d_kdesc = nullptr;
     int4* d_in_info = nullptr;
@@ -160,7 +162,7 @@ struct h3g_problem {
         t.in_next = d_chains; t.in_heads = d_chains + off_in_heads;
         t.out_next = d_chains + off_out_next; t.out_heads = d_chains + off_out_heads;
         t.all_mask = S >= 64 ? ~uint64_t(0) : ((uint64_t(1) << S) - 1);
-        t.vidx = nullptr;
+        t.vidx = d_vidx;
         t.ncp = 0;
         t.few_in = d_few; t.few_out = d_few ? d_few + 2 * in_nodes.size() : nullptr;
         t.few_in_lv = d_few_lv; t.few_out_lv = d_few_lv + in_off.size();
@@ -379,11 +381,21 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
             const int u = pr->in_nodes[k];
             in_info[k] = make_int4(u, pr->iidx[u], pr->ch_off[u], pr->ch_off[u + 1]);
         }
+        // gradient-operand slots of the mixed path, none for a leaf with one sibling (leaf_on_the_fly)
+        std::vector<int> vidx(n, 0);
+        int stored = 0;
+        pr->no_operand.assign(size_t(n), 0);
+        for (int c = 0; c < n; ++c) {
+            if (parent[c] < 0) continue;
+            if (is_leaf[c] && kids[size_t(parent[c])].size() == 2) pr->no_operand[size_t(c)] = 1;
+            else vidx[c] = stored++;
+        }
+        pr->n_stored = std::max(stored, 1);
         std::vector<int4> out_info(2 * std::max<size_t>(pr->out_nodes.size(), 1));
         for (size_t k = 0; k < pr->out_nodes.size(); ++k) {
             const int c = pr->out_nodes[k], u = parent[c];
             out_info[2 * k] = make_int4(c, u, pr->iidx[u], is_leaf[c] ? -1 : pr->iidx[c]);
-            out_info[2 * k + 1] = make_int4(pr->ch_off[u], pr->ch_off[u + 1], 0, 0);
+            out_info[2 * k + 1] = make_int4(pr->ch_off[u], pr->ch_off[u + 1], vidx[c], 0);
         }
         // chains (see Topo): inside, a node whose parent has no other internal child hands its
         // message to the parent in the same CTA; outside, a node continues with its deepest
@@ -419,7 +431,7 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         // (no item for a leaf with one sibling: leaf_on_the_fly)
         for (size_t k = 0; k < pr->out_nodes.size(); ++k) {
             const int c = pr->out_nodes[k];
-            if (!fused_out[k] && !(is_leaf[c] && kids[size_t(parent[c])].size() == 2)) out_heads.push_back(int(k));
+            if (!fused_out[k] && !pr->no_operand[size_t(c)]) out_heads.push_back(int(k));
         }
         pr->n_in_heads = int(in_heads.size());
         pr->n_out_heads = int(out_heads.size());
@@ -436,6 +448,8 @@ extern "C" h3g_status h3g_problem_create(h3g_ctx* ctx, int n_nodes, const int32_
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_kdesc, kdesc.size()));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_in_info, in_info.size()));
         H3G_TRY_CUDA(ctx, A.alloc(&pr->d_out_info, out_info.size()));
+        H3G_TRY_CUDA(ctx, A.alloc(&pr->d_vidx, size_t(n)));
+        H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_vidx, vidx.data(), size_t(n) * sizeof(int), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_kdesc, kdesc.data(), kdesc.size() * sizeof(int2), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_in_info, in_info.data(), in_info.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
         H3G_TRY_CUDA(ctx, cudaMemcpyAsync(pr->d_out_info, out_info.data(), out_info.size() * sizeof(int4), cudaMemcpyHostToDevice, s));
@@ -610,8 +624,8 @@ struct WsLayout {
 // Patterns per A-accumulation chunk come in multiples of this: two stages of the FP64 kernels, one tile of the mixed one.
 constexpr int kChunkGrain = 64;
 
-// part_nodes / vf_nodes: partial slots of internal nodes and gradient-operand slots (NI and n, or
-// fewer under a checkpoint plan).  coarse: A chunks of 256 patterns and more also for FP64.
+// part_nodes / vf_nodes: partial slots of internal nodes and the mixed path's gradient-operand slots (NI and n unless
+// given).  coarse: A chunks of 256 patterns and more also for FP64.
 static WsLayout ws_layout(int precision, size_t n, size_t NI, size_t Pp, int M, int K, int nmod, int ndirs, const h3g_tuning& tu,
                           size_t part_nodes = 0, size_t vf_nodes = 0, bool coarse = false) {
     (void)K;
@@ -802,7 +816,7 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
             const int c = B.out_kids[k], u = pr->parent_h[c];
             pos[c] = int(k);
             info.push_back(make_int4(c, u, pl.iidx[u], pr->leaf[c] ? -1 : pl.iidx[c]));
-            info.push_back(make_int4(pr->ch_off[u], pr->ch_off[u + 1], 0, 0));
+            info.push_back(make_int4(pr->ch_off[u], pr->ch_off[u + 1], pl.vidx[c], 0));
         }
         std::vector<int> onxt(B.out_kids.size(), -1), oheads;
         std::vector<char> ofused(B.out_kids.size(), 0);
@@ -819,7 +833,7 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
         }
         for (size_t k = 0; k < B.out_kids.size(); ++k) {
             const int c = B.out_kids[k];
-            if (!ofused[k] && !(pr->leaf[c] && kids[size_t(pr->parent_h[c])].size() == 2)) oheads.push_back(int(k));
+            if (!ofused[k] && !pr->no_operand[size_t(c)]) oheads.push_back(int(k));
         }
         o.out_next = int(lists.size());
         lists.insert(lists.end(), onxt.begin(), onxt.end());
@@ -853,7 +867,7 @@ static h3g_status upload_checkpoints(h3g_problem* pr) {
 // no block size is forced; else the plan with the largest block size whose layout fits.
 static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndirs, const h3g_tuning& tu, uint64_t held,
                                 WsLayout& L) {
-    const WsLayout full = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu);
+    const WsLayout full = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), M, K, nmod, ndirs, tu, 0, size_t(pr->n_stored));
     pr->full_bytes = ws_bytes(full, pr->precision);
     uint64_t budget = pr->mem_budget;
     if (!budget) {
@@ -868,7 +882,7 @@ static h3g_status choose_layout(h3g_problem* pr, int M, int K, int nmod, int ndi
     }
     const auto kids = children_of(pr);
     auto make = [&](int target) {
-        return h3g::plan_checkpoints(pr->n, pr->root, kids, pr->leaf.data(), pr->bfs_order, pr->depth_h, pr->height_h, target);
+        return h3g::plan_checkpoints(pr->n, pr->root, kids, pr->leaf.data(), pr->bfs_order, pr->depth_h, pr->height_h, target, pr->no_operand.data());
     };
     bool coarse = false;
     auto layout_of = [&](const h3g::CkPlan& p) {
@@ -1991,7 +2005,7 @@ static h3g_status batch_prepare(h3g_batch* b) {
     for (int g = 0; g < G; ++g) {
         const h3g_problem* pr = b->probs[g];
         lay[g] = ws_layout(pr->precision, size_t(pr->n), size_t(pr->NI), size_t(pr->Pp), pr->M, pr->K, pr->nmod, pr->ndirs,
-                           effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs));
+                           effective_tuning(pr, pr->M, pr->K, pr->nmod, pr->ndirs), 0, size_t(pr->n_stored));
     }
     const bool first = b->slots[0]->genes.empty() && b->slots[0]->w.P == nullptr;
     if (first || prec != b->precision) {

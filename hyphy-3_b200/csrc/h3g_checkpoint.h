@@ -38,14 +38,15 @@ struct CkPlan {
     int ncp = 0, scratch_int = 0, scratch_all = 0;
     std::vector<uint8_t> is_ckpt;   // [n]
     std::vector<int> block_of;      // [n] block computing the node
-    std::vector<int> iidx, vidx;    // [n] partial slot (internal nodes, else -1) and gradient-operand slot
+    std::vector<int> iidx, vidx;    // [n] partial slot (internal nodes, else -1) and gradient-operand slot (0 without one)
     std::vector<CkBlock> blocks;    // post-order, the root's block last
 };
 
-// kids[u] in increasing id order; order = BFS order from the root (parents before children).
+// kids[u] in increasing id order; order = BFS order from the root (parents before children).  no_operand[u]: leaf u
+// stores no gradient operand and gets no slot for one (NULL: every node gets one).
 inline CkPlan plan_checkpoints(int n, int root, const std::vector<std::vector<int>>& kids, const uint8_t* is_leaf,
                                const std::vector<int>& order, const std::vector<int>& depth,
-                               const std::vector<int>& height, int target) {
+                               const std::vector<int>& height, int target, const uint8_t* no_operand = nullptr) {
     CkPlan pl;
     pl.target = std::max(target, 2);
     pl.is_ckpt.assign(n, 0);
@@ -90,7 +91,7 @@ inline CkPlan plan_checkpoints(int n, int root, const std::vector<std::vector<in
         for (int u : members) {
             if (u == B.root) continue;
             if (!is_leaf[u]) pl.iidx[u] = pl.ncp + li++;
-            pl.vidx[u] = pl.ncp + lv++;
+            pl.vidx[u] = no_operand && no_operand[u] ? 0 : pl.ncp + lv++;
         }
         pl.scratch_int = std::max(pl.scratch_int, li);
         pl.scratch_all = std::max(pl.scratch_all, lv);

@@ -10,8 +10,8 @@
 //                                           a warp reading one state of 32
 //                                           consecutive patterns is coalesced
 //   Ecum, Eown         [NI][M][Pp]          power-of-two scaling exponents
-//   Vf                 [n][M][64][Pp]       outside vector at the top of each branch times
-//                                           w_p * posterior_m / L_m (FP64 path: [NI], internal branches only)
+//   Vf                 [NI][M][64][Pp]      outside vector at the top of each internal branch times
+//                                           w_p * posterior_m / L_m (mixed path: slots Topo::vidx, with the leaves of polytomies)
 // Leaves never get a partial: their message P_b * leaf_vector is a column of P_b
 // (a row of PT_b), a masked column sum, or the P_b row sums for missing data.
 #pragma once
@@ -72,16 +72,15 @@ struct Topo {
     // per-item descriptors of the persistent passes, one load each instead of a chain of lookups
     const int2* kdesc;       // [children CSR] {child, code}: code = taxon (>= 0) or -1 for a leaf, -(2 + iidx) for an internal child
     const int4* in_info;     // [internal nodes, inside order] {u, iidx[u], first child slot, end}
-    const int4* out_info;    // [2 x children, outside order] {c, u, iidx[u], iidx[c] or -1}, {first sibling slot, end, 0, 0}
+    const int4* out_info;    // [2 x children, outside order] {c, u, iidx[u], iidx[c] or -1}, {first sibling slot, end, vidx[c], 0}
     // chains of the persistent passes: the items are chain heads; a CTA carries a chain's
     // message in registers from one node to the next
     const int* in_next;      // [inside position] position of the parent when its only internal child is this node, else -1
     const int* in_heads;     // [chains] inside position of each chain's first node, inside order
     const int* out_next;     // [outside position] position of this node's deepest internal child, else -1
     const int* out_heads;    // [chains] outside position of each chain's first node, outside order
-    // subtree checkpointing: Vf slot of each node (NULL: the node id).  With checkpoints, iidx and vidx
-    // map checkpoint nodes to persistent slots [0, ncp) and every other node to a scratch slot that
-    // the nodes of other blocks reuse
+    // the mixed path's Vf slot of each branch that stores one.  With checkpoints, iidx and vidx map checkpoint nodes to
+    // persistent slots [0, ncp) and every other node to a scratch slot that the nodes of other blocks reuse
     const int* vidx;
     int ncp;
     // walks of the passes for models of at most kFewStates states (h3g_few.cu): item descriptors in level order, two
@@ -97,8 +96,6 @@ constexpr int kFewStates = 4;
 __device__ __forceinline__ bool leaf_on_the_fly(const Topo& t, int b) {
     return t.leaf[b] && t.ch_off[t.parent[b] + 1] - t.ch_off[t.parent[b]] == 2;
 }
-
-__device__ __forceinline__ int vslot(const Topo& t, int b) { return t.vidx ? t.vidx[b] : b; }
 
 struct Model {
     int M, K, has_bg, nmod, time_mode, ndirs, sentinel;

@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_outside_mx(Topo t, Model md, Wo
             const int EL = mw.ED[col_off(ir, m, M, t.Pp) + p];
             const int EDc = internal ? mw.ED[col_off(ic, m, M, t.Pp) + p] : 0;
             const double scale = ldexp(w.f[size_t(m) * Pp + p], EL - EV - EDc);
-            float* vf = mw.Vf + part_off(vslot(t, c), m, M, t.Pp) + so;
+            float* vf = mw.Vf + part_off(oj.z, m, M, t.Pp) + so;
 #pragma unroll
             for (int i = 0; i < kSG; ++i) vf[i * Pp] = v[i] * float(scale);
             if (!internal) break;                          // a leaf: no outside vector below it
@@ -723,7 +723,7 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumA_mx(Topo t, Model md, 
     const bool sib_tile = fly && sb.y <= -2, sib_rows = fly && sb.y >= -1, at_root = u == t.root;
     const float* PTs = mw.PT32 + mat_off_f(m, sb.x, t.n);
     const int iu = t.iidx[u], is = sib_tile ? -(sb.y + 2) : 0;
-    const float* Vb = fly ? mw.U + part_off(at_root ? 0 : iu, m, M, t.Pp) : mw.Vf + part_off(vslot(t, b), m, M, t.Pp);
+    const float* Vb = fly ? mw.U + part_off(at_root ? 0 : iu, m, M, t.Pp) : mw.Vf + part_off(t.vidx[b], m, M, t.Pp);
     const float* Db = lf ? mw.Ms + part_off(is, m, M, t.Pp) : mw.D + part_off(t.iidx[b], m, M, t.Pp);
     const bool load_v = !(fly && at_root), load_d = !lf || sib_tile;
     unsigned char* ring = smraw + 2 * kStage;

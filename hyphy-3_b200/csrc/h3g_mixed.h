@@ -19,7 +19,7 @@ struct MixedWork {
     float* D = nullptr;      // [NI][M][64][Pp]  inside partial (normalised)
     float* Ms = nullptr;     // [NI][M][64][Pp]  message P*D to the parent (normalised)
     float* U = nullptr;      // [NI][M][64][Pp]  outside partial below the parent branch (normalised)
-    float* Vf = nullptr;     // [n][M][64][Pp]   f * V * 2^(EL - EV - ED) (gradient operand, O(1) scale)
+    float* Vf = nullptr;     // [slots Topo::vidx][M][64][Pp]   f * V * 2^(EL - EV - ED) (gradient operand, O(1) scale)
     int* ED = nullptr;       // [NI][M][Pp]      exponent of D
     int* EM = nullptr;       // [NI][M][Pp]      exponent of Ms
     int* EU = nullptr;       // [NI][M][Pp]      exponent of U

@@ -31,7 +31,8 @@ def test_the_smallest_budget_that_holds_large_chunks(oracle, sites, precision_na
     ref = {"lnl": ref["lnl"], "grad_t": ref["grad_t"].copy()}
     pr.set_memory_budget(need)
     info = pr.checkpoint_info()
-    assert info["active"] and info["workspace_bytes"] <= need
+    assert info["workspace_bytes"] <= need
+    assert info["active"] or precision_name == "mixed"            # (its full workspace may be as small)
     got = pr.eval(bl)
     # the likelihood's order of summation is the same; the gradient's sums of at most 1000 terms are regrouped
     assert got["lnl"] == ref["lnl"]
