@@ -108,11 +108,25 @@ __global__ void __launch_bounds__(32 * kFewWarps) k_inside_few(Topo t, Model md,
                 few_msg(x, t, w, m, M, make_int2(d.z, d.w), p, s1);
                 eown += few_mul(v, x);
             }
-            for (int k = k0 + 2; k < k1; ++k) {
-                const int2 c = t.kdesc[k];
+            if (k0 + 2 < k1) {
+                // a polytomy: descriptors three, states two and messages one child ahead.  One after the other they are a
+                // chain of three loads for each child: a value of a star of 400 leaves x 32000 patterns took 1740 us (the
+                // 64-state passes 1474), now 1052; of 100 leaves x 14400 257 (233), now 191
+                auto desc = [&](int k) { return k < k1 ? t.kdesc[k] : make_int2(0, -1); };
+                int2 c = desc(k0 + 2), c1 = desc(k0 + 3), c2 = desc(k0 + 4);
+                int st1 = few_state(t, c1, p);
                 few_msg(x, t, w, m, M, c, p, few_state(t, c, p));
-                eown += few_mul(v, x);
-                if (c.y <= -2) ecum += w.Ecum[col_off(-(c.y + 2), m, M, t.Pp) + p];
+                for (int k = k0 + 2; k < k1; ++k) {
+                    const int2 c3 = desc(k + 3);
+                    const int st2 = few_state(t, c2, p);
+                    double next[kFewStates];
+                    if (k + 1 < k1) few_msg(next, t, w, m, M, c1, p, st1);
+                    if (c.y <= -2) ecum += w.Ecum[col_off(-(c.y + 2), m, M, t.Pp) + p];
+                    eown += few_mul(v, x);
+#pragma unroll
+                    for (int q = 0; q < kFewStates; ++q) x[q] = next[q];
+                    c = c1; c1 = c2; c2 = c3; st1 = st2;
+                }
             }
             const size_t o = part_off(iu, m, M, t.Pp) + p, oc = col_off(iu, m, M, t.Pp) + p;
 #pragma unroll
