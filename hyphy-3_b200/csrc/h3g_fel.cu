@@ -367,9 +367,14 @@ struct LevelPlan {
 // CTA shape by the eigensystems of a request (nc tested components, plus the background's when bg): threads, CTAs to an
 // SM, and the nodes of a level that a warp takes at once (a row of U or V is then read once for all of them; the
 // nodes of a background branch use other matrices, so with a background it is one).
-template <int NC, bool BG>
+// FEW: one component and no more requests than SMs (a run's last batches, small alignments).  Three CTAs of 8 warps have
+// nothing to share an SM for then, and 8 warps take a wide level in twice the turns: CTAs of 16, one to an SM.  Whole FEL
+// runs, always 8 warps -> this: 1024 taxa x 100 codons 156 -> 89 ms (two CTAs of 16 for all, one node at a time, 145),
+// x 6 107 -> 74, 256 x 100 63 -> 46, x 300 87 -> 85, chain of 128 x 30 87 -> 66, 8 x 40 34 -> 32.
+template <int NC, bool BG, bool FEW = false>
 struct LevelShape {
-    static constexpr int kThreads = NC == 1 && !BG ? 256 : 512, kPerSm = NC == 1 && !BG ? 3 : 1;
+    static constexpr bool kSmall = NC == 1 && !BG && !FEW;
+    static constexpr int kThreads = kSmall ? 256 : 512, kPerSm = kSmall ? 3 : 1;
     static constexpr int kGroup = BG ? 1 : 2, kWarps = kThreads / 32;
     // eigensystems, and the group's vectors per warp
     static constexpr size_t kSmem = (size_t(NC + (BG ? 1 : 0)) * (2 * SP * LD + SP) + size_t(kWarps) * kGroup * NC * SP) * sizeof(double);
@@ -557,10 +562,10 @@ __device__ __forceinline__ void level_nodes(const LevelRequest<NC, BG>& q, const
     }
 }
 
-template <int NC, bool BG>
-__global__ void __launch_bounds__(LevelShape<NC, BG>::kThreads, LevelShape<NC, BG>::kPerSm) k_site_lnl(FelModel f, Topo t, const double* __restrict__ bl, LevelPlan lp,
+template <int NC, bool BG, bool FEW = false>
+__global__ void __launch_bounds__(LevelShape<NC, BG, FEW>::kThreads, LevelShape<NC, BG, FEW>::kPerSm) k_site_lnl(FelModel f, Topo t, const double* __restrict__ bl, LevelPlan lp,
                                                    double* __restrict__ work, FelReqs q, int n_req, double* __restrict__ out) {
-    using Shape = LevelShape<NC, BG>;
+    using Shape = LevelShape<NC, BG, FEW>;
     constexpr int NT = NC + (BG ? 1 : 0), W = Shape::kWarps, GM = Shape::kGroup;
     pdl_enter();
     extern __shared__ __align__(16) double sm[];
@@ -768,6 +773,7 @@ struct FelDevice {
     int H = 0;
     double* d_work = nullptr;             // level-synchronous pruning: [grid][n][64] messages
     int grid[2][2] = {{1, 1}, {1, 1}};    // persistent CTAs per [tested components - 1][background]
+    int few_requests = 0;                 // up to this many, a CTA has an SM to itself (LevelShape)
     unsigned char* d_req = nullptr;       // per batch: [om | a | w1 | eslot | eprev | pat | slot | slot2 | slot_bg], packed to the batch's sizes
     unsigned char* h_req = nullptr;       // pinned mirror
     double* d_out = nullptr;
@@ -883,6 +889,7 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
     if (ok && !configured) {
         ok = cudaFuncSetAttribute(k_fel_eig, cudaFuncAttributeMaxDynamicSharedMemorySize, int(jac::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<1, false>::kSmem)) == cudaSuccess &&
+             cudaFuncSetAttribute(k_site_lnl<1, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<1, false, true>::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<2, false>::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<1, true>::kSmem)) == cudaSuccess &&
              cudaFuncSetAttribute(k_site_lnl<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(LevelShape<2, true>::kSmem)) == cudaSuccess &&
@@ -903,6 +910,7 @@ FelDevice* fel_device_alloc(h3g_problem* pr, const FelProblemView& v, int max_re
         --ctas;
     }
     if (!d->d_work) { *err = "device allocation failed"; delete d; return nullptr; }
+    d->few_requests = sms;
     for (int c = 0; c < 2; ++c)
         for (int b = 0; b < 2; ++b) d->grid[c][b] = std::max(1, std::min(per[c][b], ctas) * std::max(sms, 1));
     return d;
@@ -1049,7 +1057,12 @@ bool fel_device_eval(FelDevice* d, int n_eig, const double* eig_omega, const int
         double* o = d->d_out + k0;
         const int grid = std::min(cnt, d->grid[g & 1][g >> 1]);
         switch (g) {
-            case 0: launch_k(k_site_lnl<1, false>, grid, LevelShape<1, false>::kThreads, LevelShape<1, false>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
+            case 0:
+                if (cnt <= d->few_requests) {
+                    launch_k(k_site_lnl<1, false, true>, cnt, LevelShape<1, false, true>::kThreads, LevelShape<1, false, true>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o);
+                    break;
+                }
+                launch_k(k_site_lnl<1, false>, grid, LevelShape<1, false>::kThreads, LevelShape<1, false>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
             case 1: launch_k(k_site_lnl<2, false>, grid, LevelShape<2, false>::kThreads, LevelShape<2, false>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
             case 2: launch_k(k_site_lnl<1, true>, grid, LevelShape<1, true>::kThreads, LevelShape<1, true>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
             default: launch_k(k_site_lnl<2, true>, grid, LevelShape<2, true>::kThreads, LevelShape<2, true>::kSmem, s, d->f, d->t, bl, lp, d->d_work, qg, cnt, o); break;
