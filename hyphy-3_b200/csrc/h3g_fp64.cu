@@ -579,9 +579,8 @@ constexpr int kAL = kAccP + 4;                                 // row stride of 
 constexpr size_t kAccStage = size_t(2) * SP * kAL;             // V and D tiles of one stage
 static const size_t kAccIntSmem = 2 * kAccStage * sizeof(double);
 
-__global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, const int* __restrict__ branches) {
-    extern __shared__ __align__(16) double smA[];
-    const int b = branches[blockIdx.x], m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
+__device__ __forceinline__ void accumA_int(double* smA, const Topo& t, const Model& md, const Work& w, int b) {
+    const int m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
     const size_t Pp = size_t(t.Pp);
     const int p_begin = ck * w.chunk, nst = (min(t.Pp, p_begin + w.chunk) - p_begin) / kAccP;
     const size_t o = part_off(t.iidx[b], m, M, t.Pp) + p_begin;
@@ -633,6 +632,11 @@ __global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, co
             *reinterpret_cast<double2*>(dst + frag_row(i) * SP + frag_col(j, 0)) = make_double2(acc.v[i][j][0], acc.v[i][j][1]);
 }
 
+__global__ void __launch_bounds__(256) k_accumA_int(Topo t, Model md, Work w, const int* __restrict__ branches) {
+    extern __shared__ __align__(16) double smA[];
+    accumA_int(smA, t, md, w, branches[blockIdx.x]);
+}
+
 // Leaf branches: D is a 0/1 vector, one state of each pattern for an unambiguous codon, so A[:, s] is the sum of the f V
 // columns of the patterns in state s: 64 additions a pattern instead of a 64 x 64 outer product.  `leaves` holds
 // one leaf, or the two of a node whose children are just these (x, y; y = -1 without): V of both comes from one read
@@ -681,13 +685,11 @@ __device__ __forceinline__ void leaf_add(double* sA, const double* sV, int own, 
 // 636 (451 and 34), of 12 x 100 31 us in place of 39.  With up to 9 children it is no faster (ladder of 9-child nodes: 108 us
 // each way), and its registers would cost the pairs a third (256 taxa x 2000 codons 547 us in place of 407).
 template <bool kMany>
-__global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w, const int2* __restrict__ leaves) {
-    extern __shared__ __align__(16) double smA[];
+__device__ __forceinline__ void accumA_leaf(double* smA, const Topo& t, const Model& md, const Work& w, int2 cc) {
     double* sA = smA + 2 * SP * kLV;
     double* smax = sA + 2 * kLCols * kLA;
     const int m = blockIdx.y, ck = blockIdx.z, tid = threadIdx.x, M = md.M;
     const int g = tid >> 5, lane = tid & 31;
-    const int2 cc = leaves[blockIdx.x];
     const bool pair = !kMany && cc.y >= 0;
     const int u = t.parent[cc.x], iu = t.iidx[u], k0 = t.ch_off[u], k1 = t.ch_off[u + 1];
     const size_t Pp = size_t(t.Pp);
@@ -799,6 +801,25 @@ __global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w
         }
     }
 }
+
+template <bool kMany>
+__global__ void __launch_bounds__(256, 2) k_accumA_leaf(Topo t, Model md, Work w, const int2* __restrict__ leaves) {
+    extern __shared__ __align__(16) double smA[];
+    accumA_leaf<kMany>(smA, t, md, w, leaves[blockIdx.x]);
+}
+
+// Both where they fit side by side (kAccSideBySide CTAs): a checkpoint block's few branches or a small gene leave most SMs
+// idle, and two launches wait for each other.  256 taxa x 2000 codons x 2 rates in 33 blocks 14.2 -> 11.6 ms an
+// evaluation, 600 x 1000 in 6 blocks 3.54 -> 3.20, in 80 17.5 -> 15.0; a star of 12 x 60 80 -> 70 us.
+// The leaves come first: theirs is the longer chain.  grid (n_leaves + internal branches, M, nchunk), block 256.
+__global__ void __launch_bounds__(256, 2) k_accumA_both(Topo t, Model md, Work w, const int2* __restrict__ leaves, int n_leaves,
+                                                        const int* __restrict__ branches) {
+    extern __shared__ __align__(16) double smA[];
+    const int x = blockIdx.x;
+    if (x < n_leaves) accumA_leaf<false>(smA, t, md, w, leaves[x]);
+    else accumA_int(smA, t, md, w, branches[x - n_leaves]);
+}
+constexpr long kAccSideBySide = 2 * 148;
 
 __device__ __forceinline__ double block_sum_256(double x, double* red) {
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -1051,6 +1072,7 @@ void fp64_configure() {
     cudaFuncSetAttribute(k_frechet, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kFrechetSmem));
     cudaFuncSetAttribute(k_dir, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kDirSmem));
     cudaFuncSetAttribute(k_accumA_int, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccIntSmem));
+    cudaFuncSetAttribute(k_accumA_both, cudaFuncAttributeMaxDynamicSharedMemorySize, int(std::max(kAccIntSmem, kAccLeafSmem)));
     cudaFuncSetAttribute(k_accumA_leaf<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccLeafSmem));
     cudaFuncSetAttribute(k_accumA_leaf<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kAccLeafSmem));
 }
@@ -1091,10 +1113,16 @@ int launch_outside_fp64(const Topo& t, const Model& md, const Work& w, const int
 }
 int launch_accumA_fp64(const Topo& t, const Model& md, const Work& w, const int* d_internal, int n_internal, const int2* d_leaves,
                        int n_leaves, int n_many, cudaStream_t s) {
-    if (n_internal) launch_k(k_accumA_int, dim3(n_internal, md.M, w.nchunk), 256, kAccIntSmem, s, t, md, w, d_internal);
-    if (n_leaves) launch_k(k_accumA_leaf<false>, dim3(n_leaves, md.M, w.nchunk), 256, kAccLeafSmem, s, t, md, w, d_leaves);
+    const bool both = n_internal && n_leaves && long(n_internal + n_leaves) * md.M * w.nchunk <= kAccSideBySide;
+    if (both) {
+        launch_k(k_accumA_both, dim3(n_leaves + n_internal, md.M, w.nchunk), 256, std::max(kAccIntSmem, kAccLeafSmem), s, t, md, w, d_leaves,
+                 n_leaves, d_internal);
+    } else {
+        if (n_internal) launch_k(k_accumA_int, dim3(n_internal, md.M, w.nchunk), 256, kAccIntSmem, s, t, md, w, d_internal);
+        if (n_leaves) launch_k(k_accumA_leaf<false>, dim3(n_leaves, md.M, w.nchunk), 256, kAccLeafSmem, s, t, md, w, d_leaves);
+    }
     if (n_many) launch_k(k_accumA_leaf<true>, dim3(n_many, md.M, w.nchunk), 256, kAccLeafSmem, s, t, md, w, d_leaves + n_leaves);
-    return (n_internal > 0) + (n_leaves > 0) + (n_many > 0);
+    return both ? 1 + (n_many > 0) : (n_internal > 0) + (n_leaves > 0) + (n_many > 0);
 }
 int launch_frechet(const Topo& t, const Model& md, const Work& w, int want_global, cudaStream_t s) {
     launch_k(k_areduce, dim3(t.n, md.M), 256, 0, s, t, md, w);
