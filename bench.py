@@ -60,10 +60,11 @@ WORKLOADS = {
 # summed over the stage's launches in the ncu launch list of `bench.py --profile` (one evaluation,
 # --clock-control none).  The 1024-taxon workload is captured on its 512-codon prefix and scaled by
 # the padded pattern count (5120 / 512): these stages stream per-pattern partials, so their traffic is
-# proportional to the patterns processed.
+# proportional to the patterns processed.  (accum_A: its reads; its writes are one 64 x 64 block for every branch,
+# rate class and chunk of patterns, two chunks here.)
 MEASURED_TRAFFIC = {
     (1, "mixed"): {"inside": 19.5e6},
-    (3, "mixed"): {"inside": 14.724e9},
+    (3, "mixed"): {"inside": 14.71e9, "outside": 16.81e9, "accum_A": 17.16e9},
     # alignment compression, 1024 taxa x 100000 codons, captured at full size (one pass:
     # dram__bytes_read.sum + dram__bytes_write.sum of the call's launch)
     ("compress", "translate"): 479.30e6,

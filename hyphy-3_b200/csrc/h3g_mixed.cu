@@ -770,7 +770,7 @@ __global__ void __launch_bounds__(kAccThreads, 1) k_accumA_mx(Topo t, Model md, 
             if (sib_rows) {
                 // the sibling leaf's message at each pattern: its row of FP32 P^T (or the row sums, or a masked sum).  The masks of
                 // unresolved states first, all at once: one after the other they are four trips to memory, and the sums' rows in
-                // pairs (256 taxa x 3000 codons with 30 % missing data 1118 -> 1080 us an evaluation, 64 x 1500 with half 359 -> 322)
+                // pairs (256 taxa x 3000 codons with 30 % missing data 1113 -> 1076 us an evaluation, 64 x 1500 with half 328 -> 317)
                 uint64_t mks[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
